@@ -138,6 +138,8 @@ DevParams kf_make_dev_params(const int n[3], const kf_params *p) {
   d.ny = n[1];
   d.nz = n[2];
   d.count = (int64_t)n[0] * n[1] * n[2];
+  d.by_row = kf_divisor((unsigned)n[0]);
+  d.by_plane = kf_divisor((unsigned)n[0] * (unsigned)n[1]);
   d.voxel_size = p->voxel_size;
   d.unknown_clip = p->unknown_clip;
   d.max_surface = p->max_surface;

@@ -153,8 +153,11 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_runs(const int2 *__rest
 // st[iter].cold.  A cold pass stops once the iteration before it was
 // skipped (the statistics of that iteration's band pass may still be in
 // flight when it runs, so it may run once after convergence, to no effect).
+// Eight CTAs per SM of the cold pass (32 registers), for the loads in flight:
+// the dense 256^3 iteration takes 41.5 us, with six CTAs 41.6 us, with five
+// (44 registers) 42.9 us.
 template <bool kCold>
-__global__ void __launch_bounds__(kThreads) k_fused_stream_runs(FusedArgs a, const int *__restrict__ run_list,
+__global__ void __launch_bounds__(kThreads, kCold ? 8 : 5) k_fused_stream_runs(FusedArgs a, const int *__restrict__ run_list,
                                                                const unsigned *__restrict__ counts,
                                                                int *__restrict__ list,
                                                                const int *__restrict__ prev_list,
@@ -204,6 +207,10 @@ __global__ void __launch_bounds__(kThreads) k_fused_stream_runs(FusedArgs a, con
 // st[iter+1].list).  kInPlace: the new psi of list entry k goes to entry k
 // of the output planes, for k_fused_scatter to write back.  kTrust: the
 // trust-region step (dp.trust), followed by k_trust_fix.
+// The dense solver runs it beside the cold passes, which live on L1 and
+// occupancy, so it takes no shared memory to speak of: with the groups of four
+// warps of the band-only solver (13 KB a group) the 256^3 iteration took 42.7 us
+// against 41.6 us, and 53 us where their carveout was half the SM's.
 template <bool kCarry, bool kInPlace, bool kTrust = false>
 __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(FusedArgs a, const int *__restrict__ list_in,
                                                              int *__restrict__ list_out) {
@@ -231,140 +238,220 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
 }
 
 // Band-only solver, every iteration in one cooperative launch.  One band pass
-// per iteration as k_fused_band<kCarry> (ping-pong buffers, the updated
-// voxels carried to the next iteration's list), then a grid-wide barrier
-// (kf_grid_sync.cuh) instead of a kernel boundary.
-// - Each block takes an equal contiguous slice of the first band list and
-//   keeps its own voxels from then on: the band can only shrink, so a
-//   block's carried voxels are compacted into its own slice of the other
-//   list, with no global atomic on the iteration's critical path.
-// - A block's voxels alternate between its warps, so that a small band (a
-//   few dozen voxels per block at 256^3) keeps every scheduler of the SM
-//   busy; neighbouring band voxels (which share psi neighbours) stay in one
-//   SM's L1.
+// per iteration (ping-pong buffers, the updated voxels carried to the next
+// iteration's list), then a grid-wide barrier (kf_grid_sync.cuh) instead of
+// a kernel boundary.
+// - Each group of four warps (group_update) takes an equal contiguous slice
+//   of the first band list and keeps its own voxels from then on: the band
+//   can only shrink, so a group's carried voxels are compacted into its own
+//   slice of the other list by a ballot of its warp 0, with no atomic and no
+//   block-wide step.  Neighbouring band voxels (which share psi neighbours)
+//   stay in one SM's L1.
 // - psi is read through L1 and L2 (kPsiL1: the blocks write it between
 //   iterations, ordered by the barrier's fences), the SDFs through the
 //   read-only path.  A gated iteration (converged, diverged) ends the kernel
 //   in every block alike: the barrier brings each block the same verdict
-//   (grid_sync_verdict), so no block reads the statistics after it, and a
-//   block's first round of voxels comes from shared memory: the psi loads
+//   (grid_verdict), so no block reads the statistics after it, and a
+//   group's first round of voxels comes from shared memory: the psi loads
 //   of the next iteration start as soon as the barrier lets a block go.
-// 96-thread blocks, 1 per SM: a 255-register budget (the band update does
-// not spill), three warps a block, most of each SM's registers left to the
-// frame's other kernels, which run beside the solve.  The grid barrier's
-// cost grows with the number of blocks (alone, with no work between
-// barriers: 2.3 us for 608 blocks, 1.5 us for 304, 1.3 us for 152); of
-// 64-256 threads a block, 96 gave the bench's band (about 95 voxels a block)
-// its shortest iterations.
-constexpr int kPersistThreads = 96;
-constexpr int kPersistWarps = kPersistThreads / 32;
-constexpr int kPersistBlocksPerSM = 1;
+// - Before the barrier a group only votes on the two facts that the verdict
+//   carries; its statistics are summed while the block waits and committed
+//   after it.
+//
+// What bounds it: the latency of an iteration's chain -- psi loads from L2
+// (the barrier's acquire empties L1), the parts of group_update, the barrier.
+// Four groups per SM: 128 voxels a round, the bench's band (14.7 k voxels, 97
+// per SM) in one round.  All 128 registers of 512 threads: at 96 and 80 the
+// compiler keeps loop state in memory, which costs a trip to L2 after every
+// barrier.  Measured at 256^3 (14.7 k band voxels, 200 iterations): 4.8 us an
+// iteration (0.95 ms a solve) against 8.9 us (1.79 ms) with one thread per
+// voxel in 96-thread blocks, where 97 voxels took two rounds; 64^3 (1.7 k band
+// voxels): 3.4 us against 6.0 us.
+// Blocks: a band of few voxels uses fewer, one per kPersistPerBlock voxels (a
+// barrier of fewer blocks is shorter, a block of fewer voxels no faster).
+// Whole 64^3 frames with 24, 32, 48, 64, 96 and 128 voxels a block: 1788, 1783,
+// 1807, 1849, 2003 and 2129 us for three.
+constexpr int kPersistGroups = 4;
+constexpr int kPersistThreads = kGroupThreads * kPersistGroups;
+constexpr unsigned kPersistPerBlock = 32;
 
-// Compacts the voxels `next` (>= 0 on the threads that carry one) of the
-// block into out[base...] (capacity entries), with no atomic; returns how
-// many there were.  The first kPersistThreads entries of out (the next
-// iteration's first round) also go to first[].  Every thread of the block
-// calls it.
-__device__ __forceinline__ unsigned block_compact(int next, int *__restrict__ out, unsigned base,
-                                                  unsigned capacity, int *first) {
-  __shared__ unsigned s_w[kPersistWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool has = next >= 0;
-  const unsigned ball = __ballot_sync(0xffffffffu, has);
-  if (lane == 0) s_w[warp] = (unsigned)__popc(ball);
-  __syncthreads();
-  unsigned before = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < kPersistWarps; ++w) {
-    const unsigned c = s_w[w];
-    before += w < warp ? c : 0u;
-    total += c;
+struct PersistShared {
+  GroupShared group[kPersistGroups];
+  int first[kPersistGroups][32];   // the next iteration's first round
+  unsigned k0[kPersistGroups];     // each group's slice of the lists: [k0, k0 + per)
+  unsigned n[kPersistGroups];      // voxels each group carries
+  unsigned carried[kPersistGroups];
+  bool fail[kPersistGroups], open[kPersistGroups];
+  bool shell[kPersistGroups];      // the slice holds voxels of the grid's outer shell
+  GroupStats stats[kPersistGroups];
+  BlockStats part[kPersistGroups];
+  FusedArgs args;                  // for group_shell
+  bool ok, any_open, any_fail;     // the barrier's verdict
+  unsigned long long seen[2];      // grid_verdict's record of the two barrier words
+};
+
+// Compacts a warp's carried voxels `next` (-1: none) into the group's slice of
+// `out`, after those already there.
+__device__ __forceinline__ void group_carry(int next, int lane, int *__restrict__ out, unsigned per, PersistShared &sh,
+                                            int g) {
+  const unsigned ball = __ballot_sync(0xffffffffu, next >= 0), carried = sh.carried[g];
+  if (next >= 0) {
+    const unsigned pos = carried + (unsigned)__popc(ball & ((1u << lane) - 1u));
+    if (KF_IN_BOUNDS(pos, per, KF_SITE_BAND_APPEND)) out[sh.k0[g] + pos] = next;
+    if (pos < 32u) sh.first[g][pos] = next;
   }
-  if (has) {
-    const unsigned pos = base + before + (unsigned)__popc(ball & ((1u << lane) - 1u));
-    if (KF_IN_BOUNDS(pos, capacity, KF_SITE_BAND_APPEND)) out[pos] = next;
-    if (pos < (unsigned)kPersistThreads) first[pos] = next;
-  }
-  __syncthreads();  // s_w is written again by the next call
-  return total;
+  __syncwarp();
+  if (lane == 0) sh.carried[g] = carried + (unsigned)__popc(ball);
+  __syncwarp();
 }
 
-// Iteration `it` of the block's n voxels in[0..n) (carried ones to out,
-// n updated); false when the kernel must end (the iteration was the last,
-// a barrier wait gave up, or the next iteration is gated).  The entries
-// in[0..kPersistThreads) are read from first[] (from `in` at it == 0), so
-// that a thread's first voxel is known as soon as the barrier lets it go.
-// seen: grid_sync_verdict's record of this iteration's barrier word.
-__device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, int it, bool last,
-                                                          const int *__restrict__ in, int *__restrict__ out,
-                                                          unsigned &n, unsigned capacity, GridSync *sync,
-                                                          unsigned long long limit_ns, int *first,
-                                                          unsigned long long &seen) {
-  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned k0 = lane * kPersistWarps + warp;  // this thread's voxel of round 0
-  const int v0 = k0 < n ? (it == 0 ? __ldcg(in + k0) : first[k0]) : -1;
-  const unsigned rounds = (n + kPersistThreads - 1) / kPersistThreads;
-  float maxd = 0.f;
-  double energy = 0.0;
-  unsigned active = 0, carried = 0;
+// Iteration `it` of the group's voxels, the entries [k0, k0 + n) of lst0 (lst1
+// in odd iterations); carried ones go to the other list.  False when the
+// kernel must end (the iteration was the last, a barrier wait gave up, or the
+// next iteration is gated).  The first 32 entries are read from first[] (from
+// lst0 at it == 0).  What a group keeps from one round to the next is in shared
+// memory, not in registers (group_shell).
+__device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, int it, bool last, int *lst0, int *lst1,
+                                                          unsigned per, GridSync *sync, unsigned nblocks,
+                                                          unsigned long long limit_ns, PersistShared &sh) {
+  // group g on warps 4g..4g+3, its roles rotated by g so that every scheduler
+  // has each role once; part 3 is on a warp of another scheduler in each group
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = warp / kGroupWarps, w = (warp + g) % kGroupWarps, last_role = (2 * g) % kGroupWarps;
+  const bool odd = it & 1;
+  GroupStep t;
+  t.active = false;
   bool diverged = false;
-  for (unsigned r = 0; r < rounds; ++r) {
-    const unsigned k = r * kPersistThreads + k0;
-    int next = -1;
-    if (k < n) {
-      const int v = r == 0 ? v0 : __ldcg(in + k);
-      next = update_band_voxel<false, kPsiL1>(a, v, v, maxd, energy, active, diverged);
+  int v = (unsigned)lane < sh.n[g] ? (it == 0 ? __ldcg(lst0 + sh.k0[g] + lane) : sh.first[g][lane]) : -1;
+  for (unsigned k = 0; k < sh.n[g]; k += 32) {
+    if (w == last_role && k > 0) group_count(a, t, sh.stats[g], lane);  // the round before
+    const int next = group_update<kPsiL1>(a, odd, v, v, sh.group[g], g, w, last_role, lane, t, diverged);
+    v = k + 32 + lane < sh.n[g] ? __ldcg((odd ? lst1 : lst0) + sh.k0[g] + k + 32 + lane) : -1;
+    if (w == last_role) group_carry(next, lane, odd ? lst0 : lst1, per, sh, g);
+  }
+  if (w == last_role) {
+    const bool fail = __any_sync(0xffffffffu, diverged);
+    if (lane == 0) sh.fail[g] = fail;
+    __syncwarp();
+    if (sh.shell[g] || a.dp.early_exit) {
+      group_count(a, t, sh.stats[g], lane);
+      t.active = false;
     }
-    carried += block_compact(next, out, carried, capacity, first);
+    if (sh.shell[g]) {
+      for (unsigned k = 0; k < sh.n[g]; k += 32) {
+        const int i = k + lane < sh.n[g] ? __ldcg((odd ? lst1 : lst0) + sh.k0[g] + k + lane) : -1;
+        group_carry(group_shell<kPsiL1>(&sh.args, odd, i, i, &sh.stats[g], &sh.fail[g]), lane, odd ? lst0 : lst1, per,
+                    sh, g);
+      }
+    }
+    // (the verdict needs the largest step only then)
+    const bool open = a.dp.early_exit && __any_sync(0xffffffffu, sh.stats[g].maxd[lane] > (float)a.dp.threshold);
+    if (lane == 0) sh.open[g] = open;
   }
-  n = carried;
-  BlockStats b{};  // the block's totals, on thread 0
-  reduce_iter_stats<kPersistThreads>(a.st + it, active, maxd, energy, diverged, &b);
-  if (last) {
-    if (threadIdx.x == 0) commit_iter_stats(a.st + it, b);
-    return false;
+  __syncthreads();
+  if (threadIdx.x == 96 && !last) {
+    bool open = false, fail = false;
+#pragma unroll
+    for (int k = 0; k < kPersistGroups; ++k) {
+      open |= sh.open[k];
+      fail |= sh.fail[k];
+    }
+    // the gate of iteration it + 1 (iteration_gated): no block diverged, and
+    // with early_exit some block moved psi by more than the threshold
+    sh.ok = grid_verdict(sync, nblocks, limit_ns, it, open, fail, sh.seen[it & 1], sh.any_open, sh.any_fail);
   }
-  // the gate of iteration it + 1 (iteration_gated): no block diverged, and
-  // with early_exit some block moved psi by more than the threshold; the
-  // statistics are committed while the barrier completes
-  bool any_open = false, any_fail = false;
-  if (!grid_sync_verdict(sync, gridDim.x, limit_ns, it, b.max_delta > (float)a.dp.threshold, b.diverged, seen,
-                         any_open, any_fail, [&] { commit_iter_stats(a.st + it, b); })) {
+  if (w == last_role) {  // while the polling thread (of another warp) waits
+    group_count(a, t, sh.stats[g], lane);
+    float maxd = sh.stats[g].maxd[lane];
+    double energy = sh.stats[g].energy[lane];
+    unsigned active = sh.stats[g].active[lane];
+    sh.stats[g].maxd[lane] = 0.f;
+    sh.stats[g].energy[lane] = 0.0;
+    sh.stats[g].active[lane] = 0u;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      energy += __shfl_xor_sync(0xffffffffu, energy, o);
+      maxd = fmaxf(maxd, __shfl_xor_sync(0xffffffffu, maxd, o));
+      active += __shfl_xor_sync(0xffffffffu, active, o);
+    }
+    if (lane == 0) {
+      sh.part[g] = BlockStats{energy, active, maxd, sh.fail[g]};
+      sh.n[g] = sh.carried[g];
+      sh.carried[g] = 0u;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 64) {
+    BlockStats b = sh.part[0];
+#pragma unroll
+    for (int k = 1; k < kPersistGroups; ++k) {
+      b.energy += sh.part[k].energy;
+      b.active += sh.part[k].active;
+      b.max_delta = fmaxf(b.max_delta, sh.part[k].max_delta);
+      b.diverged |= sh.part[k].diverged;
+    }
+    commit_iter_stats(a.st + it, b);
+  }
+  if (last) return false;
+  if (!sh.ok) {
     if (threadIdx.x == 0) a.st[0].timeout = 1;
     return false;
   }
-  if (any_fail || (a.dp.early_exit && !any_open)) {
+  if (sh.any_fail || (a.dp.early_exit && !sh.any_open)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) a.st[it + 1].skipped = 1;
     return false;
   }
   return true;
 }
 
-// even: psi in the primary planes, out to the second; odd: the reverse.
+// a: psi in the primary planes, out to the second (iteration 0, then every
+// other one; the others read the second planes and write the primary ones).
 // The band list of the dense first pass is lst0[0, st[0].list).  touched
 // (or NULL): a copy of that list and its length, the only voxels whose psi
-// the solve can change (the iterations overwrite lst0).
-__global__ void __launch_bounds__(kPersistThreads, kPersistBlocksPerSM)
-    k_band_persistent(FusedArgs even, FusedArgs odd, int *lst0, int *lst1, int iterations, GridSync *sync,
-                      unsigned long long limit_ns, int *touched, unsigned *touched_n) {
-  const unsigned nq = __ldcg(&even.st[0].list);
-  const unsigned per = (nq + gridDim.x - 1) / gridDim.x;  // this block's slice [k0, k0 + per)
-  const unsigned k0 = min(blockIdx.x * per, nq);
-  unsigned n = min(k0 + per, nq) - k0;
-  if (touched) {
-    for (unsigned j = threadIdx.x; j < n; j += kPersistThreads) touched[k0 + j] = __ldcg(lst0 + k0 + j);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *touched_n = nq;
+// the solve can change (the iterations overwrite lst0).  per_block: the
+// fewest band voxels worth a block; a smaller band leaves the last blocks
+// without any, and they end at once.
+__global__ void __launch_bounds__(kPersistThreads, 1)
+    k_band_persistent(FusedArgs a, int *lst0, int *lst1, int iterations, GridSync *sync,
+                      unsigned long long limit_ns, int *touched, unsigned *touched_n, unsigned per_block) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  PersistShared &sh = *reinterpret_cast<PersistShared *>(smem);
+  const unsigned nq = __ldcg(&a.st[0].list);
+  const unsigned nblocks = max(min(gridDim.x, (nq + per_block - 1) / per_block), 1u);
+  if (blockIdx.x >= nblocks) return;
+  const unsigned groups = nblocks * kPersistGroups;
+  const unsigned per = (nq + groups - 1) / groups;  // a group's slice
+  if (threadIdx.x == 0) {
+    sh.args = a;
+    sh.seen[0] = sh.seen[1] = 0;
   }
-  __shared__ int s_first[kPersistThreads];
-  unsigned long long seen_even = 0, seen_odd = 0;
-  for (int it = 0; it < iterations; it += 2) {
-    if (!persistent_band_iteration(even, it, it + 1 == iterations, lst0 + k0, lst1 + k0, n, per, sync, limit_ns,
-                                   s_first, seen_even))
-      return;
-    if (it + 1 < iterations && !persistent_band_iteration(odd, it + 1, it + 2 == iterations, lst1 + k0, lst0 + k0,
-                                                          n, per, sync, limit_ns, s_first, seen_odd))
-      return;
+  if (threadIdx.x < kPersistGroups) {
+    const unsigned k0 = min((blockIdx.x * kPersistGroups + threadIdx.x) * per, nq);
+    sh.k0[threadIdx.x] = k0;
+    sh.n[threadIdx.x] = min(k0 + per, nq) - k0;
+    sh.carried[threadIdx.x] = 0u;
+    sh.shell[threadIdx.x] = false;
   }
+  if (threadIdx.x < 32 * kPersistGroups) {
+    GroupStats &st = sh.stats[threadIdx.x / 32];
+    st.energy[threadIdx.x % 32] = 0.0;
+    st.maxd[threadIdx.x % 32] = 0.f;
+    st.active[threadIdx.x % 32] = 0u;
+  }
+  if (touched && blockIdx.x == 0 && threadIdx.x == 0) *touched_n = nq;
+  __syncthreads();
+  const int g = threadIdx.x / kGroupThreads;
+  for (unsigned j = threadIdx.x % kGroupThreads; j < sh.n[g]; j += kGroupThreads) {
+    const unsigned k = sh.k0[g] + j;
+    const int v = __ldcg(lst0 + k);
+    if (touched) touched[k] = v;
+    int x, y, z;
+    voxel_xyz(a.dp, v, x, y, z);
+    if (!interior_voxel(a.dp, x, y, z)) sh.shell[g] = true;
+  }
+  __syncthreads();
+  for (int it = 0; it < iterations; ++it)
+    if (!persistent_band_iteration(a, it, it + 1 == iterations, lst0, lst1, per, sync, nblocks, limit_ns, sh)) return;
 }
 
 // In-place update after the last iteration: psi(list[k]) = entry k of the
@@ -625,18 +712,15 @@ static void launch_iterations(kf_grid live, kf_grid can, kf_field psi, const Dev
                                                         (float *)in[2]);
     } else {
       if (it == 0) k_fused_stream<true><<<grid, block, 0, s>>>(a, lst[0], nullptr, nullptr);
-      if (dp.trust) {
-        k_fused_band<true, false, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1]);
-        k_trust_fix<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], false, next_rows);
-      } else {
-        k_fused_band<true, false><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1]);
-      }
+      // (with the trust-region step; without it the solver is k_band_persistent)
+      k_fused_band<true, false, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1]);
+      k_trust_fix<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], false, next_rows);
     }
   }
 }
 
 // Resident blocks per SM of k_band_persistent on the current device (at most
-// kPersistBlocksPerSM): the cooperative launch must fit on the GPU at once.
+// one): the cooperative launch must fit on the GPU at once.
 // Its shared-memory carveout is kBesideSolveCarveout (kf_internal.h), the
 // one of the kernels that run beside it.
 static int persistent_blocks_per_sm() {
@@ -647,10 +731,12 @@ static int persistent_blocks_per_sm() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   if (!cached[dev]) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_band_persistent, kPersistThreads, 0) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute((const void *)k_band_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(PersistShared)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_band_persistent, kPersistThreads,
+                                                      sizeof(PersistShared)) != cudaSuccess)
       return 0;
-    cached[dev] = std::min(n, kPersistBlocksPerSM);
+    cached[dev] = std::min(n, 1);
   }
   return cached[dev];
 }
@@ -677,13 +763,6 @@ static int launch_band_persistent(kf_grid live, kf_grid can, kf_field psi, const
   even.ox = (float *)psi->q[0];
   even.oy = (float *)psi->q[1];
   even.oz = (float *)psi->q[2];
-  FusedArgs odd = even;
-  odd.ix = (const float *)psi->q[0];
-  odd.iy = (const float *)psi->q[1];
-  odd.iz = (const float *)psi->q[2];
-  odd.ox = (float *)psi->p[0];
-  odd.oy = (float *)psi->p[1];
-  odd.oz = (float *)psi->p[2];
   int *lst0 = psi->band, *lst1 = psi->band + dp.count;
   int *touched = nullptr;
   unsigned *touched_n = nullptr;
@@ -703,10 +782,11 @@ static int launch_band_persistent(kf_grid live, kf_grid can, kf_field psi, const
   GridSync *gs = static_cast<GridSync *>(sync);
   unsigned long long limit = kf_wait_limit_ns();
   int iters = iterations;
-  void *args[] = {&even, &odd, &lst0, &lst1, &iters, &gs, &limit, &touched, &touched_n};
+  unsigned per_block = kPersistPerBlock;
+  void *args[] = {&even, &lst0, &lst1, &iters, &gs, &limit, &touched, &touched_n, &per_block};
   KF_CHECK_CUDA(cudaLaunchCooperativeKernel((const void *)k_band_persistent,
-                                            dim3((unsigned)(kf_num_sms() * bps)), dim3(kPersistThreads), args, 0,
-                                            s));
+                                            dim3((unsigned)(kf_num_sms() * bps)), dim3(kPersistThreads), args,
+                                            sizeof(PersistShared), s));
   if (p_zero) {
     psi->p_state = psi->q_state = kPsiRecorded;
     psi->side_recorded = false;

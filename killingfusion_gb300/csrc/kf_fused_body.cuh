@@ -48,6 +48,8 @@ struct FusedArgs {
   DevParams dp;
   // float copies of the parameters
   float h, alpha, omega_k, gamma_k, omega_s, clamp, eps, voxel, oob, band_hi, band_lo;
+  float inv2h, inv4hh;  // 1 / 2h and 1 / 4h^2
+  int64_t row, plane;   // voxels from one to the next along y and along z
 };
 
 // Float arithmetic with every rounding spelled out: fm, fa and fsb never
@@ -63,11 +65,13 @@ __device__ __forceinline__ float ff(float a, float b, float c) { return __fmaf_r
 
 // utils.h:6-25 in float with explicit roundings: a * (1 - t) + b * t, along
 // x, then y, then z.
-__device__ __forceinline__ float lerp1f(float a, float b, float t) { return ff(b, t, fm(a, fsb(1.f, t))); }
+// u = 1 - t, t each axis's fraction.
+__device__ __forceinline__ float lerp1f(float a, float b, float u, float t) { return ff(b, t, fm(a, u)); }
 __device__ __forceinline__ float lerp3f(const float v[8], float x, float y, float z) {
-  const float s = lerp1f(lerp1f(v[0], v[1], x), lerp1f(v[2], v[3], x), y);
-  const float t = lerp1f(lerp1f(v[4], v[5], x), lerp1f(v[6], v[7], x), y);
-  return lerp1f(s, t, z);
+  const float ux = fsb(1.f, x), uy = fsb(1.f, y), uz = fsb(1.f, z);
+  const float s = lerp1f(lerp1f(v[0], v[1], ux, x), lerp1f(v[2], v[3], ux, x), uy, y);
+  const float t = lerp1f(lerp1f(v[4], v[5], ux, x), lerp1f(v[6], v[7], ux, x), uy, y);
+  return lerp1f(s, t, uz, z);
 }
 
 __device__ __forceinline__ float phi_at(const FusedArgs &a, int x, int y, int z) {
@@ -298,7 +302,7 @@ __device__ __forceinline__ void gradient_lane(const FusedArgs &a, int x, int y, 
   const float s = phi_tri(a, fsb(fa(fa((float)x, c0[0]), 0.5f), 0.5f), fsb(fa(fa((float)y, c0[1]), 0.5f), 0.5f),
                           fsb(fa(fa((float)z, c0[2]), 0.5f), 0.5f));
   const float cv = __ldg(a.can + idx);
-  const float inv2h = 1.f / fm(2.f, h), inv4hh = 1.f / fm(fm(4.f, h), h);
+  const float inv2h = a.inv2h, inv4hh = a.inv4hh;
   // SDF.cpp:726-744: (f(p + h e_k) - f(p - h e_k)) / 2h
   const float g[3] = {fm(fsb(f[1], f[2]), inv2h), fm(fsb(f[3], f[4]), inv2h), fm(fsb(f[5], f[6]), inv2h)};
   // SDF.cpp:867-881 on the same samples
@@ -349,6 +353,253 @@ __device__ __forceinline__ void gradient_lane(const FusedArgs &a, int x, int y, 
   e_out = e;
 }
 
+// ---------------------------------------------------------------------------
+// A band voxel by a group of four warps
+// ---------------------------------------------------------------------------
+// A group takes 32 voxels at a time, one per lane of each of its warps, and
+// cuts a voxel's update into parts that do not depend on one another, so that
+// little is computed twice and every rounding is gradient_lane's:
+//   part 1  roles 0-2 take one psi component each: its 20 neighbours, the
+//           Killing second differences, the cell's moments and the corner
+//           cell of the samples along that axis.  Role 3 takes the warped
+//           value at i + psi(i) and phi_can(i).
+//   part 2  the 25 cell-centre samples by the stencil they belong to, eight
+//           or nine a warp (roles 0-2), and the Killing gradient (role 3: a
+//           chain of divisions and a square root that nothing in its own warp
+//           would hide).
+//   part 3  one warp adds the terms up and steps psi.
+// The parts hand their values over in shared memory, between two barriers of
+// the group's 128 threads.
+constexpr int kGroupWarps = 4;
+constexpr int kGroupThreads = 32 * kGroupWarps;
+
+struct GroupShared {
+  // part 1's values of component c: {m0, m1, m2, m3}, {m4, m5, m6, the
+  // samples' corner cell or -1} and {-2 (xx + yy + zz), the component's
+  // shares of the divergence term}, {the row of the Jacobian, psi_c(i)}
+  float4 mom[3][2][32], kil[3][2][32];
+  // part 2's: {hxx, hyy, hzz, psi_0(i)}, {g, psi_1(i)}, {hxz, hxy, psi_2(i),
+  // yz's last sample}, {kg, the Killing term of the monitored energy}; the
+  // warped value, phi_can and yz's first samples
+  float4 out[4][32];
+  float more[4][32];
+  float spread[25][32];  // group_samples_spread's samples
+};
+
+// psi's planes of one iteration: a.ix.. read and a.ox.. written, or (odd) the
+// reverse.  Chosen where they are used, from the kernel's parameters: six
+// pointers would take twelve registers through the whole iteration.
+template <int kC>
+__device__ __forceinline__ const float *plane_in(const FusedArgs &a, bool odd) {
+  return kC == 0 ? (odd ? a.ox : a.ix) : (kC == 1 ? (odd ? a.oy : a.iy) : (odd ? a.oz : a.iz));
+}
+template <int kC>
+__device__ __forceinline__ float *plane_out(const FusedArgs &a, bool odd) {
+  return const_cast<float *>(plane_in<kC>(a, !odd));
+}
+
+// A barrier of the 128 threads of the block's group g (0..3): barrier 1 + g of
+// the block, each by its number (a number in a register would reserve all 16).
+__device__ __forceinline__ void group_sync(int g) {
+  if (g == 0)
+    asm volatile("bar.sync 1, %0;" ::"n"(kGroupThreads) : "memory");
+  else if (g == 1)
+    asm volatile("bar.sync 2, %0;" ::"n"(kGroupThreads) : "memory");
+  else if (g == 2)
+    asm volatile("bar.sync 3, %0;" ::"n"(kGroupThreads) : "memory");
+  else
+    asm volatile("bar.sync 4, %0;" ::"n"(kGroupThreads) : "memory");
+}
+
+// Part 1 of component c from its 20 neighbours v: the voxel's coordinate
+// along axis c is xc, the grid's size there nc.
+__device__ __forceinline__ void group_component(const FusedArgs &a, int c, int xc, int nc, const float v[20],
+                                                GroupShared &sh, int lane) {
+  const float h = a.h, two_h = fm(2.f, h), hh = fm(h, h), v000 = v[N000];
+  // moments of the cell [i, i+1]^3 (corner k_abc = psi(i + (a,b,c)))
+  const float k000 = v000, k100 = v[NXP], k010 = v[NYP], k110 = v[NXPYP];
+  const float k001 = v[NZP], k101 = v[NXPZP], k011 = v[NYPZP], k111 = v[N111];
+  const float sx0 = fa(fa(k000, k010), fa(k001, k011)), sx1 = fa(fa(k100, k110), fa(k101, k111));
+  const float sy0 = fa(fa(k000, k100), fa(k001, k101)), sy1 = fa(fa(k010, k110), fa(k011, k111));
+  const float sz0 = fa(fa(k000, k100), fa(k010, k110)), sz1 = fa(fa(k001, k101), fa(k011, k111));
+  float m[7];
+  m[0] = fm(0.125f, fa(sx0, sx1));
+  m[1] = fm(0.25f, fsb(sx1, sx0));
+  m[2] = fm(0.25f, fsb(sy1, sy0));
+  m[3] = fm(0.25f, fsb(sz1, sz0));
+  m[4] = fm(0.5f, fsb(fa(fsb(fsb(k110, k010), fsb(k100, k000)), fsb(k111, k011)), fsb(k101, k001)));
+  m[5] = fm(0.5f, fsb(fa(fsb(fsb(k101, k001), fsb(k100, k000)), fsb(k111, k011)), fsb(k110, k010)));
+  m[6] = fm(0.5f, fsb(fa(fsb(fsb(k011, k001), fsb(k010, k000)), fsb(k111, k101)), fsb(k110, k100)));
+  // Along axis c every sample lies within
+  // h * (2 + 2 (|m1| + |m2| + |m3|) + h (|m4| + |m5| + |m6|)) of the centre
+  // sample: the offsets are at most 2 and the products of the mixed samples'
+  // offsets are +-1.  When that interval, widened for the roundings of the
+  // positions (1e-3 voxel plus 2^-20 of the coordinate, several float ulps
+  // of it), has one truncated base and that base is inside the grid, all 25
+  // samples have it.
+  const float m1 = fabsf(m[1]) + fabsf(m[2]) + fabsf(m[3]), m2 = fabsf(m[4]) + fabsf(m[5]) + fabsf(m[6]);
+  const float ctr = fa(fa((float)xc, 0.5f), m[0]);
+  const float r = h * (2.f + 2.f * m1 + h * m2) + 1e-3f + fabsf(ctr) * 0x1p-20f;
+  const float lo = ctr - r, hi = ctr + r;
+  const int b = (int)lo;
+  const bool tight = lo >= 0.f && (int)hi == b && (unsigned)b < (unsigned)(nc - 1);
+  sh.mom[c][0][lane] = make_float4(m[0], m[1], m[2], m[3]);
+  sh.mom[c][1][lane] = make_float4(m[4], m[5], m[6], __int_as_float(tight ? b : -1));
+  // Killing second differences (DisplacementField.cpp:326-331)
+  const float xx = fm(two_h, fa(fsb(v[NXP], v000), fsb(v[NXM], v000)));
+  const float yy = fm(two_h, fa(fsb(v[NYP], v000), fsb(v[NYM], v000)));
+  const float zz = fm(two_h, fa(fsb(v[NZP], v000), fsb(v[NZM], v000)));
+  const float xy = fm(hh, fsb(fsb(v[NXPYP], v[NXPYM]), fsb(v[NXMYP], v[NXMYM])));
+  const float xz = fm(hh, fsb(fsb(v[NXPZP], v[NXPZM]), fsb(v[NXMZP], v[NXMZM])));
+  const float yz = fm(hh, fsb(fsb(v[NYPZP], v[NYPZM]), fsb(v[NYMZP], v[NYMZM])));
+  sh.kil[c][0][lane] = make_float4(fm(-2.f, fa(fa(xx, yy), zz)), c == 0 ? xx : (c == 1 ? xy : xz),
+                                   c == 0 ? xy : (c == 1 ? yy : yz), c == 0 ? xz : (c == 1 ? yz : zz));
+  sh.kil[c][1][lane] = make_float4(fm(0.5f, fsb(v[NXP], v[NXM])), fm(0.5f, fsb(v[NYP], v[NYM])),
+                                   fm(0.5f, fsb(v[NZP], v[NZM])), v000);
+}
+
+// Part 2's inputs, read back by every warp.
+struct GroupCell {
+  float base[3], m[3][7];
+  float b[3];       // the samples' corner cell (kTight)
+  float corner[8];  // and its values
+};
+
+// The position of the cell-centre sample at offset o (SDF::getDistancef at
+// i+0.5+h*o; the half voxel it adds is removed again by getDistance): psi~
+// there is the cell's trilinear form in its moments, terms with a zero
+// offset left out (at compile time where o is known then).
+__device__ __forceinline__ void group_position(const FusedArgs &a, const GroupCell &q, int o0, int o1, int o2,
+                                               float t[3]) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    float lin = 0.f, quad = 0.f;
+    if (o0) lin = ff((float)o0, q.m[c][1], lin);
+    if (o1) lin = ff((float)o1, q.m[c][2], lin);
+    if (o2) lin = ff((float)o2, q.m[c][3], lin);
+    if (o0 * o1) quad = ff((float)(o0 * o1), q.m[c][4], quad);
+    if (o0 * o2) quad = ff((float)(o0 * o2), q.m[c][5], quad);
+    if (o1 * o2) quad = ff((float)(o1 * o2), q.m[c][6], quad);
+    const int oc = c == 0 ? o0 : (c == 1 ? o1 : o2);
+    t[c] = fa(fa(q.base[c], fm(a.h, (float)oc)), ff(a.h, ff(a.h, quad, lin), q.m[c][0]));
+  }
+}
+
+// The samples of role w in the order its stencils take them: the centre, the
+// axes' +-2 and one of yz; the gradient's +-1 and two of yz; xz, xy and the last
+// of yz.
+__host__ __device__ constexpr int group_sample_id(int w, int k) {
+  constexpr signed char t[3][9] = {
+      {0, 7, 8, 9, 10, 11, 12, 22, -1}, {1, 2, 3, 4, 5, 6, 15, 21, -1}, {13, 19, 20, 14, 17, 23, 24, 18, 16}};
+  return t[w][k];
+}
+
+// The same tables for loops that are not unrolled.
+__constant__ signed char c_group_sample[3][9] = {
+    {0, 7, 8, 9, 10, 11, 12, 22, -1}, {1, 2, 3, 4, 5, 6, 15, 21, -1}, {13, 19, 20, 14, 17, 23, 24, 18, 16}};
+__constant__ signed char c_off25[25][3] = {
+    {0, 0, 0},   {1, 0, 0},   {-1, 0, 0},  {0, 1, 0},  {0, -1, 0},  {0, 0, 1},  {0, 0, -1},
+    {2, 0, 0},   {-2, 0, 0},  {0, 2, 0},   {0, -2, 0}, {0, 0, 2},   {0, 0, -2}, {1, 0, 1},
+    {-1, 0, 1},  {0, 1, 1},   {0, -1, 1},  {1, 1, 0},  {-1, 1, 0},  {-1, 0, -1}, {1, 0, -1},
+    {0, -1, -1}, {0, 1, -1},  {-1, -1, 0}, {1, -1, 0}};
+
+// Role kW's samples when those of every lane lie in one cell, whose corners
+// are in registers.
+template <int kW>
+__device__ __forceinline__ void group_samples(const FusedArgs &a, const GroupCell &q, float f[9]) {
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const int j = group_sample_id(kW, k);
+    if (j < 0) break;
+    float t[3];
+    group_position(a, q, off25_at(j, 0), off25_at(j, 1), off25_at(j, 2), t);
+    f[k] = lerp3f(q.corner, fsb(t[0], q.b[0]), fsb(t[1], q.b[1]), fsb(t[2], q.b[2]));
+  }
+}
+
+// The same when some lane's samples do not share a cell: each gathers its
+// own corners.  A loop that is not unrolled, through shared memory, so that this rarer
+// form takes no registers from the other.
+__device__ __forceinline__ void group_samples_spread(const FusedArgs &a, const GroupCell &q, int w, int lane,
+                                                     float (*spread)[32]) {
+#pragma unroll 1
+  for (int k = 0; k < 9; ++k) {
+    const int j = c_group_sample[w][k];
+    if (j < 0) break;
+    float t[3];
+    group_position(a, q, c_off25[j][0], c_off25[j][1], c_off25[j][2], t);
+    spread[j][lane] = phi_tri(a, t[0], t[1], t[2]);
+  }
+}
+
+// Part 2's stencils of role w from its samples (w: what goes with them in
+// `out`).  SDF.cpp:726-744 (the gradient's differences over 2h) and
+// SDF.cpp:867-881 (the second differences over 4h^2).
+__device__ __forceinline__ float4 group_stencils(const FusedArgs &a, int w, const float f[9]) {
+  const float inv2h = a.inv2h, inv4hh = a.inv4hh;
+  if (w == 0) {
+    const float f02 = fm(2.f, f[0]);
+    return make_float4(fm(fa(fsb(f[1], f02), f[2]), inv4hh), fm(fa(fsb(f[3], f02), f[4]), inv4hh),
+                       fm(fa(fsb(f[5], f02), f[6]), inv4hh), 0.f);
+  }
+  if (w == 1)
+    return make_float4(fm(fsb(f[0], f[1]), inv2h), fm(fsb(f[2], f[3]), inv2h), fm(fsb(f[4], f[5]), inv2h), 0.f);
+  return make_float4(fm(fsb(fsb(fa(f[0], f[1]), f[2]), f[3]), inv4hh),
+                     fm(fsb(fsb(fa(f[4], f[5]), f[6]), f[7]), inv4hh), 0.f, f[8]);
+}
+
+// The Killing gradient (x, y, z) and the Killing term of the monitored
+// energy (w) from part 1's values: damped divergence term, clamp |g| to
+// killing_clamp, /4h^2.
+__device__ __forceinline__ float4 group_killing(const FusedArgs &a, const GroupShared &sh, int lane) {
+  const float h = a.h, m2g = fm(-2.f, a.gamma_k);
+  const float4 k0 = sh.kil[0][0][lane], k1 = sh.kil[1][0][lane], k2 = sh.kil[2][0][lane];
+  float kg[3];
+  kg[0] = ff(m2g, fa(fa(fa(0.f, k0.y), k1.y), k2.y), k0.x);
+  kg[1] = ff(m2g, fa(fa(fa(0.f, k0.z), k1.z), k2.z), k1.x);
+  kg[2] = ff(m2g, fa(fa(fa(0.f, k0.w), k1.w), k2.w), k2.x);
+  const float nrm = sqrtf(ff(kg[2], kg[2], ff(kg[1], kg[1], fm(kg[0], kg[0]))));
+  const float sc = nrm > a.clamp ? a.clamp / nrm : 1.f;
+  const float den = fm(fm(4.f, h), h);
+  const float4 j0 = sh.kil[0][1][lane], j1 = sh.kil[1][1][lane], j2 = sh.kil[2][1][lane];
+  const float J[3][3] = {{j0.x, j0.y, j0.z}, {j1.x, j1.y, j1.z}, {j2.x, j2.y, j2.z}};
+  float fr = 0.f, tr = 0.f;
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      fr = ff(J[p][k], J[p][k], fr);
+      tr = ff(J[p][k], J[k][p], tr);
+    }
+  return make_float4(fm(kg[0], sc) / den, fm(kg[1], sc) / den, fm(kg[2], sc) / den, ff(a.gamma_k, tr, fr));
+}
+
+// A group's voxel between the step and its statistics (part 3).
+struct GroupStep {
+  float d[3], r, gn, ke;  // the step; the terms its monitored energy is made of
+  bool active;
+};
+
+// The monitored energy of the step's voxel and |d|, added to the statistics.
+__device__ __forceinline__ void group_statistics(const FusedArgs &a, const GroupStep &t, float &maxd, double &energy,
+                                                 unsigned &active) {
+  if (!t.active) return;
+  float e = 0.f;
+  if (a.dp.use_data) e = ff(fm(0.5f, t.r), t.r, e);
+  if (a.dp.use_killing) e = ff(a.omega_k, t.ke, e);
+  if (a.dp.use_levelset) {
+    const float r = fsb(t.gn / a.voxel, 1.f);
+    e = ff(fm(fm(a.omega_s, 0.5f), r), r, e);
+  }
+  maxd = fmaxf(maxd, sqrtf(ff(t.d[2], t.d[2], ff(t.d[1], t.d[1], fm(t.d[0], t.d[0])))));
+  energy += e;
+  ++active;
+}
+
+__device__ __forceinline__ bool interior_voxel(const DevParams &dp, int x, int y, int z) {
+  return x >= 1 && y >= 1 && z >= 1 && x <= dp.nx - 2 && y <= dp.ny - 2 && z <= dp.nz - 2;
+}
+
 // A psi value read as load_psi<kLoad> reads it: the element type of psi
 // views in kernels that write psi themselves.  Same layout as float.
 template <int kLoad>
@@ -379,11 +630,17 @@ __device__ __noinline__ void gradient_generic(const FusedArgs &a, int x, int y, 
   e_out = monitor_energy(px, py, pz, dp.nx, dp.ny, dp.nz, x, y, z, s_out, cv.at(x, y, z), gd, dp);
 }
 
+// i / d for 0 <= i < 2^31 as (umulhi(i, mul) + i) >> shift (Granlund and
+// Montgomery's division by an invariant integer): 3 instructions where a
+// 32-bit division by a register takes about 20.
+__device__ __forceinline__ unsigned divided(unsigned i, const KfDivisor &d) {
+  return (__umulhi(i, d.mul) + i) >> d.shift;
+}
+
 __device__ __forceinline__ void voxel_xyz(const DevParams &dp, int i, int &x, int &y, int &z) {
-  const unsigned plane = (unsigned)dp.nx * (unsigned)dp.ny;
-  z = (int)((unsigned)i / plane);
-  const unsigned r = (unsigned)i - (unsigned)z * plane;
-  y = (int)(r / (unsigned)dp.nx);
+  z = (int)divided((unsigned)i, dp.by_plane);
+  const unsigned r = (unsigned)i - (unsigned)z * ((unsigned)dp.nx * (unsigned)dp.ny);
+  y = (int)divided(r, dp.by_row);
   x = (int)(r - (unsigned)y * (unsigned)dp.nx);
 }
 
@@ -468,29 +725,28 @@ __device__ __forceinline__ void stream_tile(const FusedArgs &a, int bx, int by, 
 constexpr int kFlatGroups = 2;
 constexpr int kFlatVoxels = kThreads * kFlatGroups * 4;
 
-__device__ __forceinline__ void flat_test(const FusedArgs &a, int64_t i, float qx, float qy, float qz, float ph,
-                                          int *queue, int *qn, unsigned &moved, int bit) {
+__device__ __forceinline__ void flat_test(const FusedArgs &a, float qx, float qy, float qz, float ph,
+                                          unsigned &moved, unsigned &hit, int bit) {
   if (qx != 0.f || qy != 0.f || qz != 0.f)
     moved |= 1u << bit;
-  else if (in_band(ph, a.band_hi, a.band_lo)) {
-    const int q = atomicAdd(qn, 1);
-    if (KF_IN_BOUNDS(q, kFlatVoxels + 4, KF_SITE_STREAM_QUEUE)) queue[q] = (int)i;
-  }
+  else if (in_band(ph, a.band_hi, a.band_lo))
+    hit |= 1u << bit;
 }
 
 // kCheck: the run is only tested, its band voxels are counted in *count and
 // not listed (the split schedule's runs without band voxels, where a band
 // voxel would break an invariant of the solver).  kPsiZero: psi is zero at
 // every voxel (nothing of it is read), so the test reads phi_live alone.
+// A run's voxels are listed in index order: the lanes of a band pass then
+// hold neighbours along x, whose psi and phi share cache lines (in the order
+// of an atomic counter, 25 lanes' loads touched about 20 lines).
 template <bool kPassThrough, bool kCheck = false, bool kPsiZero = false>
 __device__ __forceinline__ void stream_flat(const FusedArgs &a, int64_t run, int *__restrict__ list,
                                             unsigned *count, int2 *__restrict__ range = nullptr) {
-  __shared__ int queue[kFlatVoxels + 4];
-  __shared__ int qn, qbase;
+  __shared__ unsigned s_warp[kThreads / 32];
+  __shared__ unsigned s_base;
   const DevParams &dp = a.dp;
   const int tid = threadIdx.x;
-  if (tid == 0) qn = 0;
-  __syncthreads();
   const int64_t n4 = dp.count >> 2;
   const float4 *ix = reinterpret_cast<const float4 *>(a.ix), *iy = reinterpret_cast<const float4 *>(a.iy),
                *iz = reinterpret_cast<const float4 *>(a.iz), *lv = reinterpret_cast<const float4 *>(a.live);
@@ -506,15 +762,15 @@ __device__ __forceinline__ void stream_flat(const FusedArgs &a, int64_t run, int
     pz[g] = read_psi ? __ldcs(iz + q[g]) : zero;
     ph[g] = ok ? __ldg(lv + q[g]) : zero;
   }
-  unsigned moved = 0;  // bit 4g + e: element e of group g has moved
+  // bit 4g + e: element e of group g has moved / is in the band
+  unsigned moved = 0, hit = 0;
 #pragma unroll
   for (int g = 0; g < kFlatGroups; ++g) {
     if (q[g] >= n4) continue;
-    const int64_t i = 4 * q[g];
-    flat_test(a, i, px[g].x, py[g].x, pz[g].x, ph[g].x, queue, &qn, moved, 4 * g);
-    flat_test(a, i + 1, px[g].y, py[g].y, pz[g].y, ph[g].y, queue, &qn, moved, 4 * g + 1);
-    flat_test(a, i + 2, px[g].z, py[g].z, pz[g].z, ph[g].z, queue, &qn, moved, 4 * g + 2);
-    flat_test(a, i + 3, px[g].w, py[g].w, pz[g].w, ph[g].w, queue, &qn, moved, 4 * g + 3);
+    flat_test(a, px[g].x, py[g].x, pz[g].x, ph[g].x, moved, hit, 4 * g);
+    flat_test(a, px[g].y, py[g].y, pz[g].y, ph[g].y, moved, hit, 4 * g + 1);
+    flat_test(a, px[g].z, py[g].z, pz[g].z, ph[g].z, moved, hit, 4 * g + 2);
+    flat_test(a, px[g].w, py[g].w, pz[g].w, ph[g].w, moved, hit, 4 * g + 3);
     if (kPassThrough) {
       __stcs(reinterpret_cast<float4 *>(a.ox) + q[g], px[g]);
       __stcs(reinterpret_cast<float4 *>(a.oy) + q[g], py[g]);
@@ -525,43 +781,70 @@ __device__ __forceinline__ void stream_flat(const FusedArgs &a, int64_t run, int
   if (run == 0 && tid < (int)(dp.count & 3)) {
     const int64_t i = 4 * n4 + tid;
     const float qx = kPsiZero ? 0.f : a.ix[i], qy = kPsiZero ? 0.f : a.iy[i], qz = kPsiZero ? 0.f : a.iz[i];
-    flat_test(a, i, qx, qy, qz, __ldg(a.live + i), queue, &qn, moved, 4 * kFlatGroups);
+    flat_test(a, qx, qy, qz, __ldg(a.live + i), moved, hit, 4 * kFlatGroups);
     if (kPassThrough) {
       a.ox[i] = qx;
       a.oy[i] = qy;
       a.oz[i] = qz;
     }
   }
+  // the voxel of a thread's bit
+  const auto voxel = [&](int bit) -> int64_t {
+    return bit < 4 * kFlatGroups ? 4 * (run * (kThreads * kFlatGroups) + (bit >> 2) * kThreads + tid) + (bit & 3)
+                                 : 4 * n4 + tid;
+  };
   // voxels that have moved: the warped value is a trilinear gather
   while (moved) {
     const int bit = __ffs(moved) - 1;
     moved &= moved - 1;
-    const int64_t i = bit < 4 * kFlatGroups
-                          ? 4 * (run * (kThreads * kFlatGroups) + (bit >> 2) * kThreads + tid) + (bit & 3)
-                          : 4 * n4 + tid;
-    const unsigned plane = (unsigned)dp.nx * (unsigned)dp.ny, ui = (unsigned)i;
-    const int z = (int)(ui / plane);
-    const unsigned r = ui - (unsigned)z * plane;
-    const int y = (int)(r / (unsigned)dp.nx);
-    const int x = (int)(r - (unsigned)y * (unsigned)dp.nx);
+    const int64_t i = voxel(bit);
+    int x, y, z;
+    voxel_xyz(dp, (int)i, x, y, z);
     const float s = warped_value(a, x, y, z, a.ix[i], a.iy[i], a.iz[i]);
-    if (in_band(s, a.band_hi, a.band_lo)) {
-      const int q = atomicAdd(&qn, 1);
-      if (KF_IN_BOUNDS(q, kFlatVoxels + 4, KF_SITE_STREAM_QUEUE)) queue[q] = (int)i;
-    }
+    if (in_band(s, a.band_hi, a.band_lo)) hit |= 1u << bit;
   }
-  __syncthreads();
   if (kCheck) {
-    if (tid == 0 && qn) atomicAdd(count, (unsigned)qn);
+    if (hit) atomicAdd(count, (unsigned)__popc(hit));
     return;
   }
-  if (tid == 0 && qn) qbase = (int)atomicAdd(count, (unsigned)qn);
+  if (!__syncthreads_or(hit != 0u)) {
+    if (range && tid == 0) *range = make_int2(0, 0);
+    return;
+  }
+  // one scan of the three counts (group 0, group 1, ragged end), packed
+  static_assert(kFlatGroups == 2, "two groups are packed");
+  const unsigned mine = (unsigned)__popc(hit & 15u) | (unsigned)__popc(hit >> 4 & 15u) << 12 | (hit >> 8) << 24;
+  const int lane = tid & 31, warp = tid >> 5;
+  unsigned incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) s_warp[warp] = incl;
   __syncthreads();
-  for (int k = tid; k < min(qn, kFlatVoxels + 4); k += kThreads)
-    if (KF_IN_BOUNDS(qbase + k, dp.count, KF_SITE_STREAM_LIST)) list[qbase + k] = queue[k];
+  unsigned before = incl - mine, total = 0;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) {
+    const unsigned c = s_warp[w];
+    before += w < warp ? c : 0u;
+    total += c;
+  }
+  const unsigned n0 = total & 0xfffu, n1 = total >> 12 & 0xfffu, n = n0 + n1 + (total >> 24);
+  if (tid == 0) s_base = atomicAdd(count, n);
+  __syncthreads();
+  const unsigned base = s_base;
+  unsigned at[3] = {before & 0xfffu, n0 + (before >> 12 & 0xfffu), n0 + n1 + (before >> 24)};
+#pragma unroll
+  for (int g = 0; g < 3; ++g) {
+    for (unsigned h = g < 2 ? hit >> (4 * g) & 15u : hit >> 8; h; h &= h - 1) {
+      const unsigned pos = base + at[g]++;
+      if (KF_IN_BOUNDS(pos, dp.count, KF_SITE_STREAM_LIST)) list[pos] = (int)voxel(4 * g + __ffs(h) - 1);
+    }
+  }
   // where this run's band voxels sit in the list (for the next iteration's
   // write-back of their new psi)
-  if (range && tid == 0) *range = make_int2(qn ? qbase : 0, qn);
+  if (range && tid == 0) *range = make_int2((int)base, (int)n);
 }
 
 // Appends the voxels `next` (>= 0 on the threads that carry one) of the
@@ -619,6 +902,38 @@ __device__ __noinline__ bool trust_step_f(const FusedArgs &a, int x, int y, int 
   return ok;
 }
 
+// Steps band voxel i, whose warped value is s, monitored energy en, psi c0
+// and step d: writes its new psi to entry `slot` of the output planes,
+// accumulates the statistics and returns the voxel for the next iteration's
+// list (-1 if it left the band).
+template <bool kTrust>
+__device__ __forceinline__ int settle_band_voxel(const FusedArgs &a, int i, int slot, int x, int y, int z, float s,
+                                                 float en, const float c0[3], float d[3], float &maxd, double &energy,
+                                                 unsigned &active, bool &diverged) {
+  const DevParams &dp = a.dp;
+  int next = -1;
+  if (in_band(s, a.band_hi, a.band_lo)) {
+    if (!isfinite(c0[0]) || !isfinite(c0[1]) || !isfinite(c0[2])) diverged = true;
+    if (kTrust && !trust_step_f(a, x, y, z, i, c0, d)) {
+      // this voxel and the rest of its row keep psi (k_trust_fix)
+      atomicMin(a.rows + (z * dp.ny + y), x);
+      d[0] = d[1] = d[2] = 0.f;
+    }
+    a.ox[slot] = c0[0] + d[0];
+    a.oy[slot] = c0[1] + d[1];
+    a.oz[slot] = c0[2] + d[2];
+    maxd = fmaxf(maxd, sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0])))));
+    energy += en;
+    ++active;
+    next = i;
+  } else {  // left the band: its psi is final, settle the output buffer
+    a.ox[slot] = c0[0];
+    a.oy[slot] = c0[1];
+    a.oz[slot] = c0[2];
+  }
+  return next;
+}
+
 // Update band voxel i (one thread) and write its new psi to entry `slot` of
 // the output planes (slot == i for ping-pong buffers; the voxel's list
 // position for in-place updates).  The voxel is re-tested with its warped
@@ -647,26 +962,202 @@ __device__ __forceinline__ int update_band_voxel(const FusedArgs &a, int i, int 
     c0[1] = kLoad == kPsiReadOnly ? a.iy[i] : load_psi<kLoad>(a.iy + i);
     c0[2] = kLoad == kPsiReadOnly ? a.iz[i] : load_psi<kLoad>(a.iz + i);
   }
-  int next = -1;
-  if (in_band(s, a.band_hi, a.band_lo)) {
-    if (!isfinite(c0[0]) || !isfinite(c0[1]) || !isfinite(c0[2])) diverged = true;
-    if (kTrust && !trust_step_f(a, x, y, z, i, c0, d)) {
-      // this voxel and the rest of its row keep psi (k_trust_fix)
-      atomicMin(a.rows + (z * dp.ny + y), x);
-      d[0] = d[1] = d[2] = 0.f;
+  return settle_band_voxel<kTrust>(a, i, slot, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
+}
+
+// Updates the voxels i (-1: none) of the lanes of group g, as
+// update_band_voxel does for one: every thread of the group calls it, in role
+// w, with its lane's voxel, whose new psi goes to entry `slot` of the output
+// planes.  Part 3 and its results (the voxel for the next iteration's list,
+// or -1; the step for group_statistics; whether psi(i) is finite) are role
+// `last`'s; the other warps return -1.
+// Voxels of the outer shell are left alone (group_shell).
+template <int kLoad>
+__device__ __forceinline__ int group_update(const FusedArgs &a, bool odd, int i, int slot, GroupShared &sh, int g,
+                                            int w, int last, int lane, GroupStep &t, bool &diverged) {
+  const DevParams &dp = a.dp;
+  t.active = false;
+  bool have = i >= 0;
+  if (have && (!KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST) || !KF_IN_BOUNDS(slot, dp.count, KF_SITE_BAND_LIST)))
+    have = false;
+  int x = 0, y = 0, z = 0;
+  if (have) voxel_xyz(dp, i, x, y, z);
+  const bool interior = have && interior_voxel(dp, x, y, z);
+  float own = 0.f, can = 0.f;  // roles 0-2: psi_w(i); role 3: the warped value and phi_can(i)
+  if (interior) {
+    if (w < 3) {
+      const float *r0 = (w == 0 ? plane_in<0>(a, odd) : (w == 1 ? plane_in<1>(a, odd) : plane_in<2>(a, odd))) + i;
+      const float *yp = r0 + a.row, *ym = r0 - a.row, *zp = r0 + a.plane, *zm = r0 - a.plane;
+      const float *ypzp = zp + a.row, *ymzp = zp - a.row, *ypzm = zm + a.row, *ymzm = zm - a.row;
+      float v[20];
+#pragma unroll
+      for (int n = 0; n < 20; ++n) {
+        const int oy = nb20_off(n, 1), oz = nb20_off(n, 2);
+        const float *r = oz == 0 ? (oy == 0 ? r0 : (oy > 0 ? yp : ym))
+                                 : (oz > 0 ? (oy == 0 ? zp : (oy > 0 ? ypzp : ymzp))
+                                           : (oy == 0 ? zm : (oy > 0 ? ypzm : ymzm)));
+        v[n] = load_psi<kLoad>(r + nb20_off(n, 0));
+      }
+      own = v[N000];
+      group_component(a, w, w == 0 ? x : (w == 1 ? y : z), w == 0 ? dp.nx : (w == 1 ? dp.ny : dp.nz), v, sh, lane);
+    } else {
+      can = __ldg(a.can + i);
+      const float p0 = load_psi<kLoad>(plane_in<0>(a, odd) + i), p1 = load_psi<kLoad>(plane_in<1>(a, odd) + i),
+                  p2 = load_psi<kLoad>(plane_in<2>(a, odd) + i);
+      own = phi_tri(a, fsb(fa(fa((float)x, p0), 0.5f), 0.5f), fsb(fa(fa((float)y, p1), 0.5f), 0.5f),
+                    fsb(fa(fa((float)z, p2), 0.5f), 0.5f));
     }
-    a.ox[slot] = c0[0] + d[0];
-    a.oy[slot] = c0[1] + d[1];
-    a.oz[slot] = c0[2] + d[2];
-    maxd = fmaxf(maxd, sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0])))));
-    energy += en;
-    ++active;
-    next = i;
-  } else {  // left the band: its psi is final, settle the output buffer
-    a.ox[slot] = c0[0];
-    a.oy[slot] = c0[1];
-    a.oz[slot] = c0[2];
   }
+  group_sync(g);
+  // (the last round's `out` was read before this barrier)
+  if (w == 3) {
+    if (interior) {
+      sh.more[0][lane] = own;
+      sh.more[1][lane] = can;
+      sh.out[3][lane] = group_killing(a, sh, lane);
+    }
+  } else if (__any_sync(0xffffffffu, interior)) {
+    GroupCell q;
+    q.base[0] = fa((float)x, 0.5f);
+    q.base[1] = fa((float)y, 0.5f);
+    q.base[2] = fa((float)z, 0.5f);
+    int b[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float4 lo = sh.mom[c][0][lane], hi = sh.mom[c][1][lane];
+      q.m[c][0] = lo.x, q.m[c][1] = lo.y, q.m[c][2] = lo.z, q.m[c][3] = lo.w;
+      q.m[c][4] = hi.x, q.m[c][5] = hi.y, q.m[c][6] = hi.z;
+      b[c] = __float_as_int(hi.w);
+    }
+    const bool tight = interior && (b[0] | b[1] | b[2]) >= 0;
+    float f[9];
+    // one path per warp: the samples of every interior lane in one cell, or
+    // each sample its own corners (a warp with both kinds would run both)
+    if (__all_sync(0xffffffffu, tight || !interior)) {
+      // lanes without an interior voxel read the grid's first cell
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        b[c] = tight ? b[c] : 0;
+        q.b[c] = (float)b[c];
+      }
+      const float *l = a.live + (((unsigned)b[2] * (unsigned)dp.ny + (unsigned)b[1]) * (unsigned)dp.nx + (unsigned)b[0]);
+      const float *ly = l + a.row, *lz = l + a.plane, *lyz = lz + a.row;
+      q.corner[0] = __ldg(l);
+      q.corner[1] = __ldg(l + 1);
+      q.corner[2] = __ldg(ly);
+      q.corner[3] = __ldg(ly + 1);
+      q.corner[4] = __ldg(lz);
+      q.corner[5] = __ldg(lz + 1);
+      q.corner[6] = __ldg(lyz);
+      q.corner[7] = __ldg(lyz + 1);
+      if (w == 0)
+        group_samples<0>(a, q, f);
+      else if (w == 1)
+        group_samples<1>(a, q, f);
+      else
+        group_samples<2>(a, q, f);
+    } else {
+      if (interior) group_samples_spread(a, q, w, lane, sh.spread);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) f[k] = sh.spread[max((int)c_group_sample[w][k], 0)][lane];
+    }
+    float4 o = group_stencils(a, w, f);
+    if (w == 2)
+      o.z = own;
+    else
+      o.w = own;
+    sh.out[w][lane] = o;
+    if (w == 0) sh.more[2][lane] = f[7];
+    if (w == 1) sh.more[3][lane] = fa(f[6], f[7]);
+  }
+  group_sync(g);
+  if (w != last || !interior) return -1;
+  const float4 hd = sh.out[0][lane], gr = sh.out[1][lane], ho = sh.out[2][lane], kg = sh.out[3][lane];
+  const float c0[3] = {hd.w, gr.w, ho.z}, s = sh.more[0][lane];
+  t.ke = kg.w;
+  // KillingFusion.cpp:399-476
+  float grad[3] = {0.f, 0.f, 0.f};
+  if (dp.use_data) {
+    t.r = fsb(s, sh.more[1][lane]) / a.voxel;
+    grad[0] = ff(t.r, gr.x, grad[0]);
+    grad[1] = ff(t.r, gr.y, grad[1]);
+    grad[2] = ff(t.r, gr.z, grad[2]);
+  }
+  if (dp.use_killing) {
+    grad[0] = ff(kg.x, a.omega_k, grad[0]);
+    grad[1] = ff(kg.y, a.omega_k, grad[1]);
+    grad[2] = ff(kg.z, a.omega_k, grad[2]);
+  }
+  if (dp.use_levelset) {
+    t.gn = sqrtf(ff(gr.z, gr.z, ff(gr.y, gr.y, fm(gr.x, gr.x))));
+    const float hxz = ho.x, hxy = ho.y;
+    const float hyz = fm(fsb(fsb(sh.more[3][lane], sh.more[2][lane]), ho.w), a.inv4hh);
+    const float hg0 = ff(hxz, gr.z, ff(hxy, gr.y, fm(hd.x, gr.x)));
+    const float hg1 = ff(hyz, gr.z, ff(hd.y, gr.y, fm(hxy, gr.x)));
+    const float hg2 = ff(hd.z, gr.z, ff(hyz, gr.y, fm(hxz, gr.x)));
+    const float f = fm(fsb(t.gn, 1.f) / fa(t.gn, a.eps), a.omega_s);
+    grad[0] = ff(hg0, f, grad[0]);
+    grad[1] = ff(hg1, f, grad[1]);
+    grad[2] = ff(hg2, f, grad[2]);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) t.d[k] = fm(-a.alpha, grad[k]);
+  t.active = in_band(s, a.band_hi, a.band_lo);
+  if (t.active && (!isfinite(c0[0]) || !isfinite(c0[1]) || !isfinite(c0[2]))) diverged = true;
+  // a voxel that left the band keeps psi: settle the output buffer
+  plane_out<0>(a, odd)[slot] = t.active ? c0[0] + t.d[0] : c0[0];
+  plane_out<1>(a, odd)[slot] = t.active ? c0[1] + t.d[1] : c0[1];
+  plane_out<2>(a, odd)[slot] = t.active ? c0[2] + t.d[2] : c0[2];
+  return t.active ? i : -1;
+}
+
+// A lane's statistics of an iteration, in shared memory.
+struct GroupStats {
+  double energy[32];
+  float maxd[32];
+  unsigned active[32];
+};
+
+// Adds the step t of a lane's voxel to its statistics.
+__device__ __forceinline__ void group_count(const FusedArgs &a, const GroupStep &t, GroupStats &st, int lane) {
+  float maxd = st.maxd[lane];
+  double energy = st.energy[lane];
+  unsigned active = st.active[lane];
+  group_statistics(a, t, maxd, energy, active);
+  st.maxd[lane] = maxd;
+  st.energy[lane] = energy;
+  st.active[lane] = active;
+}
+
+// The voxels of the outer shell among a warp's i (-1: none), one a lane, their
+// new psi to entry `slot`, with their statistics (st, *diverged).  Out of line, and its callers keep next to
+// nothing in registers across it: a value that has to survive a call is
+// kept in memory for good, and after a grid barrier (whose acquire empties L1)
+// every such load goes to L2.  args, st and diverged: in shared memory.
+template <int kLoad>
+__device__ __noinline__ int group_shell(const FusedArgs *args, bool odd, int i, int slot, GroupStats *st, bool *diverged) {
+  if (i < 0 || !KF_IN_BOUNDS(i, args->dp.count, KF_SITE_BAND_LIST) ||
+      !KF_IN_BOUNDS(slot, args->dp.count, KF_SITE_BAND_LIST))
+    return -1;
+  int x, y, z;
+  voxel_xyz(args->dp, i, x, y, z);
+  if (interior_voxel(args->dp, x, y, z)) return -1;
+  FusedArgs a = *args;
+  a.ix = plane_in<0>(*args, odd), a.iy = plane_in<1>(*args, odd), a.iz = plane_in<2>(*args, odd);
+  a.ox = plane_out<0>(*args, odd), a.oy = plane_out<1>(*args, odd), a.oz = plane_out<2>(*args, odd);
+  float d[3], s, en;
+  gradient_generic<kLoad>(a, x, y, z, d, s, en);
+  const float c0[3] = {load_psi<kLoad>(a.ix + i), load_psi<kLoad>(a.iy + i), load_psi<kLoad>(a.iz + i)};
+  float m = 0.f;
+  double e = 0.0;
+  unsigned n = 0;
+  bool div = false;
+  const int next = settle_band_voxel<false>(a, i, slot, x, y, z, s, en, c0, d, m, e, n, div);
+  const int lane = threadIdx.x & 31;
+  st->maxd[lane] = fmaxf(st->maxd[lane], m);
+  st->energy[lane] += e;
+  st->active[lane] += n;
+  if (div) *diverged = true;
   return next;
 }
 
@@ -678,6 +1169,10 @@ FusedArgs make_args(kf_grid live, kf_grid can, const DevParams &dp, IterStats *s
   a.st = st;
   a.dp = dp;
   a.h = (float)dp.delta_size;
+  a.row = dp.nx;
+  a.plane = (int64_t)dp.nx * dp.ny;
+  a.inv2h = 1.f / (2.f * a.h);
+  a.inv4hh = 1.f / ((4.f * a.h) * a.h);
   a.alpha = (float)dp.alpha;
   a.omega_k = (float)dp.omega_k;
   a.gamma_k = (float)dp.gamma_k;

@@ -29,7 +29,7 @@ struct GridSync {
   unsigned pad_;
   int timed_out;   // set by the first block whose wait gave up
   int where;       // the barrier (iteration) at which it gave up
-  unsigned long long word[2];  // grid_sync_verdict's arrivals, by barrier parity
+  unsigned long long word[2];  // grid_verdict's arrivals, by barrier parity
 };
 
 __device__ __forceinline__ unsigned long long kf_globaltimer_ns() {
@@ -70,8 +70,10 @@ __device__ __forceinline__ bool kf_bounded_poll(GridSync *g, unsigned long long 
   }
   unsigned long long t0 = 0;
   for (int spin = 0;; ++spin) {
-    if (done(load())) return !*timed_out;
-    if (*timed_out) return false;
+    // both loads are in flight together: a poll is one round trip to L2
+    const int gave_up = *timed_out;
+    if (done(load())) return !gave_up;
+    if (gave_up) return false;
     // the first polls run back to back (a barrier normally completes
     // within a few microseconds); then sleep between polls and watch
     // the clock
@@ -105,47 +107,39 @@ __device__ __forceinline__ bool grid_sync(GridSync *g, unsigned nblocks, unsigne
   return s_ok != 0;
 }
 
-// The same barrier, whose arrival also carries two facts about the block's
-// iteration: they come back with the barrier, in the round trip of its last
-// poll, where reading them from memory after the barrier would take one
-// more.  Barrier b uses word[b % 2]; a block adds
+// The same barrier for one thread of each block, whose arrival also carries
+// two facts about the block's iteration: they come back with the barrier, in
+// the round trip of its last poll, where reading them from memory after the
+// barrier would take one more.  Barrier b uses word[b % 2]; a block adds
 //   1 + (kVerdictOpen if `open`) + (kVerdictFail if `fail`)
 // (bits 0-31 count arrivals, 32-47 and 48-63 the blocks with each fact),
-// and thread 0 keeps in `seen` the word's value when its previous barrier
+// and the thread keeps in `seen` the word's value when its previous barrier
 // completed.  The increase since then is barrier b's alone: no block
 // arrives at barrier b + 2 before every block has arrived at b + 1, and a
 // block reads the word of barrier b only before its own arrival at b + 1.
 // The barrier is complete when the increase counts nblocks arrivals
-// (nblocks < 2^16); *any_open and *any_fail then tell whether some block
-// had each fact.  `after_arrive` runs on thread 0 between its arrival and
-// its wait (writes that no block reads before the kernel ends).
+// (nblocks < 2^16); any_open and any_fail then tell whether some block
+// had each fact.  The block synchronises (__syncthreads) before the call, so
+// that its writes of the iteration precede the arrival, and after it, so
+// that no thread reads the others' before the wait is over; between the two
+// its other threads may do work that no block waits for.
 constexpr unsigned long long kVerdictOpen = 1ull << 32;
 constexpr unsigned long long kVerdictFail = 1ull << 48;
 
-template <typename AfterArrive>
-__device__ __forceinline__ bool grid_sync_verdict(GridSync *g, unsigned nblocks, unsigned long long limit_ns,
-                                                  int where, bool open, bool fail, unsigned long long &seen,
-                                                  bool &any_open, bool &any_fail, AfterArrive after_arrive) {
-  __shared__ int s_ok, s_open, s_fail;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long *w = &g->word[where & 1];
-    kf_red_release_add64(w, 1ull + (open ? kVerdictOpen : 0ull) + (fail ? kVerdictFail : 0ull));
-    after_arrive();
-    unsigned long long inc = 0;
-    const bool ok = kf_bounded_poll(
-        g, limit_ns, where, [&] { return kf_ld_acquire64(w); },
-        [&](unsigned long long v) {
-          inc = v - seen;
-          return (unsigned)inc == nblocks;
-        });
-    seen += inc;
-    s_ok = ok;
-    s_open = (inc >> 32 & 0xffffu) != 0;
-    s_fail = (inc >> 48) != 0;
-  }
-  __syncthreads();
-  any_open = s_open != 0;
-  any_fail = s_fail != 0;
-  return s_ok != 0;
+__device__ __forceinline__ bool grid_verdict(GridSync *g, unsigned nblocks, unsigned long long limit_ns, int where,
+                                             bool open, bool fail, unsigned long long &seen, bool &any_open,
+                                             bool &any_fail) {
+  unsigned long long *w = &g->word[where & 1];
+  kf_red_release_add64(w, 1ull + (open ? kVerdictOpen : 0ull) + (fail ? kVerdictFail : 0ull));
+  unsigned long long inc = 0;
+  const bool ok = kf_bounded_poll(
+      g, limit_ns, where, [&] { return kf_ld_acquire64(w); },
+      [&](unsigned long long v) {
+        inc = v - seen;
+        return (unsigned)inc == nblocks;
+      });
+  seen += inc;
+  any_open = (inc >> 32 & 0xffffu) != 0;
+  any_fail = (inc >> 48) != 0;
+  return ok;
 }

@@ -122,6 +122,18 @@ inline cudaStream_t kf_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 // ---------------------------------------------------------------------------
 // device-side parameter block (all thresholds precomputed on the host)
 // ---------------------------------------------------------------------------
+// A divisor d, 1 <= d < 2^31, of dividends below 2^31: with shift =
+// ceil(log2 d) and mul = floor(2^32 (2^shift - d) / d) + 1, i / d is
+// (umulhi(i, mul) + i) >> shift.
+struct KfDivisor {
+  unsigned mul, shift;
+};
+inline KfDivisor kf_divisor(unsigned d) {
+  unsigned s = 0;
+  while ((1ull << s) < d) ++s;
+  return KfDivisor{(unsigned)((((1ull << s) - d) << 32) / d + 1), s};
+}
+
 struct DevParams {
   int nx, ny, nz;
   int64_t count;
@@ -141,6 +153,7 @@ struct DevParams {
   int trust;             // the trust-region step applies: use_trust with the
                          // data term alone (KillingFusion.cpp:289)
   int pad_;
+  KfDivisor by_row, by_plane;  // nx and nx ny
 };
 
 DevParams kf_make_dev_params(const int n[3], const kf_params *p);
