@@ -903,61 +903,277 @@ __global__ void __launch_bounds__(kBlock) k_fuse_warped(float *__restrict__ phi1
 // ---------------------------------------------------------------------------
 // float64 replay of the Jacobi psi update (KillingFusion.cpp:248-352)
 // ---------------------------------------------------------------------------
+// A voxel outside the band keeps psi, so its band test keeps failing: one dense
+// pass (k_exact_first) lists the band and copies the other voxels' psi to the
+// second buffer, and each iteration (k_exact_band) takes the voxels that the
+// one before handed on.
+
+// The band test of the first iteration: lists the band (st[0].list counts
+// it); psi of the other voxels goes to the output buffer too.
+__global__ void __launch_bounds__(kBlock) k_exact_first(PhiView<double> live, PsiView<double, double> fin,
+                                                        double *__restrict__ ox, double *__restrict__ oy,
+                                                        double *__restrict__ oz, DevParams dp, IterStats *st,
+                                                        int *__restrict__ list) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  bool active = false;
+  if (i < dp.count) {
+    int x, y, z;
+    voxel_xyz(i, dp.nx, dp.ny, x, y, z);
+    active = in_band(warped_distance(live, fin, x, y, z), dp.band_hi, -dp.unknown_clip);
+    if (!active) {
+      ox[i] = fin.px[i] + 0.0;
+      oy[i] = fin.py[i] + 0.0;
+      oz[i] = fin.pz[i] + 0.0;
+    }
+  }
+  const unsigned ball = __ballot_sync(0xffffffffu, active);
+  if (!ball) return;
+  const int lane = threadIdx.x & 31;
+  unsigned base = 0;
+  if (lane == 0) base = atomicAdd(&st[0].list, (unsigned)__popc(ball));
+  base = __shfl_sync(0xffffffffu, base, 0) + (unsigned)__popc(ball & ((1u << lane) - 1u));
+  if (active && KF_IN_BOUNDS(base, dp.count, KF_SITE_STREAM_LIST)) list[base] = (int)i;
+}
+
+// Iteration `iter` over the listed voxels, up to kExactVoxels at a time per
+// CTA (one CTA per SM).  The 44 psi samples of a voxel (25 at the cell centre, each
+// followed by its phi_live sample, and 19 of the Killing stencil) are
+// independent: one thread each.  What comes after them is cut into the
+// entries, components and voxels it has, in the reference's operation order.
+// Voxels still in the band go to list_out (st[iter + 1].list).
 // With dp.trust each step goes through trust_step; a voxel whose step
 // failed keeps its psi and records its x in rows[z * ny + y] (the smallest
 // such x of the row wins), for k_exact_trust_rows.
-__global__ void __launch_bounds__(kBlock) k_exact_step(PhiView<double> live, PhiView<double> can,
-                                                       PsiView<double, double> fin,
-                                                       double *__restrict__ ox,
-                                                       double *__restrict__ oy,
-                                                       double *__restrict__ oz, DevParams dp,
-                                                       IterStats *st, int iter, int *__restrict__ rows) {
+//
+// What bounds it: float64 arithmetic, about 4000 operations a voxel at two a
+// cycle and SM; a warp's instruction costs the same with one lane active as
+// with 32, so the band is dealt out evenly, the same number of voxels to
+// every SM, and no part runs on a lane or two.  One thread per voxel (1.7 k
+// band voxels at 64^3 in 53 warps, clustered in a few CTAs of the dense grid)
+// took 410 us an iteration at 64^3.
+constexpr int kExactVoxels = 16;
+constexpr int kExactSamples = 44;
+constexpr int kExactThreads = kExactVoxels * kExactSamples;  // 22 warps
+
+// The cell-centre offsets (units of h): the gradient's +-e_k, then the 19 of
+// kHessOff.
+__device__ __constant__ static const signed char kGradOff[6][3] = {{1, 0, 0},  {-1, 0, 0}, {0, 1, 0},
+                                                                  {0, -1, 0}, {0, 0, 1},  {0, 0, -1}};
+
+// A Killing sample of psi, at the voxel (x, y, z) + o, where o is zero along
+// some axis: psi_sample's lerps along it have the fraction 0, a (1 - 0) + b 0,
+// which is a while b is finite, and are left out then (39 of 66 float64
+// operations).  One form for every offset: a0 and a1 are the axes that stay.
+__device__ __forceinline__ void killing_sample(const PsiView<double, double> &f, int x, int y, int z, const double o[3],
+                                               const signed char off[3], double out[3]) {
+  const double p[3] = {(double)x + o[0], (double)y + o[1], (double)z + o[2]};
+  const int b[3] = {(int)p[0], (int)p[1], (int)p[2]};
+  const int a0 = off[0] ? 0 : 1, a1 = off[0] && !off[2] ? 1 : 2;  // the third axis: 3 - a0 - a1
+  double v[4][3];
+  bool finite = true;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    // corner c: bit 0 along a0, bit 1 along a1, bit 2 along the third axis
+    const int e0 = c & 1, e1 = c >> 1 & 1, e2 = c >> 2;
+    double w[3];
+    f.at(b[0] + (a0 == 0 ? e0 : e2), b[1] + (a0 == 1 ? e0 : (a1 == 1 ? e1 : e2)), b[2] + (a1 == 2 ? e1 : e2), w);
+    if (c < 4) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[c][k] = w[k];
+    } else {
+      finite = finite && isfinite(w[0]) && isfinite(w[1]) && isfinite(w[2]);
+    }
+  }
+  if (!finite) {
+    psi_sample(f, p[0], p[1], p[2], out);
+    return;
+  }
+  const double t0 = a0 == 0 ? p[0] - (double)b[0] : p[1] - (double)b[1];
+  const double t1 = a1 == 1 ? p[1] - (double)b[1] : p[2] - (double)b[2];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) out[k] = lerp1(lerp1(v[0][k], v[1][k], t0), lerp1(v[2][k], v[3][k], t0), t1);
+}
+
+__global__ void __launch_bounds__(kExactThreads, 1) k_exact_band(PhiView<double> live, PhiView<double> can,
+                                                                 PsiView<double, double> fin,
+                                                                 double *__restrict__ ox, double *__restrict__ oy,
+                                                                 double *__restrict__ oz, DevParams dp, IterStats *st,
+                                                                 int iter, const int *__restrict__ list,
+                                                                 int *__restrict__ list_out, int *__restrict__ rows) {
+  __shared__ double s_f[25][kExactVoxels];      // the cell-centre samples
+  __shared__ double s_d[kExactVoxels][19][3];   // the Killing samples
+  __shared__ double s_s[kExactVoxels];          // the warped value
+  __shared__ double s_g[9][kExactVoxels];       // gradient, then the Hessian's xx, yy, zz, xz, yz, xy
+  __shared__ double s_k[6][3][kExactVoxels];    // psi's second differences in the same order, per component
+  __shared__ double s_n[3][kExactVoxels];       // |g| - 1, |g| + eps and the norm of the Killing gradient
+  __shared__ double s_u[3][kExactVoxels];       // the Killing gradient, then the energy gradient
+  __shared__ int s_v[kExactVoxels];
   if (iteration_gated(st, iter, dp)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) st[iter].skipped = 1;
     return;
   }
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  bool active = false;
-  double dn = 0.0;
-  if (i < dp.count) {
-    int x, y, z;
-    voxel_xyz(i, dp.nx, dp.ny, x, y, z);
-    double p0 = fin.px[i], p1 = fin.py[i], p2 = fin.pz[i];
-    double s = warped_distance(live, fin, x, y, z);
-    double d[3] = {0.0, 0.0, 0.0};
-    if (in_band(s, dp.band_hi, -dp.unknown_clip)) {
-      active = true;
-      TParams<double> tp(dp);
-      double g[3], u[3];
-      energy_gradient(live, can, fin, tp, x, y, z, g);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) u[k] = -tp.alpha * g[k];
-      const double c[3] = {p0, p1, p2};
-      if (dp.trust && !trust_step(live, can.at(x, y, z), s, x, y, z, c, g, tp.alpha, u)) {
-        atomicMin(rows + ((int64_t)z * dp.ny + y), x);
-      } else {
-        // the update field starts at zero (KillingFusion.cpp:256, 316)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) d[k] = d[k] + u[k];
-      }
-      if (!isfinite(p0) || !isfinite(p1) || !isfinite(p2)) st[iter].diverged = 1;
-      dn = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+  const TParams<double> tp(dp);
+  const double h = tp.delta_size;
+  const unsigned n = st[iter].list;
+  const unsigned per = min(max((n + gridDim.x - 1) / gridDim.x, 1u), (unsigned)kExactVoxels);
+  const int tid = threadIdx.x;
+  for (unsigned k0 = blockIdx.x * per; k0 < n; k0 += gridDim.x * per) {
+    const int m = (int)min(n - k0, per);
+    if (tid < m) {
+      const int v = list[k0 + tid];
+      s_v[tid] = KF_IN_BOUNDS(v, dp.count, KF_SITE_BAND_LIST) ? v : -1;
     }
-    ox[i] = p0 + d[0];
-    oy[i] = p1 + d[1];
-    oz[i] = p2 + d[2];
-  }
-  unsigned ballot = __ballot_sync(0xffffffffu, active);
-  float m = (float)dn;
+    __syncthreads();
+    // the samples: 25 m at the cell centre, 19 m of the Killing stencil, m
+    // warped values
+    for (int t = tid; t < (kExactSamples + 1) * m; t += kExactThreads) {
+      const bool centre = t < 25 * m, killing = !centre && t < kExactSamples * m;
+      const int vox = centre ? t / 25 : (killing ? (t - 25 * m) / 19 : t - kExactSamples * m);
+      const int j = centre ? t % 25 : (t - 25 * m) % 19;
+      const int i = s_v[vox];
+      if (i < 0) continue;
+      int x, y, z;
+      voxel_xyz(i, dp.nx, dp.ny, x, y, z);
+      if (!centre && !killing) {
+        s_s[vox] = warped_distance(live, fin, x, y, z);
+        continue;
+      }
+      const signed char *off = centre && j < 6 ? kGradOff[j] : kHessOff[centre ? j - 6 : j];
+      const double o[3] = {h * (double)off[0], h * (double)off[1], h * (double)off[2]};
+      double d[3];
+      if (centre) {
+        const double p[3] = {((double)x + 0.5) + o[0], ((double)y + 0.5) + o[1], ((double)z + 0.5) + o[2]};
+        psi_sample(fin, p[0], p[1], p[2], d);
+        s_f[j][vox] = phi_sample(live, (p[0] + d[0]) + 0.5, (p[1] + d[1]) + 0.5, (p[2] + d[2]) + 0.5);
+      } else {
+        killing_sample(fin, x, y, z, o, off, d);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && ballot) {
-    atomicAdd(&st[iter].active, (unsigned)__popc(ballot));
-    atomicMax(&st[iter].max_delta, __float_as_uint(m));
+        for (int q = 0; q < 3; ++q) s_d[vox][j][q] = d[q];
+      }
+    }
+    __syncthreads();
+    // distance_gradient and distance_hessian, an entry a thread; the second
+    // differences of killing_gradient, a component's a thread
+    for (int t = tid; t < 12 * m; t += kExactThreads) {
+      const int v = t % m, q = t / m;
+      if (q < 3) {
+        s_g[q][v] = (s_f[2 * q][v] - s_f[2 * q + 1][v]) / (2.0 * h);
+      } else if (q < 9) {
+        // hess_assemble's xx, yy, zz (samples 1 and 2, 3 and 4, 5 and 6), then
+        // xz, yz, xy (7 + 13 - 14 - 8, 9 + 15 - 16 - 10, 11 + 17 - 18 - 12)
+        const int e = q - 3;
+        const double(*f)[kExactVoxels] = s_f + 6;
+        const double H = e < 3 ? (f[1 + 2 * e][v] - 2.0 * f[0][v] + f[2 + 2 * e][v])
+                               : (f[1 + 2 * e][v] + f[7 + 2 * e][v] - f[8 + 2 * e][v] - f[2 + 2 * e][v]);
+        s_g[q][v] = H / (4.0 * h * h);
+      } else {
+        const int c = q - 9;
+        const double(*d)[3] = s_d[v];
+#pragma unroll
+        for (int e = 0; e < 6; ++e)
+          s_k[e][c][v] = e < 3 ? (d[1 + 2 * e][c] - 2.0 * d[0][c] + d[2 + 2 * e][c])
+                               : (d[1 + 2 * e][c] + d[7 + 2 * e][c] - d[8 + 2 * e][c] - d[2 + 2 * e][c]);
+      }
+    }
+    __syncthreads();
+    // the norms (levelset_gradient, killing_assemble)
+    for (int t = tid; t < 64; t += kExactThreads) {
+      const int v = t & 31;
+      if (v >= m) continue;
+      if (t < 32) {
+        const double g[3] = {s_g[0][v], s_g[1][v], s_g[2][v]};
+        const double nrm = norm3(g);
+        s_n[0][v] = nrm - 1.0;
+        s_n[1][v] = nrm + tp.epsilon;
+      } else {
+        enum { XX, YY, ZZ, XZ, YZ, XY };
+        const double div[3] = {s_k[XX][0][v] + s_k[XY][1][v] + s_k[XZ][2][v],
+                               s_k[XY][0][v] + s_k[YY][1][v] + s_k[YZ][2][v],
+                               s_k[XZ][0][v] + s_k[YZ][1][v] + s_k[ZZ][2][v]};
+        const double gk = -2.0 * tp.gamma_k;
+        double kg[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          kg[c] = -2.0 * (s_k[XX][c][v] + s_k[YY][c][v] + s_k[ZZ][c][v]) + gk * div[c];
+          s_u[c][v] = kg[c];
+        }
+        s_n[2][v] = norm3(kg);
+      }
+    }
+    __syncthreads();
+    // a component of the energy gradient a thread (energy_gradient)
+    for (int t = tid; t < 3 * m; t += kExactThreads) {
+      const int v = t % m, r = t / m, i = s_v[v];
+      if (i < 0) continue;
+      const double g0 = s_g[0][v], g1 = s_g[1][v], g2 = s_g[2][v];
+      double dg = 0.0, kg = 0.0, lg = 0.0;
+      if (tp.use_data) {
+        int x, y, z;
+        voxel_xyz(i, dp.nx, dp.ny, x, y, z);
+        dg = ((s_s[v] - can.at(x, y, z)) / tp.voxel_size) * (r == 0 ? g0 : (r == 1 ? g1 : g2));
+      }
+      if (tp.use_killing) {
+        double k = s_u[r][v];
+        if (s_n[2][v] > tp.killing_clamp) k = (k / s_n[2][v]) * tp.killing_clamp;
+        kg = (k / (4.0 * h * h)) * tp.omega_k;
+      }
+      if (tp.use_levelset) {
+        // row r of the Hessian
+        const double h0 = r == 0 ? s_g[3][v] : (r == 1 ? s_g[8][v] : s_g[6][v]);
+        const double h1 = r == 0 ? s_g[8][v] : (r == 1 ? s_g[4][v] : s_g[7][v]);
+        const double h2 = r == 0 ? s_g[6][v] : (r == 1 ? s_g[7][v] : s_g[5][v]);
+        lg = (((h0 * g0 + h1 * g1 + h2 * g2) * s_n[0][v]) / s_n[1][v]) * tp.omega_s;
+      }
+      s_u[r][v] = (dg + kg) + lg;
+    }
+    __syncthreads();
+    if (tid < 32) {
+      bool active = false;
+      float md = 0.f;
+      const int i = tid < m ? s_v[tid] : -1;
+      if (i >= 0) {
+        int x, y, z;
+        voxel_xyz(i, dp.nx, dp.ny, x, y, z);
+        const double c[3] = {fin.px[i], fin.py[i], fin.pz[i]}, s = s_s[tid];
+        double d[3] = {0.0, 0.0, 0.0};
+        active = in_band(s, dp.band_hi, -dp.unknown_clip);
+        if (active) {
+          double g[3], u[3];
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            g[q] = s_u[q][tid];
+            u[q] = -tp.alpha * g[q];
+          }
+          if (dp.trust && !trust_step(live, can.at(x, y, z), s, x, y, z, c, g, tp.alpha, u)) {
+            atomicMin(rows + ((int64_t)z * dp.ny + y), x);
+          } else {
+            // the update field starts at zero (KillingFusion.cpp:256, 316)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) d[q] = d[q] + u[q];
+          }
+          if (!isfinite(c[0]) || !isfinite(c[1]) || !isfinite(c[2])) st[iter].diverged = 1;
+          md = (float)sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+        }
+        ox[i] = c[0] + d[0];
+        oy[i] = c[1] + d[1];
+        oz[i] = c[2] + d[2];
+      }
+      const unsigned ball = __ballot_sync(0xffffffffu, active);
+      md = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(md)));
+      unsigned base = 0;
+      if (tid == 0 && ball) {
+        atomicAdd(&st[iter].active, (unsigned)__popc(ball));
+        atomicMax(&st[iter].max_delta, __float_as_uint(md));
+        base = atomicAdd(&st[iter + 1].list, (unsigned)__popc(ball));
+      }
+      base = __shfl_sync(0xffffffffu, base, 0) + (unsigned)__popc(ball & ((1u << tid) - 1u));
+      if (active && KF_IN_BOUNDS(base, dp.count, KF_SITE_BAND_APPEND)) list_out[base] = i;
+    }
+    __syncthreads();  // this chunk's values are read before the next one's
   }
 }
 
-// Trust-region step, after k_exact_step: the voxels of a row from its first
+// Trust-region step, after k_exact_band: the voxels of a row from its first
 // failed step on keep their psi (the reference's break out of the x loop,
 // KillingFusion.cpp:312-313).  One warp per row; the warp clears the row's
 // entry for the next iteration.
@@ -1136,18 +1352,23 @@ int kf_solve_exact(kf_grid live, kf_grid can, kf_field psi, const DevParams &dp,
     if (rc) return rc;
     KF_CHECK_CUDA(cudaMemsetAsync(rows, 0x7f, (size_t)nrows * sizeof(int), s));
   }
+  rc = kf_field_band_list(psi, &psi->band);
+  if (rc) return rc;
+  int *lists[2] = {psi->band, psi->band + dp.count};
+  const unsigned grid = (unsigned)kf_num_sms();
   for (int it = 0; it < iterations; ++it) {
     void **in = buf[it & 1], **out = buf[(it + 1) & 1];
     PsiView<double, double> fin{(const double *)in[0], (const double *)in[1],
                                 (const double *)in[2], dp.nx, dp.ny, dp.nz};
-    k_exact_step<<<blocks_for(dp.count), kBlock, 0, s>>>(lv, cv, fin, (double *)out[0],
-                                                         (double *)out[1], (double *)out[2], dp,
-                                                         st, it, rows);
+    double *o[3] = {(double *)out[0], (double *)out[1], (double *)out[2]};
+    if (it == 0)
+      k_exact_first<<<blocks_for(dp.count), kBlock, 0, s>>>(lv, fin, o[0], o[1], o[2], dp, st, lists[0]);
+    k_exact_band<<<grid, kExactThreads, 0, s>>>(lv, cv, fin, o[0], o[1], o[2], dp, st, it, lists[it & 1],
+                                                lists[(it + 1) & 1], rows);
     if (dp.trust)
       k_exact_trust_rows<<<(unsigned)(((int64_t)nrows * 32 + kBlock - 1) / kBlock), kBlock, 0, s>>>(
-          (const double *)in[0], (const double *)in[1], (const double *)in[2], (double *)out[0],
-          (double *)out[1], (double *)out[2], rows, dp.nx, nrows);
-    KF_CHECK_LAUNCH("k_exact_step");
+          (const double *)in[0], (const double *)in[1], (const double *)in[2], o[0], o[1], o[2], rows, dp.nx, nrows);
+    KF_CHECK_LAUNCH("float64 solve");
   }
   return KF_OK;
 }
