@@ -499,73 +499,177 @@ __global__ void __launch_bounds__(kThreads) k_trust_fix(FusedArgs a, const int *
 }
 
 // KillingFusion::computeDisplacementField, default per-voxel schedule
-// (KillingFusion.cpp:353-396), for the listed voxels (inside the symmetric
-// band) of one colour (x&1) | (y&1)<<1 | (z&1)<<2: each is taken by one
-// thread, which steps its psi in place -- a.ix and a.ox are the same planes --
-// until the step or the gradient is at most the threshold or max_iters steps
-// were taken.  A voxel's gradient reads psi only in its 3x3x3 neighbourhood,
-// where no other voxel has its colour, so its neighbours stay fixed while it
-// iterates, as in the reference's sequential loop, and the result does not
-// depend on scheduling.  Statistics: record 0 voxels (list, from the band
-// pass), last step, last monitored energy, divergence; record 1 voxels that
-// hit the cap (active) and the most steps of one voxel (list).
-__global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_pervoxel(FusedArgs a, const int *__restrict__ list,
-                                                            int max_iters, int color) {
+// (KillingFusion.cpp:353-396), in eight colours (x&1) | (y&1)<<1 | (z&1)<<2.
+// The listed voxels of a colour (inside the symmetric band) step their psi in
+// place -- a.ix and a.ox are the same planes -- until the step or the
+// gradient is at most the threshold or max_iters steps were taken.  A
+// voxel's gradient reads psi only in its 3x3x3 neighbourhood, where no other
+// voxel has its colour, so its neighbours stay fixed while it iterates, as
+// in the reference's sequential loop, and the result does not depend on
+// scheduling.
+
+// The dense pass's list sorted into one list per colour: counts[c] voxels
+// from the sum of counts[0..c) on.  Two launches, kFill = false to count
+// (counts are zero before), then kFill = true to write (cursors are).
+template <bool kFill>
+__global__ void __launch_bounds__(kThreads) k_colour_lists(FusedArgs a, const int *__restrict__ list,
+                                                          unsigned *__restrict__ counts,
+                                                          unsigned *__restrict__ cursors, int *__restrict__ out) {
+  const unsigned nq = a.st[0].list;
+  const unsigned lane = threadIdx.x & 31;
+  // whole warps loop together
+  for (unsigned k = blockIdx.x * kThreads + threadIdx.x; k - lane < nq; k += gridDim.x * kThreads) {
+    int v = k < nq ? list[k] : -1;
+    if (v >= 0 && !KF_IN_BOUNDS(v, a.dp.count, KF_SITE_BAND_LIST)) v = -1;
+    int x = 0, y = 0, z = 0;
+    if (v >= 0) voxel_xyz(a.dp, v, x, y, z);
+    const int colour = v >= 0 ? (x & 1) | (y & 1) << 1 | (z & 1) << 2 : 8;
+    const unsigned same = __match_any_sync(0xffffffffu, colour);
+    if (v < 0) continue;
+    const int leader = __ffs(same) - 1;
+    unsigned base = 0;
+    if ((int)lane == leader) base = atomicAdd((kFill ? cursors : counts) + colour, (unsigned)__popc(same));
+    if (kFill) {
+      base = __shfl_sync(same, base, leader) + (unsigned)__popc(same & ((1u << lane) - 1u));
+      for (int c = 0; c < colour; ++c) base += counts[c];
+      if (KF_IN_BOUNDS(base, a.dp.count, KF_SITE_BAND_APPEND)) out[base] = v;
+    }
+  }
+}
+
+// Whether the step d of a voxel, its iter-th before it, was its last
+// (KillingFusion.cpp:374-394); n: its new psi, which *diverged reports when it
+// is not finite.
+__device__ __forceinline__ bool pervoxel_done(const FusedArgs &a, float dn, const float n[3], int max_iters, int &iter,
+                                              bool &diverged) {
+  const float thr = (float)a.dp.threshold;
+  if (dn <= thr) return true;
+  if (!isfinite(n[0]) || !isfinite(n[1]) || !isfinite(n[2])) {
+    diverged = true;
+    return true;
+  }
+  ++iter;
+  // |gradient| = |step| / alpha
+  return !(dn / a.alpha > thr) || iter >= max_iters;
+}
+
+// A voxel of the outer shell, by one thread with the generic gradient.
+__device__ __noinline__ void pervoxel_shell(const FusedArgs *args, int i, int x, int y, int z, int max_iters,
+                                            float *dn_out, float *en_out, int *iter_out, unsigned *steps_out,
+                                            bool *diverged) {
+  const FusedArgs &a = *args;
+  int iter = 0;
+  unsigned steps = 0;
+  bool div = false;
+  while (true) {
+    float d[3], s, e;
+    gradient_generic<kPsiL2>(a, x, y, z, d, s, e);
+    const float n[3] = {__ldcg(a.ix + i) + d[0], __ldcg(a.iy + i) + d[1], __ldcg(a.iz + i) + d[2]};
+    // DisplacementField::update (DisplacementField.cpp:65-71)
+    a.ox[i] = n[0];
+    a.oy[i] = n[1];
+    a.oz[i] = n[2];
+    ++steps;
+    *dn_out = sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0]))));
+    *en_out = e;
+    if (pervoxel_done(a, *dn_out, n, max_iters, iter, div)) break;
+  }
+  *iter_out = iter;
+  *steps_out = steps;
+  if (div) *diverged = true;
+}
+
+// The voxels of one colour, one warp each (warp_step): a voxel's neighbours are
+// loaded once and its psi stays on chip until the last step, so a step costs no
+// trip to memory beyond the samples' corners (L1).
+// Statistics: record 0 voxels (list, from the dense pass), last step, last
+// monitored energy, divergence; record 1 voxels that hit the cap (active) and
+// the most steps of one voxel (list).
+// What bounds it: the chain of a step times the steps of the slowest voxel.
+// One thread per voxel of the unsorted list (7 of 8 lanes of another colour,
+// 60 psi loads a step) took 2.4 us a step.
+constexpr int kPervoxelWarps = 4;
+constexpr int kPervoxelBlocksPerSM = 4;
+
+__global__ void __launch_bounds__(32 * kPervoxelWarps, kPervoxelBlocksPerSM)
+    k_pervoxel(FusedArgs a, const int *__restrict__ list, const unsigned *__restrict__ counts, int max_iters,
+               int colour) {
+  __shared__ WarpShared s_warp[kPervoxelWarps];
+  __shared__ FusedArgs s_args;
   const DevParams &dp = a.dp;
-  const int nq = (int)a.st[0].list;
-  const float thr = (float)dp.threshold;
+  unsigned first = 0;
+  for (int c = 0; c < colour; ++c) first += counts[c];
+  const unsigned nq = counts[colour];
+  if (blockIdx.x * kPervoxelWarps >= nq) return;
+  if (threadIdx.x == 0) s_args = a;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  WarpShared &sh = s_warp[warp];
+  const WarpLane wl = warp_lane(a, lane);
+  // the same on every lane but where noted
   float maxd = 0.f;
-  double energy = 0.0;  // float64 from the per-voxel terms up
+  double energy = 0.0;  // lane 0: float64 from the per-voxel terms up
   unsigned capped = 0, most = 0;
   bool diverged = false;
-  for (int k = blockIdx.x * kLaneThreads + threadIdx.x; k < nq; k += gridDim.x * kLaneThreads) {
-    const int i = list[k];
+  for (unsigned k = blockIdx.x * kPervoxelWarps + warp; k < nq; k += gridDim.x * kPervoxelWarps) {
+    const int i = list[first + k];
     if (!KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST)) continue;
-    int x, y, z;
-    voxel_xyz(dp, i, x, y, z);
-    if (((x & 1) | (y & 1) << 1 | (z & 1) << 2) != color) continue;
-    const bool interior = x >= 1 && y >= 1 && z >= 1 && x <= dp.nx - 2 && y <= dp.ny - 2 && z <= dp.nz - 2;
-    int iter = 0;
+    int x, y, z, iter = 0;
     unsigned steps = 0;
     float dn = 0.f, en = 0.f;
-    bool div = false;
-    while (true) {
-      float d[3] = {0.f, 0.f, 0.f}, sv = 0.f, e = 0.f, c0[3] = {0.f, 0.f, 0.f};
-      if (interior) {
-        gradient_lane<kPsiL2>(a, x, y, z, i, d, sv, e, c0);
-      } else {
-        gradient_generic<kPsiL2>(a, x, y, z, d, sv, e);
-        c0[0] = __ldcg(a.ix + i);
-        c0[1] = __ldcg(a.iy + i);
-        c0[2] = __ldcg(a.iz + i);
+    voxel_xyz(dp, i, x, y, z);
+    if (interior_voxel(dp, x, y, z)) {
+      const float can = __ldg(a.can + i);
+      __syncwarp();
+      warp_neighbours<kPsiL2>(a, i, lane, wl, sh);
+      GroupStep t;
+      float n[3];
+      while (true) {
+        const float d = warp_step(a, x, y, z, can, lane, wl, sh, t);
+        if (lane < 3) sh.nb[lane][0] = sh.nb[lane][0] + d;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t.d[c] = __shfl_sync(0xffffffffu, d, c);
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 3; ++c) n[c] = sh.nb[c][0];
+        ++steps;
+        dn = sqrtf(ff(t.d[2], t.d[2], ff(t.d[1], t.d[1], fm(t.d[0], t.d[0]))));
+        if (pervoxel_done(a, dn, n, max_iters, iter, diverged)) break;
       }
-      const float n0 = c0[0] + d[0], n1 = c0[1] + d[1], n2 = c0[2] + d[2];
-      // DisplacementField::update (DisplacementField.cpp:65-71)
-      a.ox[i] = n0;
-      a.oy[i] = n1;
-      a.oz[i] = n2;
-      ++steps;
-      dn = sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0]))));
-      en = e;
-      if (dn <= thr) break;
-      if (!isfinite(n0) || !isfinite(n1) || !isfinite(n2)) {
-        div = true;
-        break;
+      if (lane == 0) {
+        // DisplacementField::update (DisplacementField.cpp:65-71): the other
+        // colours read psi in later launches only
+        a.ox[i] = n[0];
+        a.oy[i] = n[1];
+        a.oz[i] = n[2];
+        t.active = true;
+        warp_energy_term(a, sh, t);
+        float m = 0.f;
+        double e = 0.0;
+        unsigned one = 0;
+        group_statistics(a, t, m, e, one);
+        energy += e;
       }
-      ++iter;
-      // |gradient| = |step| / alpha
-      if (!(dn / a.alpha > thr) || iter >= max_iters) break;
+    } else {
+      if (lane == 0) {
+        bool div = false;
+        pervoxel_shell(&s_args, i, x, y, z, max_iters, &dn, &en, &iter, &steps, &div);
+        diverged |= div;
+        energy += en;
+      }
+      dn = __shfl_sync(0xffffffffu, dn, 0);
+      iter = __shfl_sync(0xffffffffu, iter, 0);
+      steps = __shfl_sync(0xffffffffu, steps, 0);
     }
     maxd = fmaxf(maxd, dn);
-    energy += en;
     capped += iter >= max_iters;
     most = max(most, steps);
-    diverged |= div;
   }
-  // voxels processed are counted by the band pass (record 0's list)
-  reduce_iter_stats<kLaneThreads>(a.st, 0u, maxd, energy, diverged);
-  if (capped) atomicAdd(&a.st[1].active, capped);
-  if (most) atomicMax(&a.st[1].list, most);
+  if (lane == 0) {
+    commit_iter_stats(a.st, BlockStats{energy, 0u, maxd, diverged});
+    if (capped) atomicAdd(&a.st[1].active, capped);
+    if (most) atomicMax(&a.st[1].list, most);
+  }
 }
 
 }  // namespace
@@ -879,8 +983,19 @@ int kf_solve_pervoxel(kf_grid live, kf_grid can, kf_field psi, const DevParams &
   const unsigned grid = (unsigned)std::max<int64_t>((dp.count / 4 + kThreads * kFlatGroups - 1) /
                                                         (kThreads * kFlatGroups), 1);
   k_fused_stream<false><<<grid, kThreads, 0, s>>>(a, psi->band, nullptr, nullptr);
-  for (int color = 0; color < 8; ++color)
-    k_pervoxel<<<(unsigned)kf_num_sms() * kLaneBlocksPerSM, kLaneThreads, 0, s>>>(a, psi->band, max_iters, color);
+  // the colours' counts and cursors, and their lists in the second band list
+  void *sync = nullptr;
+  rc = kf_field_sync(psi, &sync);
+  if (rc) return rc;
+  unsigned *counts = static_cast<unsigned *>(sync), *cursors = counts + 8;
+  KF_CHECK_CUDA(cudaMemsetAsync(counts, 0, 16 * sizeof(unsigned), s));
+  int *lists = psi->band + dp.count;
+  const unsigned spread = (unsigned)kf_num_sms() * 4;
+  k_colour_lists<false><<<spread, kThreads, 0, s>>>(a, psi->band, counts, cursors, lists);
+  k_colour_lists<true><<<spread, kThreads, 0, s>>>(a, psi->band, counts, cursors, lists);
+  for (int colour = 0; colour < 8; ++colour)
+    k_pervoxel<<<(unsigned)kf_num_sms() * kPervoxelBlocksPerSM, 32 * kPervoxelWarps, 0, s>>>(a, lists, counts,
+                                                                                          max_iters, colour);
   KF_CHECK_LAUNCH("per-voxel solve");
   return KF_OK;
 }

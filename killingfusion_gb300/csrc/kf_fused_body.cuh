@@ -412,9 +412,10 @@ __device__ __forceinline__ void group_sync(int g) {
 }
 
 // Part 1 of component c from its 20 neighbours v: the voxel's coordinate
-// along axis c is xc, the grid's size there nc.
-__device__ __forceinline__ void group_component(const FusedArgs &a, int c, int xc, int nc, const float v[20],
-                                                GroupShared &sh, int lane) {
+// along axis c is xc, the grid's size there nc.  mom0, mom1, kil0, kil1: as
+// GroupShared holds them.
+__device__ __forceinline__ void component_values(const FusedArgs &a, int c, int xc, int nc, const float v[20],
+                                                 float4 &mom0, float4 &mom1, float4 &kil0, float4 &kil1) {
   const float h = a.h, two_h = fm(2.f, h), hh = fm(h, h), v000 = v[N000];
   // moments of the cell [i, i+1]^3 (corner k_abc = psi(i + (a,b,c)))
   const float k000 = v000, k100 = v[NXP], k010 = v[NYP], k110 = v[NXPYP];
@@ -443,8 +444,8 @@ __device__ __forceinline__ void group_component(const FusedArgs &a, int c, int x
   const float lo = ctr - r, hi = ctr + r;
   const int b = (int)lo;
   const bool tight = lo >= 0.f && (int)hi == b && (unsigned)b < (unsigned)(nc - 1);
-  sh.mom[c][0][lane] = make_float4(m[0], m[1], m[2], m[3]);
-  sh.mom[c][1][lane] = make_float4(m[4], m[5], m[6], __int_as_float(tight ? b : -1));
+  mom0 = make_float4(m[0], m[1], m[2], m[3]);
+  mom1 = make_float4(m[4], m[5], m[6], __int_as_float(tight ? b : -1));
   // Killing second differences (DisplacementField.cpp:326-331)
   const float xx = fm(two_h, fa(fsb(v[NXP], v000), fsb(v[NXM], v000)));
   const float yy = fm(two_h, fa(fsb(v[NYP], v000), fsb(v[NYM], v000)));
@@ -452,10 +453,10 @@ __device__ __forceinline__ void group_component(const FusedArgs &a, int c, int x
   const float xy = fm(hh, fsb(fsb(v[NXPYP], v[NXPYM]), fsb(v[NXMYP], v[NXMYM])));
   const float xz = fm(hh, fsb(fsb(v[NXPZP], v[NXPZM]), fsb(v[NXMZP], v[NXMZM])));
   const float yz = fm(hh, fsb(fsb(v[NYPZP], v[NYPZM]), fsb(v[NYMZP], v[NYMZM])));
-  sh.kil[c][0][lane] = make_float4(fm(-2.f, fa(fa(xx, yy), zz)), c == 0 ? xx : (c == 1 ? xy : xz),
-                                   c == 0 ? xy : (c == 1 ? yy : yz), c == 0 ? xz : (c == 1 ? yz : zz));
-  sh.kil[c][1][lane] = make_float4(fm(0.5f, fsb(v[NXP], v[NXM])), fm(0.5f, fsb(v[NYP], v[NYM])),
-                                   fm(0.5f, fsb(v[NZP], v[NZM])), v000);
+  kil0 = make_float4(fm(-2.f, fa(fa(xx, yy), zz)), c == 0 ? xx : (c == 1 ? xy : xz),
+                     c == 0 ? xy : (c == 1 ? yy : yz), c == 0 ? xz : (c == 1 ? yz : zz));
+  kil1 = make_float4(fm(0.5f, fsb(v[NXP], v[NXM])), fm(0.5f, fsb(v[NYP], v[NYM])),
+                     fm(0.5f, fsb(v[NZP], v[NZM])), v000);
 }
 
 // Part 2's inputs, read back by every warp.
@@ -548,6 +549,20 @@ __device__ __forceinline__ float4 group_stencils(const FusedArgs &a, int w, cons
                      fm(fsb(fsb(fa(f[4], f[5]), f[6]), f[7]), inv4hh), 0.f, f[8]);
 }
 
+// The Killing term of the monitored energy from the Jacobian's rows.
+__device__ __forceinline__ float killing_energy(const FusedArgs &a, float4 j0, float4 j1, float4 j2) {
+  const float J[3][3] = {{j0.x, j0.y, j0.z}, {j1.x, j1.y, j1.z}, {j2.x, j2.y, j2.z}};
+  float fr = 0.f, tr = 0.f;
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      fr = ff(J[p][k], J[p][k], fr);
+      tr = ff(J[p][k], J[k][p], tr);
+    }
+  return ff(a.gamma_k, tr, fr);
+}
+
 // The Killing gradient (x, y, z) and the Killing term of the monitored
 // energy (w) from part 1's values: damped divergence term, clamp |g| to
 // killing_clamp, /4h^2.
@@ -561,17 +576,8 @@ __device__ __forceinline__ float4 group_killing(const FusedArgs &a, const GroupS
   const float nrm = sqrtf(ff(kg[2], kg[2], ff(kg[1], kg[1], fm(kg[0], kg[0]))));
   const float sc = nrm > a.clamp ? a.clamp / nrm : 1.f;
   const float den = fm(fm(4.f, h), h);
-  const float4 j0 = sh.kil[0][1][lane], j1 = sh.kil[1][1][lane], j2 = sh.kil[2][1][lane];
-  const float J[3][3] = {{j0.x, j0.y, j0.z}, {j1.x, j1.y, j1.z}, {j2.x, j2.y, j2.z}};
-  float fr = 0.f, tr = 0.f;
-#pragma unroll
-  for (int p = 0; p < 3; ++p)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      fr = ff(J[p][k], J[p][k], fr);
-      tr = ff(J[p][k], J[k][p], tr);
-    }
-  return make_float4(fm(kg[0], sc) / den, fm(kg[1], sc) / den, fm(kg[2], sc) / den, ff(a.gamma_k, tr, fr));
+  return make_float4(fm(kg[0], sc) / den, fm(kg[1], sc) / den, fm(kg[2], sc) / den,
+                     killing_energy(a, sh.kil[0][1][lane], sh.kil[1][1][lane], sh.kil[2][1][lane]));
 }
 
 // A group's voxel between the step and its statistics (part 3).
@@ -965,49 +971,34 @@ __device__ __forceinline__ int update_band_voxel(const FusedArgs &a, int i, int 
   return settle_band_voxel<kTrust>(a, i, slot, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
 }
 
-// Updates the voxels i (-1: none) of the lanes of group g, as
-// update_band_voxel does for one: every thread of the group calls it, in role
-// w, with its lane's voxel, whose new psi goes to entry `slot` of the output
-// planes.  Part 3 and its results (the voxel for the next iteration's list,
-// or -1; the step for group_statistics; whether psi(i) is finite) are role
-// `last`'s; the other warps return -1.
-// Voxels of the outer shell are left alone (group_shell).
+// The 20 psi neighbours of voxel i in one plane.
 template <int kLoad>
-__device__ __forceinline__ int group_update(const FusedArgs &a, bool odd, int i, int slot, GroupShared &sh, int g,
-                                            int w, int last, int lane, GroupStep &t, bool &diverged) {
-  const DevParams &dp = a.dp;
-  t.active = false;
-  bool have = i >= 0;
-  if (have && (!KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST) || !KF_IN_BOUNDS(slot, dp.count, KF_SITE_BAND_LIST)))
-    have = false;
-  int x = 0, y = 0, z = 0;
-  if (have) voxel_xyz(dp, i, x, y, z);
-  const bool interior = have && interior_voxel(dp, x, y, z);
-  float own = 0.f, can = 0.f;  // roles 0-2: psi_w(i); role 3: the warped value and phi_can(i)
-  if (interior) {
-    if (w < 3) {
-      const float *r0 = (w == 0 ? plane_in<0>(a, odd) : (w == 1 ? plane_in<1>(a, odd) : plane_in<2>(a, odd))) + i;
-      const float *yp = r0 + a.row, *ym = r0 - a.row, *zp = r0 + a.plane, *zm = r0 - a.plane;
-      const float *ypzp = zp + a.row, *ymzp = zp - a.row, *ypzm = zm + a.row, *ymzm = zm - a.row;
-      float v[20];
+__device__ __forceinline__ void group_neighbours(const FusedArgs &a, const float *plane, int i, float v[20]) {
+  const float *r0 = plane + i;
+  const float *yp = r0 + a.row, *ym = r0 - a.row, *zp = r0 + a.plane, *zm = r0 - a.plane;
+  const float *ypzp = zp + a.row, *ymzp = zp - a.row, *ypzm = zm + a.row, *ymzm = zm - a.row;
 #pragma unroll
-      for (int n = 0; n < 20; ++n) {
-        const int oy = nb20_off(n, 1), oz = nb20_off(n, 2);
-        const float *r = oz == 0 ? (oy == 0 ? r0 : (oy > 0 ? yp : ym))
-                                 : (oz > 0 ? (oy == 0 ? zp : (oy > 0 ? ypzp : ymzp))
-                                           : (oy == 0 ? zm : (oy > 0 ? ypzm : ymzm)));
-        v[n] = load_psi<kLoad>(r + nb20_off(n, 0));
-      }
-      own = v[N000];
-      group_component(a, w, w == 0 ? x : (w == 1 ? y : z), w == 0 ? dp.nx : (w == 1 ? dp.ny : dp.nz), v, sh, lane);
-    } else {
-      can = __ldg(a.can + i);
-      const float p0 = load_psi<kLoad>(plane_in<0>(a, odd) + i), p1 = load_psi<kLoad>(plane_in<1>(a, odd) + i),
-                  p2 = load_psi<kLoad>(plane_in<2>(a, odd) + i);
-      own = phi_tri(a, fsb(fa(fa((float)x, p0), 0.5f), 0.5f), fsb(fa(fa((float)y, p1), 0.5f), 0.5f),
-                    fsb(fa(fa((float)z, p2), 0.5f), 0.5f));
-    }
+  for (int n = 0; n < 20; ++n) {
+    const int oy = nb20_off(n, 1), oz = nb20_off(n, 2);
+    const float *r = oz == 0 ? (oy == 0 ? r0 : (oy > 0 ? yp : ym))
+                             : (oz > 0 ? (oy == 0 ? zp : (oy > 0 ? ypzp : ymzp))
+                                       : (oy == 0 ? zm : (oy > 0 ? ypzm : ymzm)));
+    v[n] = load_psi<kLoad>(r + nb20_off(n, 0));
   }
+}
+
+// The warped value at x + psi (SDF::getDistance(i, psi), SDF.cpp:570-575).
+__device__ __forceinline__ float group_warped(const FusedArgs &a, int x, int y, int z, float p0, float p1, float p2) {
+  return phi_tri(a, fsb(fa(fa((float)x, p0), 0.5f), 0.5f), fsb(fa(fa((float)y, p1), 0.5f), 0.5f),
+                 fsb(fa(fa((float)z, p2), 0.5f), 0.5f));
+}
+
+// From the group's first barrier (after part 1) to its second: part 2 of role
+// w.  own: psi_w(i) on roles 0-2, the warped value on role 3; can: phi_can(i)
+// (role 3).
+__device__ __forceinline__ void group_middle(const FusedArgs &a, GroupShared &sh, int g, int w, int lane,
+                                             bool interior, int x, int y, int z, float own, float can) {
+  const DevParams &dp = a.dp;
   group_sync(g);
   // (the last round's `out` was read before this barrier)
   if (w == 3) {
@@ -1071,9 +1062,16 @@ __device__ __forceinline__ int group_update(const FusedArgs &a, bool odd, int i,
     if (w == 1) sh.more[3][lane] = fa(f[6], f[7]);
   }
   group_sync(g);
-  if (w != last || !interior) return -1;
+}
+
+// Part 3 of an interior voxel: its step, the terms of its monitored energy,
+// psi(i) (c0) and the warped value s.
+__device__ __forceinline__ void group_step(const FusedArgs &a, const GroupShared &sh, int lane, GroupStep &t,
+                                           float c0[3], float &s) {
+  const DevParams &dp = a.dp;
   const float4 hd = sh.out[0][lane], gr = sh.out[1][lane], ho = sh.out[2][lane], kg = sh.out[3][lane];
-  const float c0[3] = {hd.w, gr.w, ho.z}, s = sh.more[0][lane];
+  c0[0] = hd.w, c0[1] = gr.w, c0[2] = ho.z;
+  s = sh.more[0][lane];
   t.ke = kg.w;
   // KillingFusion.cpp:399-476
   float grad[3] = {0.f, 0.f, 0.f};
@@ -1102,6 +1100,45 @@ __device__ __forceinline__ int group_update(const FusedArgs &a, bool odd, int i,
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) t.d[k] = fm(-a.alpha, grad[k]);
+}
+
+// Updates the voxels i (-1: none) of the lanes of group g, as
+// update_band_voxel does for one: every thread of the group calls it, in role
+// w, with its lane's voxel, whose new psi goes to entry `slot` of the output
+// planes.  Part 3 and its results (the voxel for the next iteration's list,
+// or -1; the step for group_statistics; whether psi(i) is finite) are role
+// `last`'s; the other warps return -1.
+// Voxels of the outer shell are left alone (group_shell).
+template <int kLoad>
+__device__ __forceinline__ int group_update(const FusedArgs &a, bool odd, int i, int slot, GroupShared &sh, int g,
+                                            int w, int last, int lane, GroupStep &t, bool &diverged) {
+  const DevParams &dp = a.dp;
+  t.active = false;
+  bool have = i >= 0;
+  if (have && (!KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST) || !KF_IN_BOUNDS(slot, dp.count, KF_SITE_BAND_LIST)))
+    have = false;
+  int x = 0, y = 0, z = 0;
+  if (have) voxel_xyz(dp, i, x, y, z);
+  const bool interior = have && interior_voxel(dp, x, y, z);
+  float own = 0.f, can = 0.f;  // roles 0-2: psi_w(i); role 3: the warped value and phi_can(i)
+  if (interior) {
+    if (w < 3) {
+      float v[20];
+      group_neighbours<kLoad>(a, w == 0 ? plane_in<0>(a, odd) : (w == 1 ? plane_in<1>(a, odd) : plane_in<2>(a, odd)), i,
+                              v);
+      own = v[N000];
+      component_values(a, w, w == 0 ? x : (w == 1 ? y : z), w == 0 ? dp.nx : (w == 1 ? dp.ny : dp.nz), v,
+                       sh.mom[w][0][lane], sh.mom[w][1][lane], sh.kil[w][0][lane], sh.kil[w][1][lane]);
+    } else {
+      can = __ldg(a.can + i);
+      own = group_warped(a, x, y, z, load_psi<kLoad>(plane_in<0>(a, odd) + i), load_psi<kLoad>(plane_in<1>(a, odd) + i),
+                         load_psi<kLoad>(plane_in<2>(a, odd) + i));
+    }
+  }
+  group_middle(a, sh, g, w, lane, interior, x, y, z, own, can);
+  if (w != last || !interior) return -1;
+  float c0[3], s;
+  group_step(a, sh, lane, t, c0, s);
   t.active = in_band(s, a.band_hi, a.band_lo);
   if (t.active && (!isfinite(c0[0]) || !isfinite(c0[1]) || !isfinite(c0[2]))) diverged = true;
   // a voxel that left the band keeps psi: settle the output buffer
@@ -1117,6 +1154,155 @@ struct GroupStats {
   float maxd[32];
   unsigned active[32];
 };
+
+// ---------------------------------------------------------------------------
+// An interior voxel by one warp
+// ---------------------------------------------------------------------------
+// A lane per sample: for few voxels, where the length of one voxel's chain
+// is all that counts (a step of about 350 instructions a warp, 75 a voxel on a
+// group of four warps, but without the 25 samples or the components one after
+// the other, and no barrier).  The roundings are gradient_lane's.
+struct WarpShared {
+  float nb[3][20];    // psi at the 20 neighbours (nb20_off), per component
+  float4 mom[3][2];   // as GroupShared's
+  float4 kil[3][2];
+  float f[26];        // the cell-centre samples and the warped value
+};
+
+__constant__ signed char c_nb20[20][3] = {
+    {0, 0, 0},  {1, 0, 0},  {-1, 0, 0}, {0, 1, 0},   {0, -1, 0}, {0, 0, 1},  {0, 0, -1},
+    {1, 1, 0},  {1, -1, 0}, {-1, 1, 0}, {-1, -1, 0}, {1, 0, 1},  {1, 0, -1}, {-1, 0, 1},
+    {-1, 0, -1}, {0, 1, 1}, {0, 1, -1}, {0, -1, 1},  {0, -1, -1}, {1, 1, 1}};
+
+// What a lane keeps in registers through a kernel (constant memory would serve
+// a warp's different offsets one after the other): its neighbour's distance
+// and its sample's offset.
+struct WarpLane {
+  int64_t nb;
+  float o0, o1, o2;
+};
+
+__device__ __forceinline__ WarpLane warp_lane(const FusedArgs &a, int lane) {
+  WarpLane l{0, 0.f, 0.f, 0.f};
+  if (lane < 20) l.nb = c_nb20[lane][2] * a.plane + c_nb20[lane][1] * a.row + c_nb20[lane][0];
+  if (lane < 25) l.o0 = c_off25[lane][0], l.o1 = c_off25[lane][1], l.o2 = c_off25[lane][2];
+  return l;
+}
+
+// group_position with an offset of the lane's own: the terms with a zero
+// offset are left out by selects.
+__device__ __forceinline__ void warp_position(const FusedArgs &a, const GroupCell &q, const WarpLane &l, float t[3]) {
+  const float o01 = l.o0 * l.o1, o02 = l.o0 * l.o2, o12 = l.o1 * l.o2;  // 0 or +-1
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    float lin = 0.f, quad = 0.f;
+    const auto add = [](float o, float m, float &sum) {
+      const float v = ff(o, m, sum);
+      sum = o != 0.f ? v : sum;
+    };
+    add(l.o0, q.m[c][1], lin);
+    add(l.o1, q.m[c][2], lin);
+    add(l.o2, q.m[c][3], lin);
+    add(o01, q.m[c][4], quad);
+    add(o02, q.m[c][5], quad);
+    add(o12, q.m[c][6], quad);
+    const float oc = c == 0 ? l.o0 : (c == 1 ? l.o1 : l.o2);
+    t[c] = fa(fa(q.base[c], fm(a.h, oc)), ff(a.h, ff(a.h, quad, lin), q.m[c][0]));
+  }
+}
+
+// The neighbours of voxel i into sh.nb.
+template <int kLoad>
+__device__ __forceinline__ void warp_neighbours(const FusedArgs &a, int i, int lane, const WarpLane &l, WarpShared &sh) {
+  if (lane < 20) {
+    const int64_t o = i + l.nb;
+    sh.nb[0][lane] = load_psi<kLoad>(a.ix + o);
+    sh.nb[1][lane] = load_psi<kLoad>(a.iy + o);
+    sh.nb[2][lane] = load_psi<kLoad>(a.iz + o);
+  }
+}
+
+// The step of voxel (x, y, z) from sh.nb (psi(i) at entry 0): lane k < 3
+// returns component k of d = -alpha * g; t holds the terms of the monitored
+// energy (lane 0).  can: phi_can(i).
+__device__ __forceinline__ float warp_step(const FusedArgs &a, int x, int y, int z, float can, int lane,
+                                           const WarpLane &l, WarpShared &sh, GroupStep &t) {
+  const DevParams &dp = a.dp;
+  __syncwarp();
+  if (lane < 3) {
+    float v[20];
+#pragma unroll
+    for (int n = 0; n < 20; ++n) v[n] = sh.nb[lane][n];
+    component_values(a, lane, lane == 0 ? x : (lane == 1 ? y : z), lane == 0 ? dp.nx : (lane == 1 ? dp.ny : dp.nz), v,
+                     sh.mom[lane][0], sh.mom[lane][1], sh.kil[lane][0], sh.kil[lane][1]);
+  }
+  __syncwarp();
+  if (lane < 26) {
+    float p[3];
+    if (lane < 25) {
+      GroupCell q;
+      q.base[0] = fa((float)x, 0.5f);
+      q.base[1] = fa((float)y, 0.5f);
+      q.base[2] = fa((float)z, 0.5f);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float4 lo = sh.mom[c][0], hi = sh.mom[c][1];
+        q.m[c][0] = lo.x, q.m[c][1] = lo.y, q.m[c][2] = lo.z, q.m[c][3] = lo.w;
+        q.m[c][4] = hi.x, q.m[c][5] = hi.y, q.m[c][6] = hi.z;
+      }
+      warp_position(a, q, l, p);
+    } else {
+      p[0] = fsb(fa(fa((float)x, sh.nb[0][0]), 0.5f), 0.5f);
+      p[1] = fsb(fa(fa((float)y, sh.nb[1][0]), 0.5f), 0.5f);
+      p[2] = fsb(fa(fa((float)z, sh.nb[2][0]), 0.5f), 0.5f);
+    }
+    sh.f[lane] = phi_tri(a, p[0], p[1], p[2]);
+  }
+  __syncwarp();
+  float d = 0.f;
+  if (lane < 3) {
+    const float *f = sh.f, h = a.h;
+    // the Killing gradient (DisplacementField.cpp:326-345), component `lane`
+    const float4 k0 = sh.kil[0][0], k1 = sh.kil[1][0], k2 = sh.kil[2][0];
+    const float m2g = fm(-2.f, a.gamma_k);
+    const float kg[3] = {ff(m2g, fa(fa(fa(0.f, k0.y), k1.y), k2.y), k0.x),
+                         ff(m2g, fa(fa(fa(0.f, k0.z), k1.z), k2.z), k1.x),
+                         ff(m2g, fa(fa(fa(0.f, k0.w), k1.w), k2.w), k2.x)};
+    const float nrm = sqrtf(ff(kg[2], kg[2], ff(kg[1], kg[1], fm(kg[0], kg[0]))));
+    const float ksc = nrm > a.clamp ? a.clamp / nrm : 1.f;
+    const float kc = fm(lane == 0 ? kg[0] : (lane == 1 ? kg[1] : kg[2]), ksc) / fm(fm(4.f, h), h);
+    // SDF.cpp:726-744, 867-881
+    const float g[3] = {fm(fsb(f[1], f[2]), a.inv2h), fm(fsb(f[3], f[4]), a.inv2h), fm(fsb(f[5], f[6]), a.inv2h)};
+    const float gc = lane == 0 ? g[0] : (lane == 1 ? g[1] : g[2]);
+    float grad = 0.f;
+    if (dp.use_data) {
+      t.r = fsb(f[25], can) / a.voxel;
+      grad = ff(t.r, gc, grad);
+    }
+    if (dp.use_killing) grad = ff(kc, a.omega_k, grad);
+    if (dp.use_levelset) {
+      const float f02 = fm(2.f, f[0]);
+      const float hd = fm(fa(fsb(f[7 + 2 * lane], f02), f[8 + 2 * lane]), a.inv4hh);
+      const float hxz = fm(fsb(fsb(fa(f[13], f[19]), f[20]), f[14]), a.inv4hh);
+      const float hyz = fm(fsb(fsb(fa(f[15], f[21]), f[22]), f[16]), a.inv4hh);
+      const float hxy = fm(fsb(fsb(fa(f[17], f[23]), f[24]), f[18]), a.inv4hh);
+      t.gn = sqrtf(ff(g[2], g[2], ff(g[1], g[1], fm(g[0], g[0]))));
+      // row `lane` of the Hessian
+      const float r0 = lane == 0 ? hd : (lane == 1 ? hxy : hxz);
+      const float r1 = lane == 0 ? hxy : (lane == 1 ? hd : hyz);
+      const float r2 = lane == 0 ? hxz : (lane == 1 ? hyz : hd);
+      const float sc = fm(fsb(t.gn, 1.f) / fa(t.gn, a.eps), a.omega_s);
+      grad = ff(ff(r2, g[2], ff(r1, g[1], fm(r0, g[0]))), sc, grad);
+    }
+    d = fm(-a.alpha, grad);
+  }
+  return d;
+}
+
+// The Killing term of the monitored energy of a warp's voxel, into t.
+__device__ __forceinline__ void warp_energy_term(const FusedArgs &a, const WarpShared &sh, GroupStep &t) {
+  t.ke = killing_energy(a, sh.kil[0][1], sh.kil[1][1], sh.kil[2][1]);
+}
 
 // Adds the step t of a lane's voxel to its statistics.
 __device__ __forceinline__ void group_count(const FusedArgs &a, const GroupStep &t, GroupStats &st, int lane) {

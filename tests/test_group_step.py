@@ -58,3 +58,56 @@ def test_band_equals_dense_at_group_edges(gpu, count, shell, moved):
     np.testing.assert_array_equal(a[0], b[0])
     assert a[1:4] == b[1:4]
     assert abs(a[4] - b[4]) <= 1e-12 * abs(a[4])
+
+
+def oracle_params(P):
+    from oracle.oracle import Params
+    return Params(**{k: getattr(P, k) for k in Params.__dataclass_fields__})
+
+
+@pytest.mark.parametrize("count,shell", [(1, 1), (15, 0), (16, 4), (17, 0), (152, 0), (153, 20), (2432, 0), (2433, 80)])
+@pytest.mark.parametrize("moved", [False, True])
+def test_exact_solver_at_chunk_edges(gpu, oracle, count, shell, moved):
+    """The float64 solver's chunks of up to 16 voxels per CTA, bit for bit."""
+    shape = (21, 33, 27)
+    nz, ny, nx = shape
+    P = gpu.Params.reference(VOXEL, 5.0).with_(gamma_k=0.3)
+    live, can = scattered_pair(shape, count, shell, 7 * count, P)
+    psi0 = np.zeros(shape + (3,))
+    if moved:
+        psi0 = np.random.default_rng(count).normal(0.0, 0.4, psi0.shape)
+    grids = []
+    for phi in (live, can):
+        g = gpu.Grid((nx, ny, nz), VOXEL, (0.0, 0.0, 0.0), P.unknown_clip, P)
+        g.upload(phi, (phi <= P.max_surface).astype(np.int32))
+        grids.append(g)
+    f = gpu.Field((nx, ny, nz), gpu.KF_F64)
+    for iters in (1, 4):
+        f.upload(psi0)
+        gpu.psi_solve(grids[0], grids[1], f, P, iters, "exact")
+        _, want = oracle.solve(live.astype(np.float64), can.astype(np.float64), psi0, iters, oracle_params(P))
+        np.testing.assert_array_equal(f.download(), want)
+
+
+@pytest.mark.parametrize("count,shell", [(1, 0), (1, 1), (3, 1), (33, 9), (500, 60), (19500, 0)])
+def test_pervoxel_step_at_list_edges(gpu, oracle, count, shell):
+    """The per-voxel schedule's colour lists and warps, one step per voxel:
+    float32 rounding of one gradient (the bar of one Jacobi iteration)."""
+    shape = (25, 33, 27) if count < 19000 else (41, 61, 59)
+    nz, ny, nx = shape
+    P = gpu.Params.reference(VOXEL, 5.0)
+    live, can = scattered_pair(shape, count, shell, 3 * count + 1, P)
+    psi0 = np.random.default_rng(count).normal(0.0, 0.05, shape + (3,)).astype(np.float32)
+    grids = []
+    for phi in (live, can):
+        g = gpu.Grid((nx, ny, nz), VOXEL, (0.0, 0.0, 0.0), P.unknown_clip, P)
+        g.upload(phi, (phi <= P.max_surface).astype(np.int32))
+        grids.append(g)
+    f = gpu.Field((nx, ny, nz), gpu.KF_F32)
+    f.upload(psi0)
+    st = gpu.psi_solve(grids[0], grids[1], f, P, 1, "pervoxel")
+    r = oracle.solve_pervoxel(live.astype(np.float64), can.astype(np.float64), psi0.astype(np.float64), 1,
+                              oracle_params(P), colored=True)
+    want = next(v for v in r if isinstance(v, np.ndarray) and v.shape == psi0.shape)
+    assert st["active_first"] > 0 or count < 40
+    assert np.abs(f.download() - want).max() <= 1e-4
