@@ -39,6 +39,7 @@
 
 namespace {
 
+constexpr unsigned kSegments = 3;
 constexpr int kMaxBatch = 256;  // one problem per thread in the count scan (CTAs of >= 256)
 
 // One problem of the batch on the device: the argument blocks of the two
@@ -74,7 +75,8 @@ __global__ void __launch_bounds__(kThreads) k_batch_stream(const BatchEntry *__r
   const int bx = (int)(local % e.gx);
   const int by = (int)((local / e.gx) % e.gy);
   const int bz = (int)(local / ((int64_t)e.gx * e.gy));
-  stream_tile<true, kSlab>(e.a[0], bx, by, bz, e.band, &e.a[0].st[0].list);
+  // (record 1's list: the problem's shell voxels, in its second list)
+  stream_tile<true, kSlab>(e.a[0], bx, by, bz, e.band, &e.a[0].st[0].list, e.band + e.count, &e.a[0].st[1].list);
 }
 
 // exclusive prefix of cnt[0..n) into pre[0..n], n <= kMaxBatch <= blockDim.x
@@ -123,8 +125,12 @@ __device__ __forceinline__ int find_work(const unsigned *pre, int n, unsigned k)
 // The work is cut into chunks of kT * kVpt voxels that never cross a
 // problem, so a CTA works on one problem at a time: it stages that problem's
 // argument block in shared memory (the gradient reads it as often as the
-// single-grid kernel reads its constant parameters) and appends each round's
-// carried voxels with one atomic.  Returns false when every problem was
+// single-grid kernel reads its constant parameters).  A problem's list keeps
+// its order: the band only shrinks, and a voxel that leaves it empties its
+// entry.  (Appending the carried voxels anew each iteration cost two block
+// barriers and an atomic a chunk, and with an atomic per warp instead it
+// broke up the runs along x whose psi shares cache lines: 1.7 times the
+// sectors.)  Returns false when every problem was
 // skipped (converged or diverged): nothing is left to run.
 template <int kT, int kVpt>
 __device__ __forceinline__ bool batch_band_pass(const BatchEntry *__restrict__ tab, int nprob, int it) {
@@ -134,9 +140,12 @@ __device__ __forceinline__ bool batch_band_pass(const BatchEntry *__restrict__ t
   __shared__ unsigned s_maxd[kMaxBatch];
   __shared__ double s_energy[kMaxBatch];
   __shared__ int s_div[kMaxBatch];
+  __shared__ bool s_skip[kMaxBatch];
   __shared__ unsigned s_chunks[kMaxBatch];
+  __shared__ unsigned s_shell_pre[kMaxBatch + 1];  // shell voxels before each problem
   __shared__ FusedArgs s_a;
-  __shared__ int *s_list_in, *s_list_out;
+  __shared__ ShellScratch s_shell[kT / 32];
+  __shared__ int *s_list;
   __shared__ int s_live;  // problems not skipped this iteration
   constexpr int kChunk = kT * kVpt;
   const int par = it & 1;
@@ -146,8 +155,9 @@ __device__ __forceinline__ bool batch_band_pass(const BatchEntry *__restrict__ t
     const FusedArgs &a = tab[q].a[par];
     const bool gated = iteration_gated(a.st, it, a.dp);
     if (gated && blockIdx.x == 0) a.st[it].skipped = 1;
+    s_skip[q] = gated;
     if (!gated) atomicAdd(&s_live, 1);
-    s_cnt[q] = gated ? 0u : __ldcg(&a.st[it].list);
+    s_cnt[q] = gated ? 0u : __ldcg(&a.st[0].list);
     s_active[q] = 0u;
     s_maxd[q] = 0u;
     s_energy[q] = 0.0;
@@ -159,6 +169,10 @@ __device__ __forceinline__ bool batch_band_pass(const BatchEntry *__restrict__ t
   if (threadIdx.x < nprob) s_chunks[threadIdx.x] = (s_cnt[threadIdx.x] + kChunk - 1) / kChunk;
   __syncthreads();
   scan_counts<kT>(s_chunks, s_pre, nprob);
+  if (threadIdx.x < nprob)
+    s_chunks[threadIdx.x] = s_skip[threadIdx.x] ? 0u : __ldcg(&tab[threadIdx.x].a[par].st[1].list);
+  __syncthreads();
+  scan_counts<kT>(s_chunks, s_shell_pre, nprob);
   const unsigned total = s_pre[nprob];
   const int lane = threadIdx.x & 31;
   // statistics of the staged problem, per thread until the problem changes
@@ -189,32 +203,70 @@ __device__ __forceinline__ bool batch_band_pass(const BatchEntry *__restrict__ t
     active = 0;
     diverged = false;
   };
-  int cur = -1;  // problem staged in s_a (the same in every thread)
-  for (unsigned c = blockIdx.x; c < total; c += gridDim.x) {
-    const int p = find_work(s_pre, nprob, c);
-    if (p != cur) {
-      if (cur >= 0) flush(cur);
-      __syncthreads();  // the previous problem's arguments are no longer read
-      const int *src = reinterpret_cast<const int *>(&tab[p].a[par]);
-      int *dst = reinterpret_cast<int *>(&s_a);
-      for (int w = threadIdx.x; w < (int)(sizeof(FusedArgs) / sizeof(int)); w += blockDim.x) dst[w] = src[w];
-      if (threadIdx.x == 0) {
-        s_list_in = tab[p].band + (par ? tab[p].count : 0);
-        s_list_out = tab[p].band + (par ? 0 : tab[p].count);
+  // The shell voxels first, a warp each (shell_gradient), dealt out over all the
+  // grid's warps: they lie next to one another in index order, and as lanes of
+  // the chunks' warps 1.6 k of them in 40 problems of 20-50^3 held up every
+  // iteration by 110 us.
+  for (unsigned k = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; k < s_shell_pre[nprob];
+       k += (kT / 32) * gridDim.x) {
+    const int p = find_work(s_shell_pre, nprob, k);
+    const FusedArgs &a = tab[p].a[par];
+    int *entry = tab[p].band + tab[p].count + (k - s_shell_pre[p]);
+    const int i = __ldcg(entry);
+    if (i < 0 || !KF_IN_BOUNDS(i, a.dp.count, KF_SITE_BAND_LIST)) continue;
+    int x, y, z;
+    voxel_xyz(a.dp, i, x, y, z);
+    float d[3], s, en, c0[3];
+    shell_gradient<kPsiL1>(a, false, x, y, z, s_shell[threadIdx.x >> 5], d, &s, &en, c0);
+    if (lane == 0) {
+      if (settle_band_voxel<false>(a, i, i, x, y, z, s, en, c0, d, maxd, energy, active, diverged) < 0) *entry = -1;
+      if (active) {
+        atomicAdd(&s_active[p], active);
+        atomicMax(&s_maxd[p], __float_as_uint(maxd));
+        atomicAdd(&s_energy[p], energy);
       }
-      cur = p;
-      __syncthreads();
+      if (diverged) s_div[p] = 1;
+      maxd = 0.f;
+      energy = 0.0;
+      active = 0;
+      diverged = false;
     }
-#pragma unroll 1
-    for (int v = 0; v < kVpt; ++v) {
-      const unsigned k = (c - s_pre[p]) * kChunk + v * kT + threadIdx.x;
-      int next = -1;
-      if (k < s_cnt[p]) {
-        const int i = __ldcg(s_list_in + k);
-        next = update_band_voxel<false, kPsiL1>(s_a, i, i, maxd, energy, active, diverged);
+  }
+  __syncwarp();
+  int cur = -1;  // problem staged in s_a (the same in every thread)
+  // The chunks in kSegments segments, each cut into one run of consecutive
+  // chunks per CTA: a run's next chunk holds the last one's neighbours, whose
+  // psi and phi are still in L1, and each segment starts at another CTA, so
+  // that the longer runs do not add up.  64 problems, 3.4 M band voxels: 54.2 ms
+  // dealt out chunk by chunk, 49.4, 47.1, 45.8 and 45.6 ms in 10, 6, 3 and 1
+  // segments; more than one so that a slow problem's chunks spread.
+  const unsigned segments = total >= 2 * kSegments * gridDim.x ? kSegments : max(total / gridDim.x, 1u);
+  for (unsigned seg = 0; seg < segments; ++seg) {
+    const unsigned s0 = (unsigned)((uint64_t)total * seg / segments);
+    const unsigned len = (unsigned)((uint64_t)total * (seg + 1) / segments) - s0;
+    const unsigned r = (blockIdx.x + gridDim.x * seg / segments) % gridDim.x;
+    const unsigned c1 = s0 + (unsigned)((uint64_t)len * (r + 1) / gridDim.x);
+    for (unsigned c = s0 + (unsigned)((uint64_t)len * r / gridDim.x); c < c1; ++c) {
+      const int p = find_work(s_pre, nprob, c);
+      if (p != cur) {
+        if (cur >= 0) flush(cur);
+        __syncthreads();  // the previous problem's arguments are no longer read
+        const int *src = reinterpret_cast<const int *>(&tab[p].a[par]);
+        int *dst = reinterpret_cast<int *>(&s_a);
+        for (int w = threadIdx.x; w < (int)(sizeof(FusedArgs) / sizeof(int)); w += blockDim.x) dst[w] = src[w];
+        if (threadIdx.x == 0) {
+          s_list = tab[p].band;
+        }
+        cur = p;
+        __syncthreads();
       }
-      // hand the round's updated voxels to the next iteration
-      block_append<kT / 32>(next, &s_a.st[it + 1].list, s_list_out, s_a.dp.count);
+#pragma unroll 1
+      for (int v = 0; v < kVpt; ++v) {
+        const unsigned k = (c - s_pre[p]) * kChunk + v * kT + threadIdx.x;
+        const int i = k < s_cnt[p] ? __ldcg(s_list + k) : -1;
+        // a voxel that left the band leaves its entry empty
+        if (i >= 0 && update_interior_voxel<false, kPsiL1>(s_a, i, i, maxd, energy, active, diverged) < 0) s_list[k] = -1;
+      }
     }
   }
   if (cur >= 0) flush(cur);

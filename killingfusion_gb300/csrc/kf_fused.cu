@@ -218,20 +218,25 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
     if (blockIdx.x == 0 && threadIdx.x == 0) a.st[a.iter].skipped = 1;
     return;
   }
+  __shared__ FusedArgs s_args;
+  __shared__ ShellScratch s_shell[kLaneWarps];
   const int nq = (int)a.st[a.iter].list;
   const int total_threads = gridDim.x * kLaneThreads;
   const int rounds = (nq + total_threads - 1) / total_threads;
+  if ((int)blockIdx.x * kLaneThreads < nq) {
+    if (threadIdx.x == 0) s_args = a;
+    __syncthreads();
+  }
   float maxd = 0.f;
   double energy = 0.0;  // this thread's voxels, summed in float64 as the block and grid sums
   unsigned active = 0;
   bool diverged = false;
   for (int r = 0; r < rounds; ++r) {
     const int k = (r * gridDim.x + blockIdx.x) * kLaneThreads + threadIdx.x;
-    int next = -1;  // voxel this thread hands to the next iteration
-    if (k < nq) {
-      const int v = list_in[k];
-      next = update_band_voxel<kTrust>(a, v, kInPlace ? k : v, maxd, energy, active, diverged);
-    }
+    const int v = k < nq ? list_in[k] : -1;
+    // the voxel this thread hands to the next iteration
+    const int next = update_band_voxel<kTrust>(a, s_args, s_shell[threadIdx.x >> 5], v, kInPlace ? k : v, maxd, energy,
+                                               active, diverged);
     if (kCarry) block_append<kLaneWarps>(next, &a.st[a.iter + 1].list, list_out, a.dp.count);
   }
   reduce_iter_stats<kLaneThreads>(a.st + a.iter, active, maxd, energy, diverged);
@@ -286,6 +291,7 @@ struct PersistShared {
   GroupStats stats[kPersistGroups];
   BlockStats part[kPersistGroups];
   FusedArgs args;                  // for group_shell
+  ShellScratch scratch[kPersistGroups];
   bool ok, any_open, any_fail;     // the barrier's verdict
   unsigned long long seen[2];      // grid_verdict's record of the two barrier words
 };
@@ -340,7 +346,7 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
     if (sh.shell[g]) {
       for (unsigned k = 0; k < sh.n[g]; k += 32) {
         const int i = k + lane < sh.n[g] ? __ldcg((odd ? lst1 : lst0) + sh.k0[g] + k + lane) : -1;
-        group_carry(group_shell<kPsiL1>(&sh.args, odd, i, i, &sh.stats[g], &sh.fail[g]), lane, odd ? lst0 : lst1, per,
+        group_carry(group_shell<kPsiL1>(&sh.args, &sh.scratch[g], odd, i, i, &sh.stats[g], &sh.fail[g]), lane, odd ? lst0 : lst1, per,
                     sh, g);
       }
     }
@@ -553,32 +559,6 @@ __device__ __forceinline__ bool pervoxel_done(const FusedArgs &a, float dn, cons
   return !(dn / a.alpha > thr) || iter >= max_iters;
 }
 
-// A voxel of the outer shell, by one thread with the generic gradient.
-__device__ __noinline__ void pervoxel_shell(const FusedArgs *args, int i, int x, int y, int z, int max_iters,
-                                            float *dn_out, float *en_out, int *iter_out, unsigned *steps_out,
-                                            bool *diverged) {
-  const FusedArgs &a = *args;
-  int iter = 0;
-  unsigned steps = 0;
-  bool div = false;
-  while (true) {
-    float d[3], s, e;
-    gradient_generic<kPsiL2>(a, x, y, z, d, s, e);
-    const float n[3] = {__ldcg(a.ix + i) + d[0], __ldcg(a.iy + i) + d[1], __ldcg(a.iz + i) + d[2]};
-    // DisplacementField::update (DisplacementField.cpp:65-71)
-    a.ox[i] = n[0];
-    a.oy[i] = n[1];
-    a.oz[i] = n[2];
-    ++steps;
-    *dn_out = sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0]))));
-    *en_out = e;
-    if (pervoxel_done(a, *dn_out, n, max_iters, iter, div)) break;
-  }
-  *iter_out = iter;
-  *steps_out = steps;
-  if (div) *diverged = true;
-}
-
 // The voxels of one colour, one warp each (warp_step): a voxel's neighbours are
 // loaded once and its psi stays on chip until the last step, so a step costs no
 // trip to memory beyond the samples' corners (L1).
@@ -595,6 +575,7 @@ __global__ void __launch_bounds__(32 * kPervoxelWarps, kPervoxelBlocksPerSM)
     k_pervoxel(FusedArgs a, const int *__restrict__ list, const unsigned *__restrict__ counts, int max_iters,
                int colour) {
   __shared__ WarpShared s_warp[kPervoxelWarps];
+  __shared__ ShellScratch s_shell[kPervoxelWarps];
   __shared__ FusedArgs s_args;
   const DevParams &dp = a.dp;
   unsigned first = 0;
@@ -651,15 +632,22 @@ __global__ void __launch_bounds__(32 * kPervoxelWarps, kPervoxelBlocksPerSM)
         energy += e;
       }
     } else {
-      if (lane == 0) {
-        bool div = false;
-        pervoxel_shell(&s_args, i, x, y, z, max_iters, &dn, &en, &iter, &steps, &div);
-        diverged |= div;
-        energy += en;
+      while (true) {
+        float d[3], s, c0[3];
+        shell_gradient<kPsiL2>(s_args, false, x, y, z, s_shell[warp], d, &s, &en, c0);
+        const float n[3] = {c0[0] + d[0], c0[1] + d[1], c0[2] + d[2]};
+        __syncwarp();  // every lane has read psi
+        if (lane == 0) {
+          a.ox[i] = n[0];
+          a.oy[i] = n[1];
+          a.oz[i] = n[2];
+        }
+        __syncwarp();
+        ++steps;
+        dn = sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0]))));
+        if (pervoxel_done(a, dn, n, max_iters, iter, diverged)) break;
       }
-      dn = __shfl_sync(0xffffffffu, dn, 0);
-      iter = __shfl_sync(0xffffffffu, iter, 0);
-      steps = __shfl_sync(0xffffffffu, steps, 0);
+      if (lane == 0) energy += en;
     }
     maxd = fmaxf(maxd, dn);
     capped += iter >= max_iters;

@@ -606,36 +606,6 @@ __device__ __forceinline__ bool interior_voxel(const DevParams &dp, int x, int y
   return x >= 1 && y >= 1 && z >= 1 && x <= dp.nx - 2 && y <= dp.ny - 2 && z <= dp.nz - 2;
 }
 
-// A psi value read as load_psi<kLoad> reads it: the element type of psi
-// views in kernels that write psi themselves.  Same layout as float.
-template <int kLoad>
-struct PsiElem {
-  float v;
-  __device__ __forceinline__ operator float() const { return load_psi<kLoad>(&v); }
-};
-
-// Generic reference-order gradient for the outer shell (one thread), psi
-// read as kLoad says (plain loads for kPsiReadOnly).
-template <int kLoad = kPsiReadOnly>
-__device__ __noinline__ void gradient_generic(const FusedArgs &a, int x, int y, int z, float d[3],
-                                              float &s_out, float &e_out) {
-  using P = typename std::conditional<kLoad == kPsiReadOnly, float, PsiElem<kLoad>>::type;
-  const DevParams &dp = a.dp;
-  const P *px = reinterpret_cast<const P *>(a.ix), *py = reinterpret_cast<const P *>(a.iy),
-          *pz = reinterpret_cast<const P *>(a.iz);
-  PhiView<float> lv{a.live, dp.nx, dp.ny, dp.nz, a.oob};
-  PhiView<float> cv{a.can, dp.nx, dp.ny, dp.nz, a.oob};
-  PsiView<float, P> f{px, py, pz, dp.nx, dp.ny, dp.nz};
-  TParams<float> tp(dp);
-  float g[3], gd[3];
-  energy_gradient(lv, cv, f, tp, x, y, z, g);
-#pragma unroll
-  for (int k = 0; k < 3; ++k) d[k] = -tp.alpha * g[k];
-  s_out = warped_distance(lv, f, x, y, z);
-  distance_gradient(lv, f, tp.delta_size, x, y, z, gd);
-  e_out = monitor_energy(px, py, pz, dp.nx, dp.ny, dp.nz, x, y, z, s_out, cv.at(x, y, z), gd, dp);
-}
-
 // i / d for 0 <= i < 2^31 as (umulhi(i, mul) + i) >> shift (Granlund and
 // Montgomery's division by an invariant integer): 3 instructions where a
 // 32-bit division by a register takes about 20.
@@ -652,21 +622,21 @@ __device__ __forceinline__ void voxel_xyz(const DevParams &dp, int i, int &x, in
 
 // Dense pass over one tile (kTX x kTY columns, kSlab planes) of block
 // coordinates (bx, by, bz): stream the slab, apply the band test, append the
-// band voxels to list (*count counts them).  kPassThrough (ping-pong
+// band voxels to list in index order (*count counts them), but those of the
+// grid's outer shell to shell_list (*shell_count).  kPassThrough (ping-pong
 // buffers): copy psi of the voxels outside the band to the output buffer;
 // without it (psi updated in place) they are only read.
 template <bool kPassThrough, int kSlab = kZSlab>
 __device__ __forceinline__ void stream_tile(const FusedArgs &a, int bx, int by, int bz,
-                                            int *__restrict__ list, unsigned *count) {
-  __shared__ int queue[kThreads * kSlab];
-  __shared__ int qn, qbase;
+                                            int *__restrict__ list, unsigned *count,
+                                            int *__restrict__ shell_list, unsigned *shell_count) {
+  static_assert(kTX == 32, "a warp is a row of the tile");
+  __shared__ unsigned s_rows[kSlab * kTY];  // band voxels of each row, then of the rows before it
+  __shared__ unsigned s_base;
   const DevParams &dp = a.dp;
-  const int tid = threadIdx.y * kTX + threadIdx.x;
   const int x = bx * kTX + threadIdx.x;
   const int y = by * kTY + threadIdx.y;
   const int z0 = bz * kSlab;
-  if (tid == 0) qn = 0;
-  __syncthreads();
   const bool col = x < dp.nx && y < dp.ny;
   const int64_t sz = (int64_t)dp.nx * dp.ny;
   const int64_t base = ((int64_t)z0 * dp.ny + y) * dp.nx + x;
@@ -683,7 +653,7 @@ __device__ __forceinline__ void stream_tile(const FusedArgs &a, int bx, int by, 
   // psi == 0 samples its own cell with zero weights: the warped value is
   // phi_live(i) exactly.  Voxels that have moved are tested after the
   // streamed values are dead (their trilinear gather is the rare, long path).
-  unsigned moved = 0;
+  unsigned moved = 0, hit = 0;
 #pragma unroll
   for (int j = 0; j < kSlab; ++j) {
     int z = z0 + j;
@@ -692,8 +662,7 @@ __device__ __forceinline__ void stream_tile(const FusedArgs &a, int bx, int by, 
     if (px[j] != 0.f || py[j] != 0.f || pz[j] != 0.f) {
       moved |= 1u << j;
     } else if (in_band(ph[j], a.band_hi, a.band_lo)) {
-      const int q = atomicAdd(&qn, 1);
-      if (KF_IN_BOUNDS(q, kThreads * kSlab, KF_SITE_STREAM_QUEUE)) queue[q] = (int)i;
+      hit |= 1u << j;
     } else if (kPassThrough) {
       __stcs(a.ox + i, 0.f);
       __stcs(a.oy + i, 0.f);
@@ -707,19 +676,57 @@ __device__ __forceinline__ void stream_tile(const FusedArgs &a, int bx, int by, 
     const float qx = a.ix[i], qy = a.iy[i], qz = a.iz[i];
     const float s = warped_value(a, x, y, z0 + j, qx, qy, qz);
     if (in_band(s, a.band_hi, a.band_lo)) {
-      const int q = atomicAdd(&qn, 1);
-      if (KF_IN_BOUNDS(q, kThreads * kSlab, KF_SITE_STREAM_QUEUE)) queue[q] = (int)i;
+      hit |= 1u << j;
     } else if (kPassThrough) {
       __stcs(a.ox + i, qx);
       __stcs(a.oy + i, qy);
       __stcs(a.oz + i, qz);
     }
   }
+  if (hit) {
+    unsigned shell = hit;  // the planes of this column that lie on the shell
+    if (x >= 1 && x <= dp.nx - 2 && y >= 1 && y <= dp.ny - 2) {
+      shell = z0 == 0 ? hit & 1u : 0u;
+      if (z0 + kSlab >= dp.nz) shell |= hit & 1u << (dp.nz - 1 - z0);
+    }
+    hit &= ~shell;
+    for (; shell; shell &= shell - 1) {
+      const unsigned pos = atomicAdd(shell_count, 1u);
+      if (KF_IN_BOUNDS(pos, dp.count, KF_SITE_STREAM_LIST)) shell_list[pos] = (int)(base + (__ffs(shell) - 1) * sz);
+    }
+  }
+  if (!__syncthreads_or(hit != 0u)) return;
+  const int lane = threadIdx.x, warp = threadIdx.y;
+#pragma unroll
+  for (int j = 0; j < kSlab; ++j) {
+    const unsigned ball = __ballot_sync(0xffffffffu, hit >> j & 1u);
+    if (lane == 0) s_rows[j * kTY + warp] = (unsigned)__popc(ball);
+  }
   __syncthreads();
-  if (tid == 0 && qn) qbase = (int)atomicAdd(count, (unsigned)qn);
+  if (warp == 0) {  // the rows' counts to offsets
+    unsigned before = 0;
+#pragma unroll
+    for (int r = 0; r < kSlab * kTY; r += 32) {
+      const unsigned c = s_rows[r + lane];
+      unsigned incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      s_rows[r + lane] = before + incl - c;
+      before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) s_base = atomicAdd(count, before);
+  }
   __syncthreads();
-  for (int k = tid; k < min(qn, kThreads * kSlab); k += kThreads)
-    if (KF_IN_BOUNDS(qbase + k, dp.count, KF_SITE_STREAM_LIST)) list[qbase + k] = queue[k];
+#pragma unroll
+  for (int j = 0; j < kSlab; ++j) {
+    const bool mine = hit >> j & 1u;
+    const unsigned ball = __ballot_sync(0xffffffffu, mine);
+    const unsigned pos = s_base + s_rows[j * kTY + warp] + (unsigned)__popc(ball & ((1u << lane) - 1u));
+    if (mine && KF_IN_BOUNDS(pos, dp.count, KF_SITE_STREAM_LIST)) list[pos] = (int)(base + j * sz);
+  }
 }
 
 // Dense pass over one run of kFlatVoxels consecutive voxels (flat index
@@ -908,69 +915,6 @@ __device__ __noinline__ bool trust_step_f(const FusedArgs &a, int x, int y, int 
   return ok;
 }
 
-// Steps band voxel i, whose warped value is s, monitored energy en, psi c0
-// and step d: writes its new psi to entry `slot` of the output planes,
-// accumulates the statistics and returns the voxel for the next iteration's
-// list (-1 if it left the band).
-template <bool kTrust>
-__device__ __forceinline__ int settle_band_voxel(const FusedArgs &a, int i, int slot, int x, int y, int z, float s,
-                                                 float en, const float c0[3], float d[3], float &maxd, double &energy,
-                                                 unsigned &active, bool &diverged) {
-  const DevParams &dp = a.dp;
-  int next = -1;
-  if (in_band(s, a.band_hi, a.band_lo)) {
-    if (!isfinite(c0[0]) || !isfinite(c0[1]) || !isfinite(c0[2])) diverged = true;
-    if (kTrust && !trust_step_f(a, x, y, z, i, c0, d)) {
-      // this voxel and the rest of its row keep psi (k_trust_fix)
-      atomicMin(a.rows + (z * dp.ny + y), x);
-      d[0] = d[1] = d[2] = 0.f;
-    }
-    a.ox[slot] = c0[0] + d[0];
-    a.oy[slot] = c0[1] + d[1];
-    a.oz[slot] = c0[2] + d[2];
-    maxd = fmaxf(maxd, sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0])))));
-    energy += en;
-    ++active;
-    next = i;
-  } else {  // left the band: its psi is final, settle the output buffer
-    a.ox[slot] = c0[0];
-    a.oy[slot] = c0[1];
-    a.oz[slot] = c0[2];
-  }
-  return next;
-}
-
-// Update band voxel i (one thread) and write its new psi to entry `slot` of
-// the output planes (slot == i for ping-pong buffers; the voxel's list
-// position for in-place updates).  The voxel is re-tested with its warped
-// value: one outside the band keeps its psi (it left the band in the
-// previous iteration).  Returns the voxel for the next iteration's list (-1
-// if it left the band) and accumulates the statistics.
-// kTrust: the trust-region step (dp.trust set), a separate instantiation so
-// that the plain band pass carries no call to it.
-// kLoad: how psi is read (PsiLoad); the persistent passes, which write psi
-// between iterations, read it with kPsiL1.
-template <bool kTrust = false, int kLoad = kPsiReadOnly>
-__device__ __forceinline__ int update_band_voxel(const FusedArgs &a, int i, int slot, float &maxd,
-                                                 double &energy, unsigned &active, bool &diverged) {
-  const DevParams &dp = a.dp;
-  if (!KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST) || !KF_IN_BOUNDS(slot, dp.count, KF_SITE_BAND_LIST)) return -1;
-  int x, y, z;
-  voxel_xyz(dp, i, x, y, z);
-  float d[3] = {0.f, 0.f, 0.f}, s = 0.f, en = 0.f, c0[3] = {0.f, 0.f, 0.f};
-  const bool interior = x >= 1 && y >= 1 && z >= 1 && x <= dp.nx - 2 && y <= dp.ny - 2 &&
-                        z <= dp.nz - 2;
-  if (interior) {
-    gradient_lane<kLoad>(a, x, y, z, i, d, s, en, c0);
-  } else {
-    gradient_generic<kLoad>(a, x, y, z, d, s, en);
-    c0[0] = kLoad == kPsiReadOnly ? a.ix[i] : load_psi<kLoad>(a.ix + i);
-    c0[1] = kLoad == kPsiReadOnly ? a.iy[i] : load_psi<kLoad>(a.iy + i);
-    c0[2] = kLoad == kPsiReadOnly ? a.iz[i] : load_psi<kLoad>(a.iz + i);
-  }
-  return settle_band_voxel<kTrust>(a, i, slot, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
-}
-
 // The 20 psi neighbours of voxel i in one plane.
 template <int kLoad>
 __device__ __forceinline__ void group_neighbours(const FusedArgs &a, const float *plane, int i, float v[20]) {
@@ -1156,6 +1100,243 @@ struct GroupStats {
 };
 
 // ---------------------------------------------------------------------------
+// A voxel of the outer shell by one warp
+// ---------------------------------------------------------------------------
+// KillingFusion::computeEnergyGradient (KillingFusion.cpp:399-476) with the
+// reference's own samples -- truncating casts, psi's linear-index wrap
+// (DisplacementField.cpp:22-38), values outside the grid -- which the closed
+// forms of the interior leave out.  The 25 cell-centre samples (each psi,
+// then phi_live), the warped value and the 19 Killing samples are independent:
+// a lane each.  One thread ran them one after the other, about 20 k
+// instructions that its whole warp waited for; this takes about 500 a voxel.
+// Every rounding is spelled out, so all solvers give a shell voxel the same
+// bits.
+struct ShellScratch {
+  float f[26];      // the cell-centre samples (off25_at's order) and the warped value
+  float k[19][3];   // the Killing samples, in off25_at's order of its 19 second-difference offsets
+};
+
+template <int kLoad>
+__device__ __forceinline__ void shell_psi_at(const FusedArgs &a, const float *const p[3], int x, int y, int z,
+                                             float out[3]) {
+  const int index = z * (a.dp.nx * a.dp.ny) + y * a.dp.nx + x, total = a.dp.nx * a.dp.ny * a.dp.nz;
+  const bool in = index >= 0 && index < total;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) out[c] = in ? load_psi<kLoad>(p[c] + index) : 0.f;
+}
+
+// DisplacementField::getDisplacementAtf (DisplacementField.cpp:40-58).
+template <int kLoad>
+__device__ __forceinline__ void shell_psi_sample(const FusedArgs &a, const float *const p[3], const float q[3],
+                                                 float out[3]) {
+  const int b0 = (int)q[0], b1 = (int)q[1], b2 = (int)q[2];
+  float v[3][8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    float w[3];
+    shell_psi_at<kLoad>(a, p, b0 + (c & 1), b1 + ((c >> 1) & 1), b2 + (c >> 2), w);
+    v[0][c] = w[0], v[1][c] = w[1], v[2][c] = w[2];
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    out[k] = lerp3f(v[k], fsb(q[0], (float)b0), fsb(q[1], (float)b1), fsb(q[2], (float)b2));
+}
+
+// All lanes of a warp call it with the same voxel; every lane gets the step
+// d = -alpha * g, the warped value s, the monitored energy e and psi(i) in
+// c0.  args and sc (the warp's) in shared memory; odd: psi is in the output planes.
+template <int kLoad>
+__device__ __noinline__ void shell_gradient(const FusedArgs &a, bool odd, int x, int y, int z, ShellScratch &sc,
+                                            float *d, float *s_out, float *e_out, float *c0) {
+  const DevParams &dp = a.dp;
+  const float *const p[3] = {plane_in<0>(a, odd), plane_in<1>(a, odd), plane_in<2>(a, odd)};
+  const int lane = threadIdx.x & 31;
+  const float h = a.h;
+  __syncwarp();
+  if (lane < 26) {
+    float q[3] = {(float)x, (float)y, (float)z}, w[3];
+    if (lane < 25) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) q[c] = ff(h, (float)c_off25[lane][c], fa(q[c], 0.5f));
+      shell_psi_sample<kLoad>(a, p, q, w);
+    } else {
+      shell_psi_at<kLoad>(a, p, x, y, z, w);
+    }
+    sc.f[lane] = phi_tri(a, fsb(fa(fa(q[0], w[0]), 0.5f), 0.5f), fsb(fa(fa(q[1], w[1]), 0.5f), 0.5f),
+                         fsb(fa(fa(q[2], w[2]), 0.5f), 0.5f));
+  }
+  if (lane < 19) {
+    // the 19 offsets of the second differences: off25_at's 0 and 7..24
+    const signed char *o = c_off25[lane == 0 ? 0 : 6 + lane];
+    const float q[3] = {ff(h, (float)o[0], (float)x), ff(h, (float)o[1], (float)y), ff(h, (float)o[2], (float)z)};
+    shell_psi_sample<kLoad>(a, p, q, sc.k[lane]);
+  }
+  __syncwarp();
+  const float *f = sc.f, s = f[25];
+  const float can = __ldg(a.can + ((int64_t)z * dp.ny + y) * dp.nx + x);
+  const float two_h = fm(2.f, h), four_hh = fm(fm(4.f, h), h);
+  const float g[3] = {fsb(f[1], f[2]) / two_h, fsb(f[3], f[4]) / two_h, fsb(f[5], f[6]) / two_h};
+  float grad[3] = {0.f, 0.f, 0.f}, e = 0.f;
+  if (dp.use_data) {
+    const float r = fsb(s, can) / a.voxel;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) grad[k] = ff(r, g[k], grad[k]);
+    e = ff(fm(0.5f, r), r, e);
+  }
+  if (dp.use_killing) {
+    float kg[3], div[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      // (k[n]: off25_at's sample n + 6, k[0] the centre)
+      const auto v = [&](int n) { return sc.k[n][c]; };
+      const float v2 = fm(2.f, v(0));
+      const float xx = fa(fsb(v(1), v2), v(2)), yy = fa(fsb(v(3), v2), v(4)), zz = fa(fsb(v(5), v2), v(6));
+      const float xz = fsb(fsb(fa(v(7), v(13)), v(14)), v(8)), yz = fsb(fsb(fa(v(9), v(15)), v(16)), v(10)),
+                  xy = fsb(fsb(fa(v(11), v(17)), v(18)), v(12));
+      kg[c] = fm(-2.f, fa(fa(xx, yy), zz));
+      div[0] = fa(div[0], c == 0 ? xx : (c == 1 ? xy : xz));
+      div[1] = fa(div[1], c == 0 ? xy : (c == 1 ? yy : yz));
+      div[2] = fa(div[2], c == 0 ? xz : (c == 1 ? yz : zz));
+    }
+    const float m2g = fm(-2.f, a.gamma_k);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) kg[c] = ff(m2g, div[c], kg[c]);
+    const float nrm = sqrtf(ff(kg[2], kg[2], ff(kg[1], kg[1], fm(kg[0], kg[0]))));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float k = nrm > a.clamp ? fm(kg[c] / nrm, a.clamp) : kg[c];
+      grad[c] = ff(k / four_hh, a.omega_k, grad[c]);
+    }
+    // the Jacobian's clamped neighbours (kfref::monitor_energy)
+    float J[3][3], fr = 0.f, tr = 0.f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int up[3] = {min(x + (k == 0), dp.nx - 1), min(y + (k == 1), dp.ny - 1), min(z + (k == 2), dp.nz - 1)};
+      const int dn[3] = {max(x - (k == 0), 0), max(y - (k == 1), 0), max(z - (k == 2), 0)};
+      float u[3], w[3];
+      shell_psi_at<kLoad>(a, p, up[0], up[1], up[2], u);
+      shell_psi_at<kLoad>(a, p, dn[0], dn[1], dn[2], w);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) J[c][k] = fm(0.5f, fsb(u[c], w[c]));
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        fr = ff(J[c][k], J[c][k], fr);
+        tr = ff(J[c][k], J[k][c], tr);
+      }
+    e = ff(a.omega_k, ff(a.gamma_k, tr, fr), e);
+  }
+  if (dp.use_levelset) {
+    const float f02 = fm(2.f, f[0]);
+    const float hxx = fa(fsb(f[7], f02), f[8]) / four_hh, hyy = fa(fsb(f[9], f02), f[10]) / four_hh;
+    const float hzz = fa(fsb(f[11], f02), f[12]) / four_hh, hxz = fsb(fsb(fa(f[13], f[19]), f[20]), f[14]) / four_hh;
+    const float hyz = fsb(fsb(fa(f[15], f[21]), f[22]), f[16]) / four_hh;
+    const float hxy = fsb(fsb(fa(f[17], f[23]), f[24]), f[18]) / four_hh;
+    const float gn = sqrtf(ff(g[2], g[2], ff(g[1], g[1], fm(g[0], g[0]))));
+    const float nm1 = fsb(gn, 1.f), np = fa(gn, a.eps);
+    const float hg[3] = {ff(hxz, g[2], ff(hxy, g[1], fm(hxx, g[0]))), ff(hyz, g[2], ff(hyy, g[1], fm(hxy, g[0]))),
+                         ff(hzz, g[2], ff(hyz, g[1], fm(hxz, g[0])))};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) grad[c] = ff(fm(hg[c], nm1) / np, a.omega_s, grad[c]);
+    const float r = fsb(gn / a.voxel, 1.f);
+    e = ff(fm(fm(a.omega_s, 0.5f), r), r, e);
+  }
+  float own[3];
+  shell_psi_at<kLoad>(a, p, x, y, z, own);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    d[k] = fm(-a.alpha, grad[k]);
+    c0[k] = own[k];
+  }
+  *s_out = s;
+  *e_out = e;
+}
+
+// Steps band voxel i, whose warped value is s, monitored energy en, psi c0
+// and step d: writes its new psi to entry `slot` of the output planes,
+// accumulates the statistics and returns the voxel for the next iteration's
+// list (-1 if it left the band).
+template <bool kTrust>
+__device__ __forceinline__ int settle_band_voxel(const FusedArgs &a, int i, int slot, int x, int y, int z, float s,
+                                                 float en, const float c0[3], float d[3], float &maxd, double &energy,
+                                                 unsigned &active, bool &diverged) {
+  const DevParams &dp = a.dp;
+  int next = -1;
+  if (in_band(s, a.band_hi, a.band_lo)) {
+    if (!isfinite(c0[0]) || !isfinite(c0[1]) || !isfinite(c0[2])) diverged = true;
+    if (kTrust && !trust_step_f(a, x, y, z, i, c0, d)) {
+      // this voxel and the rest of its row keep psi (k_trust_fix)
+      atomicMin(a.rows + (z * dp.ny + y), x);
+      d[0] = d[1] = d[2] = 0.f;
+    }
+    a.ox[slot] = c0[0] + d[0];
+    a.oy[slot] = c0[1] + d[1];
+    a.oz[slot] = c0[2] + d[2];
+    maxd = fmaxf(maxd, sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0])))));
+    energy += en;
+    ++active;
+    next = i;
+  } else {  // left the band: its psi is final, settle the output buffer
+    a.ox[slot] = c0[0];
+    a.oy[slot] = c0[1];
+    a.oz[slot] = c0[2];
+  }
+  return next;
+}
+
+// As update_band_voxel, for a voxel known not to lie on the outer shell.
+template <bool kTrust, int kLoad>
+__device__ __forceinline__ int update_interior_voxel(const FusedArgs &a, int i, int slot, float &maxd, double &energy,
+                                                     unsigned &active, bool &diverged) {
+  if (!KF_IN_BOUNDS(i, a.dp.count, KF_SITE_BAND_LIST) || !KF_IN_BOUNDS(slot, a.dp.count, KF_SITE_BAND_LIST)) return -1;
+  int x, y, z;
+  voxel_xyz(a.dp, i, x, y, z);
+  float d[3], s, en, c0[3];
+  gradient_lane<kLoad>(a, x, y, z, i, d, s, en, c0);
+  return settle_band_voxel<kTrust>(a, i, slot, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
+}
+
+// Update band voxel i of each lane (-1: none; every lane of the warp calls it)
+// and write its new psi to entry `slot` of the output planes (slot == i for
+// ping-pong buffers; the voxel's list position for in-place updates).  The
+// voxel is re-tested with its warped value: one outside the band keeps its
+// psi (it left the band in the previous iteration).  Returns the voxel for
+// the next iteration's list (-1 if it left the band) and accumulates the
+// statistics.
+// kTrust: the trust-region step (dp.trust set), a separate instantiation so
+// that the plain band pass carries no call to it.
+// kLoad: how psi is read (PsiLoad); the persistent passes, which write psi
+// between iterations, read it with kPsiL1.
+// args: a copy of a in shared memory, sc: the warp's (shell_gradient).
+template <bool kTrust = false, int kLoad = kPsiReadOnly>
+__device__ __forceinline__ int update_band_voxel(const FusedArgs &a, const FusedArgs &args, ShellScratch &sc, int i,
+                                                 int slot, float &maxd, double &energy, unsigned &active,
+                                                 bool &diverged) {
+  const DevParams &dp = a.dp;
+  const bool have =
+      i >= 0 && KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST) && KF_IN_BOUNDS(slot, dp.count, KF_SITE_BAND_LIST);
+  int x = 0, y = 0, z = 0, next = -1;
+  if (have) voxel_xyz(dp, i, x, y, z);
+  const bool interior = have && interior_voxel(dp, x, y, z);
+  if (interior) {
+    float d[3], s, en, c0[3];
+    gradient_lane<kLoad>(a, x, y, z, i, d, s, en, c0);
+    next = settle_band_voxel<kTrust>(a, i, slot, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
+  }
+  for (unsigned rest = __ballot_sync(0xffffffffu, have && !interior); rest; rest &= rest - 1) {
+    const int owner = __ffs(rest) - 1;
+    float d[3], s, en, c0[3];
+    shell_gradient<kLoad>(args, false, __shfl_sync(0xffffffffu, x, owner), __shfl_sync(0xffffffffu, y, owner),
+                          __shfl_sync(0xffffffffu, z, owner), sc, d, &s, &en, c0);
+    if ((int)(threadIdx.x & 31) == owner)
+      next = settle_band_voxel<kTrust>(a, i, slot, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
+  }
+  return next;
+}
+
+// ---------------------------------------------------------------------------
 // An interior voxel by one warp
 // ---------------------------------------------------------------------------
 // A lane per sample: for few voxels, where the length of one voxel's chain
@@ -1315,35 +1496,40 @@ __device__ __forceinline__ void group_count(const FusedArgs &a, const GroupStep 
   st.active[lane] = active;
 }
 
-// The voxels of the outer shell among a warp's i (-1: none), one a lane, their
-// new psi to entry `slot`, with their statistics (st, *diverged).  Out of line, and its callers keep next to
-// nothing in registers across it: a value that has to survive a call is
-// kept in memory for good, and after a grid barrier (whose acquire empties L1)
-// every such load goes to L2.  args, st and diverged: in shared memory.
+// The voxels of the outer shell among a warp's i (-1: none), their new psi to
+// entry `slot`, with their statistics (st, *diverged).  Out of line, and its
+// callers keep next to nothing in registers across it: a value that has to
+// survive a call is kept in memory for good, and after a grid barrier (whose
+// acquire empties L1) every such load goes to L2.  args, sc, st and diverged: in shared
+// memory.
 template <int kLoad>
-__device__ __noinline__ int group_shell(const FusedArgs *args, bool odd, int i, int slot, GroupStats *st, bool *diverged) {
-  if (i < 0 || !KF_IN_BOUNDS(i, args->dp.count, KF_SITE_BAND_LIST) ||
-      !KF_IN_BOUNDS(slot, args->dp.count, KF_SITE_BAND_LIST))
-    return -1;
-  int x, y, z;
-  voxel_xyz(args->dp, i, x, y, z);
-  if (interior_voxel(args->dp, x, y, z)) return -1;
-  FusedArgs a = *args;
-  a.ix = plane_in<0>(*args, odd), a.iy = plane_in<1>(*args, odd), a.iz = plane_in<2>(*args, odd);
-  a.ox = plane_out<0>(*args, odd), a.oy = plane_out<1>(*args, odd), a.oz = plane_out<2>(*args, odd);
-  float d[3], s, en;
-  gradient_generic<kLoad>(a, x, y, z, d, s, en);
-  const float c0[3] = {load_psi<kLoad>(a.ix + i), load_psi<kLoad>(a.iy + i), load_psi<kLoad>(a.iz + i)};
-  float m = 0.f;
-  double e = 0.0;
-  unsigned n = 0;
-  bool div = false;
-  const int next = settle_band_voxel<false>(a, i, slot, x, y, z, s, en, c0, d, m, e, n, div);
+__device__ __noinline__ int group_shell(const FusedArgs *args, ShellScratch *sc, bool odd, int i, int slot,
+                                        GroupStats *st, bool *diverged) {
+  const bool have = i >= 0 && KF_IN_BOUNDS(i, args->dp.count, KF_SITE_BAND_LIST) &&
+                    KF_IN_BOUNDS(slot, args->dp.count, KF_SITE_BAND_LIST);
+  int x = 0, y = 0, z = 0, next = -1;
+  if (have) voxel_xyz(args->dp, i, x, y, z);
+  const bool mine = have && !interior_voxel(args->dp, x, y, z);
   const int lane = threadIdx.x & 31;
-  st->maxd[lane] = fmaxf(st->maxd[lane], m);
-  st->energy[lane] += e;
-  st->active[lane] += n;
-  if (div) *diverged = true;
+  for (unsigned rest = __ballot_sync(0xffffffffu, mine); rest; rest &= rest - 1) {
+    const int owner = __ffs(rest) - 1;
+    float d[3], s, en, c0[3];
+    shell_gradient<kLoad>(*args, odd, __shfl_sync(0xffffffffu, x, owner), __shfl_sync(0xffffffffu, y, owner),
+                          __shfl_sync(0xffffffffu, z, owner), *sc, d, &s, &en, c0);
+    if (lane != owner) continue;
+    const bool active = in_band(s, args->band_hi, args->band_lo);
+    if (active) {
+      if (!isfinite(c0[0]) || !isfinite(c0[1]) || !isfinite(c0[2])) *diverged = true;
+      st->maxd[lane] = fmaxf(st->maxd[lane], sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0])))));
+      st->energy[lane] += en;
+      ++st->active[lane];
+      next = i;
+    }
+    plane_out<0>(*args, odd)[slot] = active ? c0[0] + d[0] : c0[0];
+    plane_out<1>(*args, odd)[slot] = active ? c0[1] + d[1] : c0[1];
+    plane_out<2>(*args, odd)[slot] = active ? c0[2] + d[2] : c0[2];
+  }
+  __syncwarp();
   return next;
 }
 

@@ -111,3 +111,33 @@ def test_pervoxel_step_at_list_edges(gpu, oracle, count, shell):
     want = next(v for v in r if isinstance(v, np.ndarray) and v.shape == psi0.shape)
     assert st["active_first"] > 0 or count < 40
     assert np.abs(f.download() - want).max() <= 1e-4
+
+
+def test_batch_with_shell_voxels_equals_band(gpu):
+    """Batched problems with bands off the chunks' 256 voxels and with shell
+    voxels (listed apart, a warp each) give their band-only solves' bits."""
+    probs, want = [], []
+    for k, (shape, count, shell) in enumerate([((9, 11, 13), 40, 40), ((21, 23, 25), 255, 0), ((21, 23, 25), 257, 31),
+                                               ((33, 29, 31), 5000, 900), ((5, 4, 3), 60, 54), ((24, 24, 24), 1, 0)]):
+        nz, ny, nx = shape
+        P = gpu.Params.reference(VOXEL, 5.0).with_(gamma_k=0.2)
+        live, can = scattered_pair(shape, count, shell, 40 + k, P)
+        psi0 = np.random.default_rng(k).normal(0.0, 0.3, shape + (3,)).astype(np.float32)
+        grids = []
+        for phi in (live, can):
+            g = gpu.Grid((nx, ny, nz), VOXEL, (0.0, 0.0, 0.0), P.unknown_clip, P)
+            g.upload(phi, (phi <= P.max_surface).astype(np.int32))
+            grids.append(g)
+        f = gpu.Field((nx, ny, nz), gpu.KF_F32)
+        f.upload(psi0)
+        st = gpu.psi_solve(grids[0], grids[1], f, P, 5, "band")
+        want.append((f.download(), st["active_first"], st["active_last"], st["max_delta_last"], st["energy_last"]))
+        fb = gpu.Field((nx, ny, nz), gpu.KF_F32)
+        fb.upload(psi0)
+        probs.append((grids[0], grids[1], fb, P))
+    batch = gpu.Batch(probs, 5)
+    for (_, _, fb, _), w, st in zip(probs, want, batch.run()):
+        np.testing.assert_array_equal(fb.download(), w[0])
+        assert (st["active_first"], st["active_last"], st["max_delta_last"]) == w[1:4]
+        assert abs(st["energy_last"] - w[4]) <= 1e-12 * max(abs(w[4]), 1e-300)
+    batch.close()
