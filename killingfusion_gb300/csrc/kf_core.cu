@@ -259,8 +259,6 @@ extern "C" int kf_grid_destroy(kf_grid g) {
   if (!g) return KF_OK;
   cudaFree(g->phi);
   cudaFree(g->w);
-  cudaFree(g->phi_alt);
-  cudaFree(g->w_alt);
   cudaFree(g->depth);
   cudaFree(g->integ);
   cudaFree(g->mc);

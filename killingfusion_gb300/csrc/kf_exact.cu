@@ -64,6 +64,8 @@ struct IntegrateArgs {
   double voxel, min0, min1, min2, unknown_clip, min_depth, max_depth;
   float min_depth_up, max_depth_down;  // float neighbours of the depth range
   double depth_scale;                  // metres per unit of 16-bit depth
+  float scaleh, scalel;                // the same as a float pair
+  int v_lo, v_hi;                      // the 16-bit values in range (v_lo > v_hi: not known)
   float cliph, clipl;                  // unknown_clip as a float pair
   float tol;                           // bound on |float-float distance - reference's|
   float clip_thr;                      // |dist.hi + cliph| above this decides the clip test
@@ -329,18 +331,24 @@ __global__ void __launch_bounds__(kTileThreads)
   if (keep) live[base + __popc(ball & ((1u << lane) - 1u))] = (int)t;
 }
 
-// A fresh voxel (w == 0, phi finite) on float depth df, in float-float: the
-// distance df - zc with the camera depth zc from the pair tables, the
-// unknown-clip test and the float rounding, all decided when they lie
-// farther than a.tol from the reference's float64 boundaries.  Returns
-// kFfWritten (phi and w written), kFfClipped (not integrated, nothing
-// written) or kFfUndecided (nothing written) when one of them is too close
-// to call.
+// A voxel with phi finite on depth d, in float-float: the distance d - zc with
+// the camera depth zc from the pair tables, the unknown-clip test, the running
+// mean (SDF.cpp:185-193) and the float rounding, all decided when they lie
+// farther than the bound from the reference's float64 boundaries.  d and zc
+// are within a few 2^-48 of the reference's doubles, the distance within
+// a.tol; the mean of w > 0 samples adds about 2^-47 of its terms for the
+// product, sum and quotient (as ff_merge_mean), for which 2^-38 of them is
+// taken.  Returns kFfWritten (phi and w written), kFfClipped (not integrated,
+// nothing written) or kFfUndecided (nothing written) when one of them is too
+// close to call.
+// In float64 this arithmetic bound k_integrate wherever the depth was 16-bit
+// or the voxel had a weight: at 250 x 231 x 243 a 16-bit view into a fresh grid
+// took 32.8 us and 17.7 us now, one into voxels with weights 40.7 and 19.8 us.
 enum FfOutcome { kFfUndecided = 0, kFfWritten = 1, kFfClipped = 2 };
 
-__device__ __forceinline__ int integrate_fresh_ff(float *__restrict__ phi, int32_t *__restrict__ w, int64_t i,
-                                                  float df, FF zc, const IntegrateArgs &a) {
-  const FF dist = ff_add_short(FF{df, 0.f}, ff_neg(zc));
+__device__ __forceinline__ int integrate_ff(float *__restrict__ phi, int32_t *__restrict__ w, int64_t i, FF d, FF zc,
+                                            const IntegrateArgs &a, int32_t wi, float ph) {
+  const FF dist = ff_add_short(d, ff_neg(zc));
   // dist + unknown_clip < 0: not integrated.  One float add decides it: its
   // error is below 2^-23 (|mf| + |unknown_clip|) plus the distance's, which
   // clip_thr = 2^-18 |unknown_clip| + 2 tol exceeds; the float-float sum
@@ -354,11 +362,46 @@ __device__ __forceinline__ int integrate_fresh_ff(float *__restrict__ phi, int32
     return kFfClipped;
   }
   bool ambiguous;
-  const float r = ff_round_checked(dist, a.tol, ambiguous);
+  float r;
+  if (wi == 0) {
+    r = ff_round_checked(dist, a.tol, ambiguous);
+  } else {
+    const float den = (float)(wi + 1);  // exact below 2^24
+    const FF p = ff_two_prod((float)wi, ph);
+    const FF sum = ff_add(p, dist);
+    const float q1 = __fdiv_rn(sum.hi, den);
+    // sum.hi - q1 * den is exact for a correctly rounded q1
+    const float rem = __fadd_rn(__fmaf_rn(-q1, den, sum.hi), sum.lo);
+    const FF q = ff_fast_two_sum(q1, __fdiv_rn(rem, den));
+    const float tol =
+        __fdiv_rn(__fmaf_rn(__fadd_rn(fabsf(p.hi), fabsf(dist.hi)), 0x1p-38f, a.tol), den);
+    r = ff_round_checked(q, tol, ambiguous);
+  }
   if (ambiguous) return kFfUndecided;
   phi[i] = r;
-  w[i] = 1;
+  w[i] = wi + 1;
   return kFfWritten;
+}
+
+// The depth at pixel k as a float pair and its range test, or false in `known`
+// when the float64 path has to take the pixel.
+__device__ __forceinline__ bool depth_ff(const float *__restrict__ depth, int64_t k, const IntegrateArgs &a, FF &d,
+                                         bool &known) {
+  const float df = depth[k];
+  d = FF{df, 0.f};
+  known = isfinite(df);
+  return !(df < a.min_depth_up || df > a.max_depth_down);  // (a NaN passes, as in the reference)
+}
+
+// 16-bit: the values in range are an interval (launch_integrate), and
+// (double)v * scale is v times the scale's float pair, to a few 2^-48.
+__device__ __forceinline__ bool depth_ff(const uint16_t *__restrict__ depth, int64_t k, const IntegrateArgs &a, FF &d,
+                                         bool &known) {
+  const int v = depth[k];
+  const FF p = ff_two_prod((float)v, a.scaleh);
+  d = ff_fast_two_sum(p.hi, __fmaf_rn((float)v, a.scalel, p.lo));
+  known = a.v_lo <= a.v_hi;
+  return !known || (v >= a.v_lo && v <= a.v_hi);
 }
 
 // The voxel on the float64 path once its pixel k is known (the float-float
@@ -405,8 +448,8 @@ __device__ __noinline__ void integrate_f64_tail(float *__restrict__ phi, int32_t
 // The margin 1.5 (|K0| (E0 + |pa| E2) + |K1| (E1 + |pb| E2)) |1/c2| + 2^-19
 // (S + 2) holds all of that with room for the second-order terms.
 // The distance and the running mean are float64 as in the reference, decided
-// in float-float for a fresh voxel (integrate_fresh_ff), with the camera
-// depth summed from the tables' pairs there.
+// in float-float (integrate_ff), with the camera depth summed from the
+// tables' pairs there.
 //
 // kFresh: the grid is taken as just reset (phi = a.fresh_phi, w = 0; nothing
 // read) and every voxel is written, the reset values where nothing is
@@ -459,19 +502,18 @@ __device__ __forceinline__ void integrate_voxel(float *__restrict__ phi, int32_t
     return;
   }
   const int64_t k = (int64_t)row * a.width + col;
-  if constexpr (sizeof(D) == 4) {
-    // float depth into a fresh voxel: float-float, float64 only when too close to call
-    const float df = depth[k];
-    if (df < a.min_depth_up || df > a.max_depth_down) {  // (a NaN passes, as in the reference)
-      leave();
-      return;
-    }
-    if (wi == 0 && isfinite(ph) && isfinite(df)) {
-      const int r = integrate_fresh_ff(phi, w, i, df,
-                                       ff_add_short(ff_add_short(FF{px.z, px.w}, FF{py.z, py.w}), FF{pz.z, pz.w}), a);
-      if (r == kFfClipped) leave();
-      if (r != kFfUndecided) return;
-    }
+  // float-float; float64 only when too close to call
+  FF d;
+  bool known;
+  if (!depth_ff(depth, k, a, d, known)) {
+    leave();
+    return;
+  }
+  if (known && wi >= 0 && wi < (1 << 23) && isfinite(ph)) {
+    const int r = integrate_ff(phi, w, i, d, ff_add_short(ff_add_short(FF{px.z, px.w}, FF{py.z, py.w}), FF{pz.z, pz.w}),
+                               a, wi, ph);
+    if (r == kFfClipped) leave();
+    if (r != kFfUndecided) return;
   }
   integrate_f64_tail<D, kFresh>(phi, w, i, x, y, z, depth, k, tx, ty, tz, a, wi, ph);
 }
@@ -544,6 +586,27 @@ static int launch_integrate(kf_grid g, const D *depth_dev, double depth_scale, i
   a.height = height;
   a.count = g->count;
   a.depth_scale = depth_scale;
+  ff_split_host(depth_scale, a.scaleh, a.scalel);
+  // (double)v * scale does not decrease with v, so the values that pass the
+  // range test are an interval; where it is empty or the scale unusual the
+  // float64 path takes every pixel
+  a.v_lo = 1;
+  a.v_hi = 0;
+  if (depth_scale >= 1e-30 && depth_scale <= 1e30 && min_depth <= max_depth) {
+    auto first = [&](auto above) {  // the smallest v in [0, 65536] with above(v)
+      int lo = 0, hi = 65536;
+      while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (above((double)mid * depth_scale))
+          hi = mid;
+        else
+          lo = mid + 1;
+      }
+      return lo;
+    };
+    a.v_lo = first([&](double d) { return !(d < min_depth); });
+    a.v_hi = first([&](double d) { return d > max_depth; }) - 1;
+  }
   a.fresh_phi = fresh_phi ? *fresh_phi : 0.0f;
   ff_split_host(g->unknown_clip, a.cliph, a.clipl);
   {
@@ -874,22 +937,16 @@ __global__ void __launch_bounds__(kBlock) k_fuse(float *__restrict__ phi1, int32
 }
 
 // SDF::fuse(other, psi) (SDF.cpp:244-297): the other SDF's weight stays an
-// interpolated double until it is stored.
-template <typename P>
-__global__ void __launch_bounds__(kBlock) k_fuse_warped(float *__restrict__ phi1, int32_t *__restrict__ w1,
-                                                        const float *__restrict__ phi2,
-                                                        const int32_t *__restrict__ w2,
-                                                        PsiPlanes<P> f, int nx, int ny, int nz,
-                                                        double oob) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (int64_t)nx * ny * nz) return;
-  int x, y, z;
-  voxel_xyz(i, nx, ny, x, y, z);
-  double d2, b;
-  bool moved;
-  warp_sample(phi2, w2, nx, ny, nz, oob, f, i, x, y, z, d2, b, moved);
-  if (fabs(b) < (double)1e-5f) return;
-  int32_t a = w1[i];
+// interpolated double until it is stored.  A voxel with psi == 0 samples its
+// own cell, so its weight and value are the other's own: a CTA fuses those of
+// its 1024 voxels, four consecutive ones a thread with 16-byte loads (the values only
+// where there is a weight), lists the moved ones in shared memory and then
+// resamples them in float64, a voxel a thread on full warps.
+// HBM-bound: psi and the weights are 16 B a voxel.  251 x 256 x 233: 40 us,
+// against 127 us with a voxel a thread and every weight and value read; 49 us with the
+// moved voxels in a list of their own and a second pass.
+__device__ __forceinline__ void fuse_sampled(float *__restrict__ phi1, int32_t *__restrict__ w1, int64_t i, int32_t a,
+                                             double d2, double b) {
   if (a == 0) {
     phi1[i] = (float)d2;
     w1[i] = (int32_t)(int64_t)b;
@@ -897,6 +954,99 @@ __global__ void __launch_bounds__(kBlock) k_fuse_warped(float *__restrict__ phi1
     double d1 = (double)phi1[i];
     phi1[i] = (float)(((double)a * d1 + b * d2) / ((double)a + b));
     w1[i] = (int32_t)(int64_t)((double)a + b);
+  }
+}
+
+// The same where b is the integer weight w2 != 0 and d2 a float: the mean
+// decided in float-float (ff_merge_mean) where it can be.
+__device__ __forceinline__ void fuse_kept(float *__restrict__ phi1, int32_t *__restrict__ w1, int64_t i, int32_t a,
+                                          float f2, int32_t w2) {
+  float r;
+  if (a != 0 && ff_merge_mean(a, phi1[i], w2, f2, r)) {
+    phi1[i] = r;
+    w1[i] = a + w2;
+  } else {
+    fuse_sampled(phi1, w1, i, a, (double)f2, (double)w2);
+  }
+}
+
+template <typename P>
+__device__ __forceinline__ unsigned moved_of_four(PsiPlanes<P> f, int64_t q) {
+  unsigned moved = 0;
+  if constexpr (sizeof(P) == 4) {
+    const float4 x = __ldcs(reinterpret_cast<const float4 *>(f.x) + q);
+    const float4 y = __ldcs(reinterpret_cast<const float4 *>(f.y) + q);
+    const float4 z = __ldcs(reinterpret_cast<const float4 *>(f.z) + q);
+    moved = (x.x != 0.f || y.x != 0.f || z.x != 0.f) | (x.y != 0.f || y.y != 0.f || z.y != 0.f) << 1 |
+            (x.z != 0.f || y.z != 0.f || z.z != 0.f) << 2 | (x.w != 0.f || y.w != 0.f || z.w != 0.f) << 3;
+  } else {
+    const P *p[3] = {f.x, f.y, f.z};
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const double2 v = __ldcs(reinterpret_cast<const double2 *>(p[c]) + 2 * q + e);
+        moved |= (unsigned)(v.x != 0.0) << (2 * e) | (unsigned)(v.y != 0.0) << (2 * e + 1);
+      }
+  }
+  return moved;
+}
+
+template <typename P>
+__global__ void __launch_bounds__(kBlock) k_fuse_warped(float *__restrict__ phi1, int32_t *__restrict__ w1,
+                                                        const float *__restrict__ phi2,
+                                                        const int32_t *__restrict__ w2, PsiPlanes<P> f, int nx, int ny,
+                                                        int nz, double oob) {
+  __shared__ int s_list[4 * kBlock];
+  __shared__ int s_n;
+  const int64_t N = (int64_t)nx * ny * nz;
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i0 = 4 * q;
+  int32_t b[4] = {0, 0, 0, 0};
+  unsigned moved = 0;
+  const bool whole = i0 + 3 < N;
+  if (whole) {
+    moved = moved_of_four(f, q);
+    const int4 v = __ldcs(reinterpret_cast<const int4 *>(w2) + q);
+    b[0] = v.x, b[1] = v.y, b[2] = v.z, b[3] = v.w;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      if (i0 + e >= N) break;
+      b[e] = w2[i0 + e];
+      if (f.x[i0 + e] != P(0) || f.y[i0 + e] != P(0) || f.z[i0 + e] != P(0)) moved |= 1u << e;
+    }
+  }
+  unsigned keep = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) keep |= (unsigned)(b[e] != 0 && !(moved >> e & 1u)) << e;
+  if (keep && whole) {
+    const float4 d = __ldcs(reinterpret_cast<const float4 *>(phi2) + q);
+    const int4 a = *(reinterpret_cast<const int4 *>(w1) + q);
+    if (keep & 1u) fuse_kept(phi1, w1, i0, a.x, d.x, b[0]);
+    if (keep & 2u) fuse_kept(phi1, w1, i0 + 1, a.y, d.y, b[1]);
+    if (keep & 4u) fuse_kept(phi1, w1, i0 + 2, a.z, d.z, b[2]);
+    if (keep & 8u) fuse_kept(phi1, w1, i0 + 3, a.w, d.w, b[3]);
+  } else if (keep) {
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+      if (keep >> e & 1u) fuse_kept(phi1, w1, i0 + e, w1[i0 + e], phi2[i0 + e], b[e]);
+  }
+  if (threadIdx.x == 0) s_n = 0;
+  if (!__syncthreads_or(moved != 0u)) return;
+  if (moved) {
+    int at = atomicAdd(&s_n, __popc(moved));
+    for (unsigned m = moved; m; m &= m - 1, ++at) s_list[at] = 4 * (int)threadIdx.x + __ffs(m) - 1;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < s_n; k += kBlock) {
+    const int64_t i = 4 * (int64_t)blockIdx.x * kBlock + s_list[k];
+    int x, y, z;
+    voxel_xyz(i, nx, ny, x, y, z);
+    double d2, b;
+    bool m;
+    warp_sample(phi2, w2, nx, ny, nz, oob, f, i, x, y, z, d2, b, m);
+    if (fabs(b) < (double)1e-5f) continue;
+    fuse_sampled(phi1, w1, i, w1[i], d2, b);
   }
 }
 
@@ -1231,18 +1381,6 @@ PhiView<T> phi_view(const kf_grid g, const float *phi, double oob) {
 
 }  // namespace
 
-int kf_grid_ensure_alt(kf_grid g) {
-  if (g->phi_alt) return KF_OK;
-  if (cudaMalloc(&g->phi_alt, g->count * sizeof(float)) != cudaSuccess)
-    return kf_fail(KF_ERR_OOM, "cudaMalloc of the resampling buffer failed");
-  if (cudaMalloc(&g->w_alt, g->count * sizeof(int32_t)) != cudaSuccess) {
-    cudaFree(g->phi_alt);
-    g->phi_alt = nullptr;
-    return kf_fail(KF_ERR_OOM, "cudaMalloc of the resampling buffer failed");
-  }
-  return KF_OK;
-}
-
 template <typename P>
 static PsiPlanes<P> planes(kf_field f) {
   return PsiPlanes<P>{(const P *)f->p[0], (const P *)f->p[1], (const P *)f->p[2]};
@@ -1324,14 +1462,13 @@ int kf_launch_fuse(kf_grid can, kf_grid other, cudaStream_t s) {
 
 int kf_launch_fuse_warped(kf_grid dst, kf_grid other, kf_field psi, const DevParams &dp,
                           cudaStream_t s) {
+  const unsigned blocks = blocks_for((dst->count + 3) / 4);
   if (psi->prec == KF_F32)
-    k_fuse_warped<float><<<blocks_for(dst->count), kBlock, 0, s>>>(
-        dst->phi, dst->w, other->phi, other->w, planes<float>(psi), dst->n[0], dst->n[1],
-        dst->n[2], dp.oob_phi);
+    k_fuse_warped<float><<<blocks, kBlock, 0, s>>>(dst->phi, dst->w, other->phi, other->w, planes<float>(psi),
+                                                   dst->n[0], dst->n[1], dst->n[2], dp.oob_phi);
   else
-    k_fuse_warped<double><<<blocks_for(dst->count), kBlock, 0, s>>>(
-        dst->phi, dst->w, other->phi, other->w, planes<double>(psi), dst->n[0], dst->n[1],
-        dst->n[2], dp.oob_phi);
+    k_fuse_warped<double><<<blocks, kBlock, 0, s>>>(dst->phi, dst->w, other->phi, other->w, planes<double>(psi),
+                                                    dst->n[0], dst->n[1], dst->n[2], dp.oob_phi);
   KF_CHECK_LAUNCH("k_fuse_warped");
   return KF_OK;
 }

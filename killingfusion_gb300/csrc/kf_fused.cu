@@ -417,7 +417,7 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
 // the solve can change (the iterations overwrite lst0).  per_block: the
 // fewest band voxels worth a block; a smaller band leaves the last blocks
 // without any, and they end at once.
-__global__ void __launch_bounds__(kPersistThreads, 1)
+__global__ void __maxnreg__(104)
     k_band_persistent(FusedArgs a, int *lst0, int *lst1, int iterations, GridSync *sync,
                       unsigned long long limit_ns, int *touched, unsigned *touched_n, unsigned per_block) {
   extern __shared__ __align__(16) unsigned char smem[];

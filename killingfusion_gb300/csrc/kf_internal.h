@@ -19,8 +19,6 @@ struct kf_grid_s {
   double unknown_clip;
   float *phi;      // device, count
   int32_t *w;      // device, count
-  float *phi_alt;  // second buffers for out-of-place resampling (lazy)
-  int32_t *w_alt;
   float *depth;    // device staging for host depth frames (lazily sized)
   size_t depth_cap;
   void *integ;     // integration scratch: counter, coordinate tables, list
