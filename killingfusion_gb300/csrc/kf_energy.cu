@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kThreads) k_energy(EArgs<T, P> a, int x0, int 
 }
 
 // One block; thread t sums the partials t, t + kSumThreads, ..., then a fixed tree.
-constexpr int kSumThreads = 256;
+constexpr int kSumThreads = 1024;
 __global__ void __launch_bounds__(kSumThreads) k_sum_partials(const double *partial, int blocks, double *out) {
   double s[3] = {0.0, 0.0, 0.0};
 #pragma unroll 4
@@ -259,8 +259,8 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_partials(const double *part
 // gathers the voxels of its run that have work in shared memory, in order, and
 // takes them on full warps; a small run keeps the CTAs that lie in the active
 // region from being the kernel's tail.  The mapping is fixed, so the sums are.
-// 121 x 128 x 115 blobs: energy 103 us (31 k_warped, 59 k_energy_runs, 13 the sum)
-// and gradient 183 us (43, 20, 119), against 401 and 943 us with a thread per voxel
+// 121 x 128 x 115 blobs: energy 106 us (31 k_warped, 59 k_energy_runs, 16 the sum)
+// and gradient 182 us (43, 20, 119), against 388 and 943 us with a thread per voxel
 // of the grid that samples phi_w seven times and takes whole Jacobians.
 constexpr int kRun = 256, kRunThreads = 128;
 
