@@ -369,7 +369,9 @@ int kf_field_stats(kf_field f, int iterations, IterStats **dev) {
 }
 
 int kf_field_band_list(kf_field f, int **out) {
-  if (!f->band && cudaMalloc(&f->band, 2 * f->count * sizeof(int)) != cudaSuccess) {
+  // (two of all voxels and one of the outer shell's)
+  const int64_t inner = (int64_t)std::max(f->n[0] - 2, 0) * std::max(f->n[1] - 2, 0) * std::max(f->n[2] - 2, 0);
+  if (!f->band && cudaMalloc(&f->band, (3 * f->count - inner) * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     f->band = nullptr;
     return kf_fail(KF_ERR_OOM, "cudaMalloc of the band voxel list failed");
@@ -968,13 +970,13 @@ static int solve_finish(kf_field psi, kf_solve_stats *stats, bool presumed_swapp
   }
   if (host[0].timeout) {
     if (stats) stats->device_ms = ms;
-    return kf_fail(KF_ERR_TIMEOUT, "a grid-wide wait of the persistent band pass gave up (limit " +
+    return kf_fail(KF_ERR_TIMEOUT, "a grid-wide wait of the persistent solver gave up (limit " +
                                        std::to_string(kf_wait_limit_ns() / 1e9) + " s); psi is undefined");
   }
   for (int k = 0; k < iterations; ++k)
     if (host[k].cold)
-      return kf_fail(KF_ERR_INTERNAL, "the split dense schedule found a band voxel in a run without band "
-                                      "voxels at the first iteration");
+      return kf_fail(KF_ERR_INTERNAL, "the dense solver found a band voxel outside the band of its first "
+                                      "iteration");
   int executed = 0;
   int diverged = 0;
   for (int k = 0; k < iterations; ++k) {

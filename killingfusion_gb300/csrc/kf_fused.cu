@@ -36,6 +36,7 @@
 // Voxels on the grid's outer shell take the generic reference-order path
 // (truncating casts, linear-index wrap, outside values).
 #include <algorithm>
+#include <type_traits>
 
 #include "kf_fused_body.cuh"
 #include "kf_grid_sync.cuh"
@@ -78,11 +79,17 @@ __global__ void __launch_bounds__(kThreads) k_fused_stream(FusedArgs a, int *__r
 // the test reads phi_live alone (4 B a voxel, against 16 B read and 12 B
 // copied by k_fused_stream<true>), and the second buffer already holds
 // every voxel's psi.  The same list as k_fused_stream<true> gives.
-__global__ void __launch_bounds__(kThreads) k_band_first_zero(FusedArgs a, int *__restrict__ list) {
-  stream_flat<false, false, true>(a, blockIdx.x, list, &a.st[a.iter].list, nullptr);
+__global__ void __launch_bounds__(kThreads) k_band_first_zero(FusedArgs a, int *__restrict__ list, int *__restrict__ shell) {
+  stream_flat<false, false, true>(a, blockIdx.x, list, &a.st[0].list, nullptr, shell, &a.st[1].list);
 }
 
-// Split dense schedule (grids of at least kSplitMinRuns runs).  After the
+// The same where psi may be anything: k_fused_stream<true> with the band's
+// voxels of the outer shell in a list of their own.
+__global__ void __launch_bounds__(kThreads) k_band_first(FusedArgs a, int *__restrict__ list, int *__restrict__ shell) {
+  stream_flat<true>(a, blockIdx.x, list, &a.st[0].list, nullptr, shell, &a.st[1].list);
+}
+
+// Split dense schedule (grids above persistent_test_blocks' limit).  After the
 // first iteration's dense pass, k_split_runs sorts the runs into those that
 // listed band voxels ("hot") and the others ("cold"), each in run order.  A
 // voxel outside the band keeps its psi and phi_live does not change, so the
@@ -93,7 +100,6 @@ __global__ void __launch_bounds__(kThreads) k_band_first_zero(FusedArgs a, int *
 // its cold runs (test only) on a second stream, beside the band pass of the
 // iteration before.  A band voxel found in a cold run is counted in
 // IterStats::cold and fails the solve.
-constexpr int kSplitMinRuns = 512;
 constexpr int kSplitThreads = 1024;
 constexpr int kHotBlocksPerSM = 5;  // resident CTAs of k_fused_stream (48 registers)
 
@@ -252,6 +258,7 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
 //   slice of the other list by a ballot of its warp 0, with no atomic and no
 //   block-wide step.  Neighbouring band voxels (which share psi neighbours)
 //   stay in one SM's L1.
+// - Voxels of the outer shell have a list of their own (k_band_first), in place.
 // - psi is read through L1 and L2 (kPsiL1: the blocks write it between
 //   iterations, ordered by the barrier's fences), the SDFs through the
 //   read-only path.  A gated iteration (converged, diverged) ends the kernel
@@ -266,12 +273,19 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
 // What bounds it: the latency of an iteration's chain -- psi loads from L2
 // (the barrier's acquire empties L1), the parts of group_update, the barrier.
 // Four groups per SM: 128 voxels a round, the bench's band (14.7 k voxels, 97
-// per SM) in one round.  All 128 registers of 512 threads: at 96 and 80 the
-// compiler keeps loop state in memory, which costs a trip to L2 after every
-// barrier.  Measured at 256^3 (14.7 k band voxels, 200 iterations): 4.8 us an
-// iteration (0.95 ms a solve) against 8.9 us (1.79 ms) with one thread per
-// voxel in 96-thread blocks, where 97 voxels took two rounds; 64^3 (1.7 k band
-// voxels): 3.4 us against 6.0 us.
+// per SM) in one round.  104 registers a thread: fewer spill loop state, which
+// costs a trip to L2 after every barrier, more leave the SM's L1 less
+// (sequences at 256^3 with 80, 88, 96, 104, 112, 128: 5258, 5297, 5210, 4913,
+// 5017, 5025 us for ten frames).
+// Measured at 256^3 (14.7 k band voxels, 200 iterations): 4.7 us an iteration
+// against 8.9 us with one thread per voxel in 96-thread blocks, where 97 voxels
+// took two rounds; 64^3 (1.7 k band voxels): 3.4 us against 6.0 us.
+// Voxels of the outer shell take about 4 us each (a warp's lanes share the 45
+// samples of one), so they are not in the groups' slices, which lie along a
+// face where one is in the band, but dealt out to all warps.  48^3 with 87 k
+// band voxels, 10 k of them on the shell, 100 iterations: 3.0 ms against 57 ms
+// with the shell's voxels in their groups and 22.9 ms with a thread per voxel;
+// 64^3 with all 236 k: 6.6 ms against 154 and 52 ms.
 // Blocks: a band of few voxels uses fewer, one per kPersistPerBlock voxels (a
 // barrier of fewer blocks is shorter, a block of fewer voxels no faster).
 // Whole 64^3 frames with 24, 32, 48, 64, 96 and 128 voxels a block: 1788, 1783,
@@ -280,6 +294,17 @@ constexpr int kPersistGroups = 4;
 constexpr int kPersistThreads = kGroupThreads * kPersistGroups;
 constexpr unsigned kPersistPerBlock = 32;
 
+// The dense solver of a small grid (persistent_test_blocks) is the same
+// kernel with four more warps a block, which test every voxel outside the
+// band in every iteration, beside the band pass (96 registers a thread: 20
+// warps of 104 do not fit the four register files).  One launch per solve and
+// the voxels' tests hidden, against three launches an iteration of which each
+// waits for the one before: 64^3 with 17.3 k band voxels 5.4 us an iteration
+// against 15.6, 100^3 with 41.8 k 11 against 20.5.
+constexpr int kTestThreads = 128;
+constexpr int kTestChunks = 16;    // most groups of four voxels a test thread takes
+constexpr int kTestChunksMin = 4;  // the fewest worth a block
+
 struct PersistShared {
   GroupShared group[kPersistGroups];
   int first[kPersistGroups][32];   // the next iteration's first round
@@ -287,14 +312,23 @@ struct PersistShared {
   unsigned n[kPersistGroups];      // voxels each group carries
   unsigned carried[kPersistGroups];
   bool fail[kPersistGroups], open[kPersistGroups];
-  bool shell[kPersistGroups];      // the slice holds voxels of the grid's outer shell
   GroupStats stats[kPersistGroups];
   BlockStats part[kPersistGroups];
-  FusedArgs args;                  // for group_shell
-  ShellScratch scratch[kPersistGroups];
+  FusedArgs args;                  // for warp_shell
+  ShellScratch scratch[kPersistGroups * kGroupWarps];
+  GroupStats shell;                // entry w: warp w's voxels of the grid's outer shell
+  unsigned nshell;                 // the grid's list of those
+  bool shell_fail;
   bool ok, any_open, any_fail;     // the barrier's verdict
   unsigned long long seen[2];      // grid_verdict's record of the two barrier words
 };
+struct DensePersistShared : PersistShared {
+  unsigned entered[kTestThreads / 32];               // voxels that a test warp found in the band
+  unsigned char first[kTestChunks][kTestThreads];    // test_outside_band
+};
+
+template <bool kDense>
+using PersistSharedOf = std::conditional_t<kDense, DensePersistShared, PersistShared>;
 
 // Compacts a warp's carried voxels `next` (-1: none) into the group's slice of
 // `out`, after those already there.
@@ -311,20 +345,125 @@ __device__ __forceinline__ void group_carry(int next, int lane, int *__restrict_
   __syncwarp();
 }
 
+// A test warp's iteration.  Thread t of the grid's test threads takes the
+// groups of four voxels t, t + threads, ...; `first` keeps the four bits of each,
+// the voxels in the band at iteration 0.  Those are in the band list, whose
+// pass tests them, until they leave it, which sets their bit of `dropped`;
+// every other voxel is tested here, on the psi that the iteration reads.  A
+// voxel that passes was never in the band or had left it: none may, as psi
+// changes in the band alone.  Returns how many did.
+__device__ __forceinline__ unsigned test_outside_band(const FusedArgs &a, int it, unsigned nblocks,
+                                                      const unsigned *dropped,
+                                                      unsigned char (*first)[kTestThreads]) {
+  const DevParams &dp = a.dp;
+  const bool odd = it & 1;
+  const int n = (int)dp.count, n4 = (n + 3) >> 2;
+  const int threads = (int)nblocks * kTestThreads;
+  const float *px = plane_in<0>(a, odd), *py = plane_in<1>(a, odd), *pz = plane_in<2>(a, odd);
+  unsigned entered = 0;
+  const int t = (int)threadIdx.x - kPersistThreads;
+  int c = 0;
+#pragma unroll 2
+  for (int q = (int)blockIdx.x * kTestThreads + t; q < n4 && c < kTestChunks; q += threads, ++c) {
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x, z = x, ph = x;
+    unsigned valid = 15u;
+    if (4 * q + 4 <= n) {
+      x = __ldcg(reinterpret_cast<const float4 *>(px) + q);
+      y = __ldcg(reinterpret_cast<const float4 *>(py) + q);
+      z = __ldcg(reinterpret_cast<const float4 *>(pz) + q);
+      ph = __ldg(reinterpret_cast<const float4 *>(a.live) + q);
+    } else {  // the ragged end of the grid
+      valid = (1u << (n & 3)) - 1u;
+      float e[4][4] = {};
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        if (valid >> k & 1u) {
+          e[0][k] = __ldcg(px + 4 * q + k);
+          e[1][k] = __ldcg(py + 4 * q + k);
+          e[2][k] = __ldcg(pz + 4 * q + k);
+          e[3][k] = __ldg(a.live + 4 * q + k);
+        }
+      x = make_float4(e[0][0], e[0][1], e[0][2], 0.f);
+      y = make_float4(e[1][0], e[1][1], e[1][2], 0.f);
+      z = make_float4(e[2][0], e[2][1], e[2][2], 0.f);
+      ph = make_float4(e[3][0], e[3][1], e[3][2], 0.f);
+    }
+    unsigned moved = 0, hit = 0;
+    flat_test(a, x.x, y.x, z.x, ph.x, moved, hit, 0);
+    flat_test(a, x.y, y.y, z.y, ph.y, moved, hit, 1);
+    flat_test(a, x.z, y.z, z.z, ph.z, moved, hit, 2);
+    flat_test(a, x.w, y.w, z.w, ph.w, moved, hit, 3);
+    if (it > 0) {
+      const unsigned was = first[c][t];
+      const unsigned left = was ? was & __ldcg(dropped + (q >> 3)) >> (4 * (q & 7)) : 0u;
+      hit &= ~was;
+      moved = (moved & ~was) | left;  // (one that left is tested as the band pass did)
+    }
+    hit &= valid;
+    for (moved &= valid; moved; moved &= moved - 1) {
+      const int b = __ffs(moved) - 1, i = 4 * q + b;
+      int vx, vy, vz;
+      voxel_xyz(dp, i, vx, vy, vz);
+      const float w = warped_value(a, vx, vy, vz, __ldcg(px + i), __ldcg(py + i), __ldcg(pz + i));
+      if (in_band(w, a.band_hi, a.band_lo)) hit |= 1u << b;
+    }
+    if (it == 0)
+      first[c][t] = (unsigned char)hit;
+    else
+      entered += (unsigned)__popc(hit);
+  }
+  return entered;
+}
+
+// Voxel v has left the band (test_outside_band tests it from the next
+// iteration on).
+__device__ __forceinline__ void note_dropped(unsigned *dropped, int v) {
+  atomicOr(dropped + (v >> 5), 1u << (v & 31));
+}
+
+// A warp's share of the shell's list: entry w * nblocks + block, and so on.  An
+// entry turns -1 when its voxel leaves the band.
+template <bool kDense>
+__device__ __forceinline__ void shell_round(const DevParams &dp, bool odd, unsigned nblocks, int *shell,
+                                            unsigned *dropped, PersistShared &sh) {
+  const unsigned warp = threadIdx.x >> 5, stride = kPersistGroups * kGroupWarps * nblocks;
+  for (unsigned j = warp * nblocks + blockIdx.x; j < sh.nshell; j += stride) {
+    const int v = __ldcg(shell + j);
+    if (v < 0) continue;
+    if (!warp_shell<kPsiL1>(&sh.args, &sh.scratch[warp], odd, v, (int)warp, &sh.shell, &sh.shell_fail) &&
+        (threadIdx.x & 31) == 0) {
+      __stcg(shell + j, -1);
+      if (kDense) note_dropped(dropped, v);
+    }
+    __syncwarp();
+  }
+}
+
 // Iteration `it` of the group's voxels, the entries [k0, k0 + n) of lst0 (lst1
 // in odd iterations); carried ones go to the other list.  False when the
 // kernel must end (the iteration was the last, a barrier wait gave up, or the
 // next iteration is gated).  The first 32 entries are read from first[] (from
 // lst0 at it == 0).  What a group keeps from one round to the next is in shared
-// memory, not in registers (group_shell).
-__device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, int it, bool last, int *lst0, int *lst1,
+// memory, not in registers (warp_shell).  The voxels of the outer shell, which are
+// in no group's slice, are dealt out to all warps of all blocks, one at a time each.
+template <bool kDense>
+__device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, int it, bool last, int *lst0, int *lst1, int *shell,
                                                           unsigned per, GridSync *sync, unsigned nblocks,
-                                                          unsigned long long limit_ns, PersistShared &sh) {
+                                                          unsigned long long limit_ns, unsigned *dropped,
+                                                          PersistShared &sh) {
   // group g on warps 4g..4g+3, its roles rotated by g so that every scheduler
   // has each role once; part 3 is on a warp of another scheduler in each group
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = warp / kGroupWarps, w = (warp + g) % kGroupWarps, last_role = (2 * g) % kGroupWarps;
   const bool odd = it & 1;
+  if (kDense && g == kPersistGroups) {  // a test warp
+    DensePersistShared &d = static_cast<DensePersistShared &>(sh);
+    const unsigned entered = __reduce_add_sync(0xffffffffu, test_outside_band(a, it, nblocks, dropped, d.first));
+    if (lane == 0) d.entered[warp - kPersistGroups * kGroupWarps] = entered;
+    __syncthreads();
+    __syncthreads();
+    return !last && sh.ok && !sh.any_fail && (!a.dp.early_exit || sh.any_open);
+  }
   GroupStep t;
   t.active = false;
   bool diverged = false;
@@ -332,6 +471,7 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
   for (unsigned k = 0; k < sh.n[g]; k += 32) {
     if (w == last_role && k > 0) group_count(a, t, sh.stats[g], lane);  // the round before
     const int next = group_update<kPsiL1>(a, odd, v, v, sh.group[g], g, w, last_role, lane, t, diverged);
+    if (kDense && w == last_role && v >= 0 && next < 0) note_dropped(dropped, v);
     v = k + 32 + lane < sh.n[g] ? __ldcg((odd ? lst1 : lst0) + sh.k0[g] + k + 32 + lane) : -1;
     if (w == last_role) group_carry(next, lane, odd ? lst0 : lst1, per, sh, g);
   }
@@ -339,24 +479,20 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
     const bool fail = __any_sync(0xffffffffu, diverged);
     if (lane == 0) sh.fail[g] = fail;
     __syncwarp();
-    if (sh.shell[g] || a.dp.early_exit) {
+    if (sh.nshell || a.dp.early_exit) {
       group_count(a, t, sh.stats[g], lane);
       t.active = false;
-    }
-    if (sh.shell[g]) {
-      for (unsigned k = 0; k < sh.n[g]; k += 32) {
-        const int i = k + lane < sh.n[g] ? __ldcg((odd ? lst1 : lst0) + sh.k0[g] + k + lane) : -1;
-        group_carry(group_shell<kPsiL1>(&sh.args, &sh.scratch[g], odd, i, i, &sh.stats[g], &sh.fail[g]), lane, odd ? lst0 : lst1, per,
-                    sh, g);
-      }
     }
     // (the verdict needs the largest step only then)
     const bool open = a.dp.early_exit && __any_sync(0xffffffffu, sh.stats[g].maxd[lane] > (float)a.dp.threshold);
     if (lane == 0) sh.open[g] = open;
   }
+  if (sh.nshell) shell_round<kDense>(a.dp, odd, nblocks, shell, dropped, sh);
   __syncthreads();
   if (threadIdx.x == 96 && !last) {
-    bool open = false, fail = false;
+    bool open = false, fail = sh.shell_fail;
+    for (int k = 0; sh.nshell && a.dp.early_exit && k < kPersistGroups * kGroupWarps; ++k)
+      open |= sh.shell.maxd[k] > (float)a.dp.threshold;
 #pragma unroll
     for (int k = 0; k < kPersistGroups; ++k) {
       open |= sh.open[k];
@@ -374,6 +510,14 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
     sh.stats[g].maxd[lane] = 0.f;
     sh.stats[g].energy[lane] = 0.0;
     sh.stats[g].active[lane] = 0u;
+    if (g == 0 && sh.nshell) {
+      energy += sh.shell.energy[lane];
+      maxd = fmaxf(maxd, sh.shell.maxd[lane]);
+      active += sh.shell.active[lane];
+      sh.shell.energy[lane] = 0.0;
+      sh.shell.maxd[lane] = 0.f;
+      sh.shell.active[lane] = 0u;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       energy += __shfl_xor_sync(0xffffffffu, energy, o);
@@ -381,7 +525,7 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
       active += __shfl_xor_sync(0xffffffffu, active, o);
     }
     if (lane == 0) {
-      sh.part[g] = BlockStats{energy, active, maxd, sh.fail[g]};
+      sh.part[g] = BlockStats{energy, active, maxd, sh.fail[g] || (g == 0 && sh.shell_fail)};
       sh.n[g] = sh.carried[g];
       sh.carried[g] = 0u;
     }
@@ -397,6 +541,12 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
       b.diverged |= sh.part[k].diverged;
     }
     commit_iter_stats(a.st + it, b);
+    if (kDense) {
+      unsigned entered = 0;
+#pragma unroll
+      for (int k = 0; k < kTestThreads / 32; ++k) entered += static_cast<DensePersistShared &>(sh).entered[k];
+      if (entered) atomicAdd(&a.st[it].cold, entered);
+    }
   }
   if (last) return false;
   if (!sh.ok) {
@@ -416,48 +566,81 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
 // (or NULL): a copy of that list and its length, the only voxels whose psi
 // the solve can change (the iterations overwrite lst0).  per_block: the
 // fewest band voxels worth a block; a smaller band leaves the last blocks
-// without any, and they end at once.
-__global__ void __maxnreg__(104)
-    k_band_persistent(FusedArgs a, int *lst0, int *lst1, int iterations, GridSync *sync,
-                      unsigned long long limit_ns, int *touched, unsigned *touched_n, unsigned per_block) {
+// without any, and they end at once.  kDense (kTestThreads more threads): the
+// dense solver; least_blocks: the blocks that its test warps need, dropped: a
+// zeroed bit per voxel (test_outside_band).
+template <bool kDense>
+__global__ void __maxnreg__(kDense ? 96 : 104)
+    k_band_persistent(FusedArgs a, int *lst0, int *lst1, int *shell, int iterations, GridSync *sync,
+                      unsigned long long limit_ns, int *touched, unsigned *touched_n, unsigned per_block,
+                      unsigned least_blocks, unsigned *dropped) {
   extern __shared__ __align__(16) unsigned char smem[];
-  PersistShared &sh = *reinterpret_cast<PersistShared *>(smem);
-  const unsigned nq = __ldcg(&a.st[0].list);
-  const unsigned nblocks = max(min(gridDim.x, (nq + per_block - 1) / per_block), 1u);
+  PersistShared &sh = *reinterpret_cast<PersistSharedOf<kDense> *>(smem);
+  const unsigned nq = __ldcg(&a.st[0].list), nshell = __ldcg(&a.st[1].list);
+  const unsigned nblocks = min(gridDim.x, max((nq + per_block - 1) / per_block,
+                                              max((nshell + kPersistGroups * kGroupWarps - 1) /
+                                                      (kPersistGroups * kGroupWarps), least_blocks)));
   if (blockIdx.x >= nblocks) return;
   const unsigned groups = nblocks * kPersistGroups;
   const unsigned per = (nq + groups - 1) / groups;  // a group's slice
   if (threadIdx.x == 0) {
     sh.args = a;
     sh.seen[0] = sh.seen[1] = 0;
+    sh.nshell = nshell;
+    sh.shell_fail = false;
   }
   if (threadIdx.x < kPersistGroups) {
     const unsigned k0 = min((blockIdx.x * kPersistGroups + threadIdx.x) * per, nq);
     sh.k0[threadIdx.x] = k0;
     sh.n[threadIdx.x] = min(k0 + per, nq) - k0;
     sh.carried[threadIdx.x] = 0u;
-    sh.shell[threadIdx.x] = false;
   }
   if (threadIdx.x < 32 * kPersistGroups) {
     GroupStats &st = sh.stats[threadIdx.x / 32];
     st.energy[threadIdx.x % 32] = 0.0;
     st.maxd[threadIdx.x % 32] = 0.f;
     st.active[threadIdx.x % 32] = 0u;
-  }
-  if (touched && blockIdx.x == 0 && threadIdx.x == 0) *touched_n = nq;
-  __syncthreads();
-  const int g = threadIdx.x / kGroupThreads;
-  for (unsigned j = threadIdx.x % kGroupThreads; j < sh.n[g]; j += kGroupThreads) {
-    const unsigned k = sh.k0[g] + j;
-    const int v = __ldcg(lst0 + k);
-    if (touched) touched[k] = v;
-    int x, y, z;
-    voxel_xyz(a.dp, v, x, y, z);
-    if (!interior_voxel(a.dp, x, y, z)) sh.shell[g] = true;
+  } else if (threadIdx.x < 32 * kPersistGroups + 32) {
+    sh.shell.energy[threadIdx.x % 32] = 0.0;
+    sh.shell.maxd[threadIdx.x % 32] = 0.f;
+    sh.shell.active[threadIdx.x % 32] = 0u;
   }
   __syncthreads();
+  if (touched) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *touched_n = nq + nshell;
+    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < nq; k += nblocks * blockDim.x)
+      touched[k] = __ldcg(lst0 + k);
+    // (a warp's own: iteration 0 already overwrites entries of this list)
+    const unsigned warps = kPersistGroups * kGroupWarps, warp = threadIdx.x >> 5;
+    if (warp < warps) {
+      for (unsigned j = (warp + (threadIdx.x & 31) * warps) * nblocks + blockIdx.x; j < nshell; j += 32 * warps * nblocks)
+        touched[nq + j] = __ldcg(shell + j);
+      __syncwarp();
+    }
+  }
   for (int it = 0; it < iterations; ++it)
-    if (!persistent_band_iteration(a, it, it + 1 == iterations, lst0, lst1, per, sync, nblocks, limit_ns, sh)) return;
+    if (!persistent_band_iteration<kDense>(a, it, it + 1 == iterations, lst0, lst1, shell, per, sync, nblocks, limit_ns,
+                                           dropped, sh)) {
+      if (kDense && blockIdx.x == 0 && threadIdx.x == 0) a.st[0].executed = it + 1;
+      return;
+    }
+}
+
+// Dense solver: psi stays in the primary planes.  After an odd number of
+// iterations the result is in the second ones, which differ at the voxels of
+// the first band list alone.
+__global__ void __launch_bounds__(kThreads) k_dense_settle(FusedArgs a, const int *__restrict__ touched,
+                                                          const unsigned *touched_n) {
+  if (!(a.st[0].executed & 1)) return;
+  float *px = const_cast<float *>(a.ix), *py = const_cast<float *>(a.iy), *pz = const_cast<float *>(a.iz);
+  const unsigned n = *touched_n;
+  for (unsigned k = blockIdx.x * kThreads + threadIdx.x; k < n; k += gridDim.x * kThreads) {
+    const int v = touched[k];
+    if (!KF_IN_BOUNDS(v, a.dp.count, KF_SITE_WRITE_BACK)) continue;
+    px[v] = a.ox[v];
+    py[v] = a.oy[v];
+    pz[v] = a.oz[v];
+  }
 }
 
 // In-place update after the last iteration: psi(list[k]) = entry k of the
@@ -689,7 +872,7 @@ static int64_t num_runs(const DevParams &dp) {
 }
 
 static bool split_schedule(const DevParams &dp, bool band_only) {
-  return !band_only && !dp.trust && num_runs(dp) >= kSplitMinRuns;
+  return !band_only && !dp.trust;
 }
 
 // A launch whose graph node carries a priority: the hot chain of the split
@@ -713,7 +896,9 @@ static void launch_prio(void (*kernel)(KArgs...), unsigned grid, unsigned block,
 // The split schedule's lists after the run table: hot runs, cold runs (one
 // int per run each) and their two counts.
 static size_t runs_table_bytes(int64_t nruns) {
-  return (size_t)nruns * sizeof(int2) + ((size_t)2 * nruns + 4) * sizeof(int);
+  const size_t table = (size_t)nruns * sizeof(int2) + ((size_t)2 * nruns + 4) * sizeof(int);
+  const size_t bits = (size_t)nruns * (kThreads * kFlatGroups * 4 / 8) + 16;  // (and a ragged end)
+  return std::max(table, bits);
 }
 
 // The dense fused iterations on the split schedule (see k_split_runs).
@@ -793,12 +978,8 @@ static void launch_iterations(kf_grid live, kf_grid can, kf_field psi, const Dev
     if (!band_only) {
       // lists alternate so that a run can still read the previous iteration's
       k_fused_stream<false><<<grid, block, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1], runs);
-      if (dp.trust) {
-        k_fused_band<false, true, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], nullptr);
-        k_trust_fix<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], true, next_rows);
-      } else {
-        k_fused_band<false, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], nullptr);
-      }
+      k_fused_band<false, true, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], nullptr);
+      k_trust_fix<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], true, next_rows);
       if (it == iterations - 1)
         k_fused_scatter<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], (float *)in[0], (float *)in[1],
                                                         (float *)in[2]);
@@ -815,18 +996,20 @@ static void launch_iterations(kf_grid live, kf_grid can, kf_field psi, const Dev
 // one): the cooperative launch must fit on the GPU at once.
 // Its shared-memory carveout is kBesideSolveCarveout (kf_internal.h), the
 // one of the kernels that run beside it.
+template <bool kDense>
 static int persistent_blocks_per_sm() {
   static int cached[64] = {};
   static bool carveout[64] = {};
-  kf_prefer_carveout((const void *)k_band_persistent, kBesideSolveCarveout, carveout);
+  const void *kernel = (const void *)k_band_persistent<kDense>;
+  kf_prefer_carveout(kernel, kBesideSolveCarveout, carveout);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   if (!cached[dev]) {
     int n = 0;
-    if (cudaFuncSetAttribute((const void *)k_band_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(PersistShared)) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_band_persistent, kPersistThreads,
-                                                      sizeof(PersistShared)) != cudaSuccess)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PersistSharedOf<kDense>)) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kPersistThreads + (kDense ? kTestThreads : 0),
+                                                      sizeof(PersistSharedOf<kDense>)) != cudaSuccess)
       return 0;
     cached[dev] = std::min(n, 1);
   }
@@ -840,12 +1023,34 @@ static int persistent_blocks_per_sm() {
 // first pass leaves both buffers zero outside its list (it copies p to q),
 // and the solve records the list: the field's buffers are then zero outside
 // its records (kf_field_zero clears just those).
+// The blocks that the dense solver's test warps need in the persistent kernel;
+// 0: it takes another schedule.  That is for large grids (above 1.2 M voxels,
+// kTestChunks: their bands take the groups of the persistent kernel many
+// rounds.  100 iterations at 104^3 with 45 k, 506 k and 1.1 M band voxels: 1.1,
+// 7.9 and 28.7 ms against 2.0, 16.6 and 49.6 on the split schedule; 128^3 with
+// 68 k and 341 k: 2.0 and 4.7 ms against 2.2 and 4.1), a wait limit
+// below the default (the other schedules wait for nothing, so no limit makes
+// them fail) and a stream that is being captured (which refuses the others'
+// graph).
+static unsigned persistent_test_blocks(const DevParams &dp, cudaStream_t s) {
+  if (dp.trust || kf_wait_limit_ns() < kDefaultWaitLimitNs) return 0;
+  const int64_t groups = (dp.count + 3) / 4, sms = kf_num_sms();
+  if (groups > sms * kTestThreads * kTestChunks || persistent_blocks_per_sm<true>() < 1) return 0;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return 0;
+  return (unsigned)std::min((groups + kTestThreads * kTestChunksMin - 1) / (kTestThreads * kTestChunksMin), sms);
+}
+
+// kDense: the dense solver (psi ends in the primary planes; nothing is
+// recorded of what the field's planes hold) with its persistent_test_blocks.
+template <bool kDense>
 static int launch_band_persistent(kf_grid live, kf_grid can, kf_field psi, const DevParams &dp,
-                                  int iterations, IterStats *st, bool p_zero, bool q_zero, cudaStream_t s) {
+                                  int iterations, IterStats *st, bool p_zero, bool q_zero, unsigned least_blocks,
+                                  cudaStream_t s) {
   void *sync = nullptr;
   int rc = kf_field_sync(psi, &sync);
   if (rc) return rc;
-  const int bps = persistent_blocks_per_sm();
+  const int bps = persistent_blocks_per_sm<kDense>();
   if (bps < 1) return kf_fail(KF_ERR_CUDA, "the persistent band pass does not fit on an SM");
   KF_CHECK_CUDA(cudaMemsetAsync(sync, 0, sizeof(GridSync), s));
   FusedArgs even = make_args(live, can, dp, st);
@@ -855,10 +1060,10 @@ static int launch_band_persistent(kf_grid live, kf_grid can, kf_field psi, const
   even.ox = (float *)psi->q[0];
   even.oy = (float *)psi->q[1];
   even.oz = (float *)psi->q[2];
-  int *lst0 = psi->band, *lst1 = psi->band + dp.count;
+  int *lst0 = psi->band, *lst1 = psi->band + dp.count, *shell = lst1 + dp.count;
   int *touched = nullptr;
-  unsigned *touched_n = nullptr;
-  if (p_zero) {
+  unsigned *touched_n = nullptr, *dropped = nullptr;
+  if (p_zero || kDense) {
     KfRecords r;
     rc = kf_field_records(psi, s, &r);
     if (rc) return rc;
@@ -866,20 +1071,28 @@ static int launch_band_persistent(kf_grid live, kf_grid can, kf_field psi, const
     touched = r.touched;
     touched_n = r.touched_n;
   }
+  if (kDense) {
+    dropped = reinterpret_cast<unsigned *>(psi->runs);
+    KF_CHECK_CUDA(cudaMemsetAsync(dropped, 0, (size_t)((dp.count + 31) / 32) * sizeof(unsigned), s));
+  }
   if (p_zero && q_zero)
-    k_band_first_zero<<<(unsigned)num_runs(dp), kThreads, 0, s>>>(even, lst0);
+    k_band_first_zero<<<(unsigned)num_runs(dp), kThreads, 0, s>>>(even, lst0, shell);
   else
-    k_fused_stream<true><<<(unsigned)num_runs(dp), kThreads, 0, s>>>(even, lst0, nullptr, nullptr);
-  KF_CHECK_LAUNCH("dense first pass of the band-only solver");
+    k_band_first<<<(unsigned)num_runs(dp), kThreads, 0, s>>>(even, lst0, shell);
+  KF_CHECK_LAUNCH("dense first pass of the persistent solver");
   GridSync *gs = static_cast<GridSync *>(sync);
   unsigned long long limit = kf_wait_limit_ns();
   int iters = iterations;
   unsigned per_block = kPersistPerBlock;
-  void *args[] = {&even, &lst0, &lst1, &iters, &gs, &limit, &touched, &touched_n, &per_block};
-  KF_CHECK_CUDA(cudaLaunchCooperativeKernel((const void *)k_band_persistent,
-                                            dim3((unsigned)(kf_num_sms() * bps)), dim3(kPersistThreads), args,
-                                            sizeof(PersistShared), s));
-  if (p_zero) {
+  void *args[] = {&even, &lst0, &lst1, &shell, &iters, &gs, &limit, &touched, &touched_n, &per_block,
+                  &least_blocks, &dropped};
+  KF_CHECK_CUDA(cudaLaunchCooperativeKernel(
+      (const void *)k_band_persistent<kDense>, dim3((unsigned)(kf_num_sms() * bps)),
+      dim3(kPersistThreads + (kDense ? kTestThreads : 0)), args, sizeof(PersistSharedOf<kDense>), s));
+  if (kDense) {
+    k_dense_settle<<<(unsigned)kf_num_sms(), kThreads, 0, s>>>(even, touched, touched_n);
+    KF_CHECK_LAUNCH("k_dense_settle");
+  } else if (p_zero) {
     psi->p_state = psi->q_state = kPsiRecorded;
     psi->side_recorded = false;
   }
@@ -892,7 +1105,7 @@ int kf_solve_fused(kf_grid live, kf_grid can, kf_field psi, const DevParams &dp,
   if (rc) return rc;
   rc = kf_field_band_list(psi, &psi->band);
   if (rc) return rc;
-  const int64_t nruns = num_runs(dp);
+  const int64_t nruns = num_runs(dp);  // (the table also holds the persistent kernel's bit per voxel)
   if (psi->runs_cap < nruns) {
     cudaFree(psi->runs);
     psi->runs = nullptr;
@@ -903,7 +1116,10 @@ int kf_solve_fused(kf_grid live, kf_grid can, kf_field psi, const DevParams &dp,
     }
     psi->runs_cap = nruns;
   }
-  if (band_only && !dp.trust) return launch_band_persistent(live, can, psi, dp, iterations, st, p_zero, q_zero, s);
+  if (band_only && !dp.trust)
+    return launch_band_persistent<false>(live, can, psi, dp, iterations, st, p_zero, q_zero, 1u, s);
+  if (const unsigned test_blocks = band_only ? 0u : persistent_test_blocks(dp, s))
+    return launch_band_persistent<true>(live, can, psi, dp, iterations, st, p_zero, q_zero, test_blocks, s);
   int *rows = nullptr;
   if (dp.trust) {
     rc = kf_field_trust_rows(psi, &rows);

@@ -605,6 +605,10 @@ __device__ __forceinline__ void group_statistics(const FusedArgs &a, const Group
 __device__ __forceinline__ bool interior_voxel(const DevParams &dp, int x, int y, int z) {
   return x >= 1 && y >= 1 && z >= 1 && x <= dp.nx - 2 && y <= dp.ny - 2 && z <= dp.nz - 2;
 }
+__host__ __device__ inline int64_t shell_voxels(const DevParams &dp) {
+  const int64_t x = dp.nx > 2 ? dp.nx - 2 : 0, y = dp.ny > 2 ? dp.ny - 2 : 0, z = dp.nz > 2 ? dp.nz - 2 : 0;
+  return dp.count - x * y * z;
+}
 
 // i / d for 0 <= i < 2^31 as (umulhi(i, mul) + i) >> shift (Granlund and
 // Montgomery's division by an invariant integer): 3 instructions where a
@@ -753,9 +757,12 @@ __device__ __forceinline__ void flat_test(const FusedArgs &a, float qx, float qy
 // A run's voxels are listed in index order: the lanes of a band pass then
 // hold neighbours along x, whose psi and phi share cache lines (in the order
 // of an atomic counter, 25 lanes' loads touched about 20 lines).
+// shell (NULL: all are in `list`): the list of the band voxels on the grid's
+// outer shell, counted in *shell_count, in any order.
 template <bool kPassThrough, bool kCheck = false, bool kPsiZero = false>
 __device__ __forceinline__ void stream_flat(const FusedArgs &a, int64_t run, int *__restrict__ list,
-                                            unsigned *count, int2 *__restrict__ range = nullptr) {
+                                            unsigned *count, int2 *__restrict__ range = nullptr,
+                                            int *__restrict__ shell = nullptr, unsigned *shell_count = nullptr) {
   __shared__ unsigned s_warp[kThreads / 32];
   __shared__ unsigned s_base;
   const DevParams &dp = a.dp;
@@ -819,6 +826,18 @@ __device__ __forceinline__ void stream_flat(const FusedArgs &a, int64_t run, int
   if (kCheck) {
     if (hit) atomicAdd(count, (unsigned)__popc(hit));
     return;
+  }
+  if (shell) {
+    for (unsigned h = hit; h; h &= h - 1) {
+      const int bit = __ffs(h) - 1;
+      const int64_t i = voxel(bit);
+      int x, y, z;
+      voxel_xyz(dp, (int)i, x, y, z);
+      if (interior_voxel(dp, x, y, z)) continue;
+      hit &= ~(1u << bit);
+      const unsigned pos = atomicAdd(shell_count, 1u);
+      if (KF_IN_BOUNDS(pos, shell_voxels(dp), KF_SITE_STREAM_LIST)) shell[pos] = (int)i;
+    }
   }
   if (!__syncthreads_or(hit != 0u)) {
     if (range && tid == 0) *range = make_int2(0, 0);
@@ -1052,7 +1071,7 @@ __device__ __forceinline__ void group_step(const FusedArgs &a, const GroupShared
 // planes.  Part 3 and its results (the voxel for the next iteration's list,
 // or -1; the step for group_statistics; whether psi(i) is finite) are role
 // `last`'s; the other warps return -1.
-// Voxels of the outer shell are left alone (group_shell).
+// Voxels of the outer shell are left alone (warp_shell).
 template <int kLoad>
 __device__ __forceinline__ int group_update(const FusedArgs &a, bool odd, int i, int slot, GroupShared &sh, int g,
                                             int w, int last, int lane, GroupStep &t, bool &diverged) {
@@ -1496,41 +1515,34 @@ __device__ __forceinline__ void group_count(const FusedArgs &a, const GroupStep 
   st.active[lane] = active;
 }
 
-// The voxels of the outer shell among a warp's i (-1: none), their new psi to
-// entry `slot`, with their statistics (st, *diverged).  Out of line, and its
-// callers keep next to nothing in registers across it: a value that has to
-// survive a call is kept in memory for good, and after a grid barrier (whose
-// acquire empties L1) every such load goes to L2.  args, sc, st and diverged: in shared
-// memory.
+// Updates voxel i of the outer shell, a warp's (all lanes the same i), and adds
+// its statistics to entry `at` of st and *diverged.  True where the voxel
+// stays in the band.  Out of line, and its callers keep next to nothing in
+// registers across it: a value that has to survive a call is kept in memory
+// for good, and after a grid barrier (whose acquire empties L1) every such
+// load goes to L2.  args, sc, st and diverged: in shared memory.
 template <int kLoad>
-__device__ __noinline__ int group_shell(const FusedArgs *args, ShellScratch *sc, bool odd, int i, int slot,
+__device__ __noinline__ bool warp_shell(const FusedArgs *args, ShellScratch *sc, bool odd, int i, int at,
                                         GroupStats *st, bool *diverged) {
-  const bool have = i >= 0 && KF_IN_BOUNDS(i, args->dp.count, KF_SITE_BAND_LIST) &&
-                    KF_IN_BOUNDS(slot, args->dp.count, KF_SITE_BAND_LIST);
-  int x = 0, y = 0, z = 0, next = -1;
-  if (have) voxel_xyz(args->dp, i, x, y, z);
-  const bool mine = have && !interior_voxel(args->dp, x, y, z);
-  const int lane = threadIdx.x & 31;
-  for (unsigned rest = __ballot_sync(0xffffffffu, mine); rest; rest &= rest - 1) {
-    const int owner = __ffs(rest) - 1;
-    float d[3], s, en, c0[3];
-    shell_gradient<kLoad>(*args, odd, __shfl_sync(0xffffffffu, x, owner), __shfl_sync(0xffffffffu, y, owner),
-                          __shfl_sync(0xffffffffu, z, owner), *sc, d, &s, &en, c0);
-    if (lane != owner) continue;
-    const bool active = in_band(s, args->band_hi, args->band_lo);
+  if (!KF_IN_BOUNDS(i, args->dp.count, KF_SITE_BAND_LIST)) return false;
+  int x, y, z;
+  voxel_xyz(args->dp, i, x, y, z);
+  float d[3], s, en, c0[3];
+  shell_gradient<kLoad>(*args, odd, x, y, z, *sc, d, &s, &en, c0);
+  const bool active = in_band(s, args->band_hi, args->band_lo);
+  if ((threadIdx.x & 31) == 0) {
     if (active) {
       if (!isfinite(c0[0]) || !isfinite(c0[1]) || !isfinite(c0[2])) *diverged = true;
-      st->maxd[lane] = fmaxf(st->maxd[lane], sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0])))));
-      st->energy[lane] += en;
-      ++st->active[lane];
-      next = i;
+      st->maxd[at] = fmaxf(st->maxd[at], sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0])))));
+      st->energy[at] += en;
+      ++st->active[at];
     }
-    plane_out<0>(*args, odd)[slot] = active ? c0[0] + d[0] : c0[0];
-    plane_out<1>(*args, odd)[slot] = active ? c0[1] + d[1] : c0[1];
-    plane_out<2>(*args, odd)[slot] = active ? c0[2] + d[2] : c0[2];
+    plane_out<0>(*args, odd)[i] = active ? c0[0] + d[0] : c0[0];
+    plane_out<1>(*args, odd)[i] = active ? c0[1] + d[1] : c0[1];
+    plane_out<2>(*args, odd)[i] = active ? c0[2] + d[2] : c0[2];
   }
   __syncwarp();
-  return next;
+  return active;
 }
 
 FusedArgs make_args(kf_grid live, kf_grid can, const DevParams &dp, IterStats *st) {

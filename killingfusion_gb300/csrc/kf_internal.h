@@ -44,7 +44,8 @@ struct kf_field_s {
   void *plain_scratch;    // intermediate fields of the per-term solver
   size_t plain_bytes;
   FusedGraph *graph;      // captured fused iteration loop
-  int *band;              // band-voxel lists (two, of one int per voxel each)
+  int *band;              // band-voxel lists (two, of one int per voxel each,
+                          // and one of one int per voxel of the outer shell)
   int2 *runs;             // per run of the dense pass: its entries of the list
   int64_t runs_cap;
   int *rows;              // trust-region step: the first x of each row (y, z)
@@ -165,12 +166,14 @@ struct IterStats {
   int diverged;           // psi non-finite inside the band
   int skipped;            // iteration skipped after convergence
   unsigned int list;      // entries of this iteration's band-voxel list
-  unsigned int cold;      // band voxels the split dense schedule found in a
-                          // run without band voxels at the first iteration
-                          // (never expected: such voxels keep psi)
+                          // (record 1, persistent solvers: of the shell's)
+  unsigned int cold;      // band voxels that the dense solver found outside
+                          // its band (split schedule: in a run without band
+                          // voxels at the first iteration; never expected:
+                          // such voxels keep psi)
   int timeout;            // record 0: a grid-wide wait of a persistent kernel
                           // gave up (KF_ERR_TIMEOUT)
-  int pad_;
+  int executed;           // record 0, persistent dense solver: iterations run
 };
 
 // The bounds-check build's record of one translation unit (kf_bounds.cuh).
@@ -191,6 +194,7 @@ int kf_bounds_tu_reset_mc(long long limit);
 
 // Limit of one device-side wait (kf_set_wait_limit), in nanoseconds.
 unsigned long long kf_wait_limit_ns();
+constexpr unsigned long long kDefaultWaitLimitNs = 1000000000ull;
 // Barrier state of the persistent kernels (GridSync, 32 bytes) of a field,
 // lazily allocated.
 int kf_field_sync(kf_field f, void **out);
