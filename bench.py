@@ -44,12 +44,13 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "voxel-updates/s at 256³ fused vs plain GPU (ψ err≤1e-4 vox); ms/frame; HBM %"
-# Compulsory DRAM bytes of one dense Jacobi iteration: every voxel reads psi
-# (12) and phi_live (4) for the band test; a voxel outside the band keeps its
-# psi, so only the band voxels also read phi_can and write psi (through the
-# side buffer and the scatter: 4 + 12 + 12 + 4 + 12 + 4 with the list).
-ALGO_BYTES_PER_VOXEL = 16
-ALGO_BYTES_PER_BAND_VOXEL = 48
+# Compulsory DRAM bytes of one dense Jacobi iteration from zero psi: every
+# voxel reads phi_live (4) for the band test; psi is read where the solve may
+# have changed it, so the band voxels also read psi (12) and phi_can and write
+# psi (through the side buffer and the scatter: 4 + 12 + 12 + 4 + 12 + 4 with
+# the list).  (The voxels beside them whose psi is read too are not counted.)
+ALGO_BYTES_PER_VOXEL = 4
+ALGO_BYTES_PER_BAND_VOXEL = 60
 MESH_CAP = 4_000_000       # triangles per mesh buffer
 
 
@@ -176,13 +177,20 @@ def mesh_once(capi, L, g, P, buf, cap):
     return n.value
 
 
+def persistent_dense(n3):
+    """Whether a dense solve of n3 voxels is one persistent launch (at most 16
+    groups of four voxels for each of 128 test threads an SM)."""
+    import torch
+    return (n3 + 3) // 4 <= torch.cuda.get_device_properties(0).multi_processor_count * 128 * 16
+
+
 def fused_solve_launches(n3, iters):
-    """Kernel launches of one dense fused solve: a stream pass and a band pass
-    per iteration and one final write-back; on grids of at least 512 runs of
-    2048 voxels the split schedule adds the run split once and a cold pass
-    per iteration after the first."""
-    runs = max((n3 // 4 + 511) // 512, 1)
-    return 3 * iters + 1 if runs >= 512 else 2 * iters + 1
+    """Kernel launches of one dense fused solve: the dense first pass, the
+    persistent solver and its write-back on small grids; above them, the split
+    schedule: a stream pass of the hot runs, one of the cold runs (after the
+    first iteration) and a band pass per iteration, the run split and the
+    final write-back."""
+    return 3 if persistent_dense(n3) else 3 * iters + 1
 
 
 WEIGHTS_TEXT = {
@@ -775,8 +783,8 @@ def run_main(args, rank, world, local):
                      "frac": achieved / peak, "traffic": traffic,
                      "kernel": ("fused psi iteration: k_fused_stream_runs over the hot and the cold runs "
                                 "+ k_fused_band, the cold runs streamed beside the band pass"
-                                if max((N3 // 4 + 511) // 512, 1) >= 512 else
-                                "fused psi iteration (k_fused_stream + k_fused_band)"),
+                                if not persistent_dense(N3) else
+                                "fused psi iteration (k_band_persistent<dense>)"),
                      "algorithmic_bytes_per_iteration": algo_bytes,
                      "algorithmic_bytes_per_voxel": ALGO_BYTES_PER_VOXEL,
                      "algorithmic_bytes_per_band_voxel": ALGO_BYTES_PER_BAND_VOXEL, "peak_source": peak_kind},

@@ -100,7 +100,15 @@ __global__ void __launch_bounds__(kThreads) k_band_first(FusedArgs a, int *__res
 // its cold runs (test only) on a second stream, beside the band pass of the
 // iteration before.  A band voxel found in a cold run is counted in
 // IterStats::cold and fails the solve.
+// Memory bounds the cold passes (16 B a voxel).  Where psi is zero at every
+// voxel of a cold run, as the first iteration found and as it stays, a voxel
+// warps to itself and its test reads phi_live alone (4 B; such a run's entry is
+// ~run).  That is all of them when psi starts at zero: an iteration at 256^3
+// with 14.7 k band voxels (8 % of the runs hot) went from 38.4 to 20.0 us, where
+// hot pass and band pass, one after the other, bound it; 384^3 with 615 k from
+// 186 to 107 us.
 constexpr int kSplitThreads = 1024;
+constexpr int kColdRuns = 4;        // runs a cold block takes
 constexpr int kHotBlocksPerSM = 5;  // resident CTAs of k_fused_stream (48 registers)
 
 __global__ void __launch_bounds__(kSplitThreads) k_split_runs(const int2 *__restrict__ runs, int nruns,
@@ -141,7 +149,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_runs(const int2 *__rest
       if (KF_IN_BOUNDS(h, nruns, KF_SITE_RUNS)) hot[h] = r;
       ++h;
     } else {
-      if (KF_IN_BOUNDS(c, nruns, KF_SITE_RUNS)) cold[c] = r;
+      if (KF_IN_BOUNDS(c, nruns, KF_SITE_RUNS)) cold[c] = runs[r].x ? ~r : r;
       ++c;
     }
   }
@@ -172,11 +180,14 @@ __global__ void __launch_bounds__(kThreads, kCold ? 8 : 5) k_fused_stream_runs(F
   if (kCold) {
     if (a.st[a.iter - 1].skipped) return;
     for (unsigned idx = blockIdx.x; idx < n; idx += gridDim.x) {
-      const int r = run_list[idx];
-      if (KF_IN_BOUNDS(r, max((a.dp.count / 4 + kThreads * kFlatGroups - 1) / (kThreads * kFlatGroups), (int64_t)1),
-                       KF_SITE_RUNS))
+      const int entry = run_list[idx], r = entry < 0 ? ~entry : entry;
+      if (!KF_IN_BOUNDS(r, max((a.dp.count / 4 + kThreads * kFlatGroups - 1) / (kThreads * kFlatGroups), (int64_t)1),
+                        KF_SITE_RUNS))
+        continue;
+      if (entry < 0)
+        stream_flat<false, true, true>(a, r, nullptr, &a.st[a.iter].cold);
+      else
         stream_flat<false, true>(a, r, nullptr, &a.st[a.iter].cold);
-      __syncthreads();
     }
     return;
   }
@@ -915,6 +926,7 @@ static void launch_split_iterations(FusedArgs a, kf_field psi, const DevParams &
   const int64_t nruns = num_runs(dp);
   const unsigned grid = (unsigned)nruns;
   const unsigned hot_grid = (unsigned)std::min<int64_t>(nruns, (int64_t)kf_num_sms() * kHotBlocksPerSM);
+  const unsigned cold_grid = (unsigned)((nruns + kColdRuns - 1) / kColdRuns);
   int *hot = reinterpret_cast<int *>(runs + nruns), *cold = hot + nruns;
   unsigned *counts = reinterpret_cast<unsigned *>(cold + nruns);
   int *lst[2] = {lists, lists + dp.count};
@@ -932,7 +944,7 @@ static void launch_split_iterations(FusedArgs a, kf_field psi, const DevParams &
     } else {
       // cold runs beside the band pass of the iteration before
       cudaStreamWaitEvent(cold_s, fork, 0);
-      launch_prio(k_fused_stream_runs<true>, grid, kThreads, cold_s, mid, a, (const int *)cold,
+      launch_prio(k_fused_stream_runs<true>, cold_grid, kThreads, cold_s, mid, a, (const int *)cold,
                   (const unsigned *)counts, (int *)nullptr, (const int *)nullptr, (int2 *)nullptr);
       launch_prio(k_fused_stream_runs<false>, hot_grid, kThreads, s, hi, a, (const int *)hot,
                   (const unsigned *)counts, lst[it & 1], (const int *)lst[(it + 1) & 1], runs);

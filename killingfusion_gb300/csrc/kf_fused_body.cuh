@@ -813,6 +813,7 @@ __device__ __forceinline__ void stream_flat(const FusedArgs &a, int64_t run, int
     return bit < 4 * kFlatGroups ? 4 * (run * (kThreads * kFlatGroups) + (bit >> 2) * kThreads + tid) + (bit & 3)
                                  : 4 * n4 + tid;
   };
+  const bool any_moved = moved != 0u;
   // voxels that have moved: the warped value is a trilinear gather
   while (moved) {
     const int bit = __ffs(moved) - 1;
@@ -840,7 +841,10 @@ __device__ __forceinline__ void stream_flat(const FusedArgs &a, int64_t run, int
     }
   }
   if (!__syncthreads_or(hit != 0u)) {
-    if (range && tid == 0) *range = make_int2(0, 0);
+    if (range) {
+      const bool zero = !__syncthreads_or(any_moved);
+      if (tid == 0) *range = make_int2(zero ? 1 : 0, 0);  // (k_split_runs)
+    }
     return;
   }
   // one scan of the three counts (group 0, group 1, ragged end), packed
