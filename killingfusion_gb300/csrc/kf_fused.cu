@@ -304,6 +304,11 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
 constexpr int kPersistGroups = 4;
 constexpr int kPersistThreads = kGroupThreads * kPersistGroups;
 constexpr unsigned kPersistPerBlock = 32;
+// Where the grid has blocks to spare, or has them without one more round of the
+// groups, they take the shell's voxels beside the groups' round, which else
+// come after it: 24^3 with 3.5 k band voxels, 100 iterations: 853 us with none,
+// 670, 604 and 561 us with one per 16, 8 and 4 shell voxels.
+constexpr unsigned kShellPerBlock = 4;
 
 // The dense solver of a small grid (persistent_test_blocks) is the same
 // kernel with four more warps a block, which test every voxel outside the
@@ -329,6 +334,7 @@ struct PersistShared {
   ShellScratch scratch[kPersistGroups * kGroupWarps];
   GroupStats shell;                // entry w: warp w's voxels of the grid's outer shell
   unsigned nshell;                 // the grid's list of those
+  unsigned band_blocks;            // the blocks that carry band voxels in their groups
   bool shell_fail;
   bool ok, any_open, any_fail;     // the barrier's verdict
   unsigned long long seen[2];      // grid_verdict's record of the two barrier words
@@ -432,13 +438,22 @@ __device__ __forceinline__ void note_dropped(unsigned *dropped, int v) {
   atomicOr(dropped + (v >> 5), 1u << (v & 31));
 }
 
-// A warp's share of the shell's list: entry w * nblocks + block, and so on.  An
-// entry turns -1 when its voxel leaves the band.
+// The first entry of the shell's list that is warp `warp`'s of this block; every
+// `nblocks` times a block's warps on is its next one.  The blocks without band
+// voxels (from band_blocks on) come first.
+__device__ __forceinline__ unsigned shell_entry(unsigned warp, unsigned band_blocks, unsigned nblocks) {
+  const unsigned extra = nblocks - band_blocks;
+  return blockIdx.x >= band_blocks ? warp * extra + blockIdx.x - band_blocks
+                                   : kPersistGroups * kGroupWarps * extra + warp * band_blocks + blockIdx.x;
+}
+
+// A warp's share of the shell's list.  An entry turns -1 when its voxel leaves
+// the band.
 template <bool kDense>
-__device__ __forceinline__ void shell_round(const DevParams &dp, bool odd, unsigned nblocks, int *shell,
-                                            unsigned *dropped, PersistShared &sh) {
+__device__ __forceinline__ void shell_round(bool odd, unsigned nblocks, int *shell, unsigned *dropped,
+                                            PersistShared &sh) {
   const unsigned warp = threadIdx.x >> 5, stride = kPersistGroups * kGroupWarps * nblocks;
-  for (unsigned j = warp * nblocks + blockIdx.x; j < sh.nshell; j += stride) {
+  for (unsigned j = shell_entry(warp, sh.band_blocks, nblocks); j < sh.nshell; j += stride) {
     const int v = __ldcg(shell + j);
     if (v < 0) continue;
     if (!warp_shell<kPsiL1>(&sh.args, &sh.scratch[warp], odd, v, (int)warp, &sh.shell, &sh.shell_fail) &&
@@ -459,7 +474,7 @@ __device__ __forceinline__ void shell_round(const DevParams &dp, bool odd, unsig
 // in no group's slice, are dealt out to all warps of all blocks, one at a time each.
 template <bool kDense>
 __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, int it, bool last, int *lst0, int *lst1, int *shell,
-                                                          unsigned per, GridSync *sync, unsigned nblocks,
+                                                          unsigned nshell, unsigned per, GridSync *sync, unsigned nblocks,
                                                           unsigned long long limit_ns, unsigned *dropped,
                                                           PersistShared &sh) {
   // group g on warps 4g..4g+3, its roles rotated by g so that every scheduler
@@ -490,7 +505,7 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
     const bool fail = __any_sync(0xffffffffu, diverged);
     if (lane == 0) sh.fail[g] = fail;
     __syncwarp();
-    if (sh.nshell || a.dp.early_exit) {
+    if (nshell || a.dp.early_exit) {
       group_count(a, t, sh.stats[g], lane);
       t.active = false;
     }
@@ -498,11 +513,11 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
     const bool open = a.dp.early_exit && __any_sync(0xffffffffu, sh.stats[g].maxd[lane] > (float)a.dp.threshold);
     if (lane == 0) sh.open[g] = open;
   }
-  if (sh.nshell) shell_round<kDense>(a.dp, odd, nblocks, shell, dropped, sh);
+  if (nshell) shell_round<kDense>(odd, nblocks, shell, dropped, sh);
   __syncthreads();
   if (threadIdx.x == 96 && !last) {
-    bool open = false, fail = sh.shell_fail;
-    for (int k = 0; sh.nshell && a.dp.early_exit && k < kPersistGroups * kGroupWarps; ++k)
+    bool open = false, fail = nshell && sh.shell_fail;
+    for (int k = 0; a.dp.early_exit && nshell && k < kPersistGroups * kGroupWarps; ++k)
       open |= sh.shell.maxd[k] > (float)a.dp.threshold;
 #pragma unroll
     for (int k = 0; k < kPersistGroups; ++k) {
@@ -521,7 +536,7 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
     sh.stats[g].maxd[lane] = 0.f;
     sh.stats[g].energy[lane] = 0.0;
     sh.stats[g].active[lane] = 0u;
-    if (g == 0 && sh.nshell) {
+    if (nshell && g == 0) {
       energy += sh.shell.energy[lane];
       maxd = fmaxf(maxd, sh.shell.maxd[lane]);
       active += sh.shell.active[lane];
@@ -536,7 +551,7 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
       active += __shfl_xor_sync(0xffffffffu, active, o);
     }
     if (lane == 0) {
-      sh.part[g] = BlockStats{energy, active, maxd, sh.fail[g] || (g == 0 && sh.shell_fail)};
+      sh.part[g] = BlockStats{energy, active, maxd, sh.fail[g] || (nshell && g == 0 && sh.shell_fail)};
       sh.n[g] = sh.carried[g];
       sh.carried[g] = 0u;
     }
@@ -588,16 +603,23 @@ __global__ void __maxnreg__(kDense ? 96 : 104)
   extern __shared__ __align__(16) unsigned char smem[];
   PersistShared &sh = *reinterpret_cast<PersistSharedOf<kDense> *>(smem);
   const unsigned nq = __ldcg(&a.st[0].list), nshell = __ldcg(&a.st[1].list);
-  const unsigned nblocks = min(gridDim.x, max((nq + per_block - 1) / per_block,
-                                              max((nshell + kPersistGroups * kGroupWarps - 1) /
-                                                      (kPersistGroups * kGroupWarps), least_blocks)));
+  // blocks for the groups' voxels and, where that takes the groups no more
+  // rounds, blocks for the shell's beside them
+  constexpr unsigned kWarps = kPersistGroups * kGroupWarps, kRound = 32 * kPersistGroups;
+  const unsigned most = gridDim.x, wanted = min(most, (nq + per_block - 1) / per_block);
+  const unsigned rounds = (nq + most * kRound - 1) / (most * kRound);
+  const unsigned least = rounds ? (nq + rounds * kRound - 1) / (rounds * kRound) : 0u;
+  const unsigned shell_blocks = min(most, (nshell + kShellPerBlock - 1) / kShellPerBlock);
+  const unsigned band_blocks = max(min(wanted, max(least, most - shell_blocks)), 1u);
+  const unsigned nblocks = min(most, max(band_blocks + shell_blocks, least_blocks));
   if (blockIdx.x >= nblocks) return;
-  const unsigned groups = nblocks * kPersistGroups;
+  const unsigned groups = band_blocks * kPersistGroups;
   const unsigned per = (nq + groups - 1) / groups;  // a group's slice
   if (threadIdx.x == 0) {
     sh.args = a;
     sh.seen[0] = sh.seen[1] = 0;
     sh.nshell = nshell;
+    sh.band_blocks = band_blocks;
     sh.shell_fail = false;
   }
   if (threadIdx.x < kPersistGroups) {
@@ -622,15 +644,16 @@ __global__ void __maxnreg__(kDense ? 96 : 104)
     for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < nq; k += nblocks * blockDim.x)
       touched[k] = __ldcg(lst0 + k);
     // (a warp's own: iteration 0 already overwrites entries of this list)
-    const unsigned warps = kPersistGroups * kGroupWarps, warp = threadIdx.x >> 5;
-    if (warp < warps) {
-      for (unsigned j = (warp + (threadIdx.x & 31) * warps) * nblocks + blockIdx.x; j < nshell; j += 32 * warps * nblocks)
+    const unsigned warp = threadIdx.x >> 5, stride = kWarps * nblocks;
+    if (warp < kWarps) {
+      for (unsigned j = shell_entry(warp, band_blocks, nblocks) + (threadIdx.x & 31) * stride; j < nshell;
+           j += 32 * stride)
         touched[nq + j] = __ldcg(shell + j);
       __syncwarp();
     }
   }
   for (int it = 0; it < iterations; ++it)
-    if (!persistent_band_iteration<kDense>(a, it, it + 1 == iterations, lst0, lst1, shell, per, sync, nblocks, limit_ns,
+    if (!persistent_band_iteration<kDense>(a, it, it + 1 == iterations, lst0, lst1, shell, nshell, per, sync, nblocks, limit_ns,
                                            dropped, sh)) {
       if (kDense && blockIdx.x == 0 && threadIdx.x == 0) a.st[0].executed = it + 1;
       return;
