@@ -104,9 +104,8 @@ __global__ void __launch_bounds__(kThreads) k_band_first(FusedArgs a, int *__res
 // voxel of a cold run, as the first iteration found and as it stays, a voxel
 // warps to itself and its test reads phi_live alone (4 B; such a run's entry is
 // ~run).  That is all of them when psi starts at zero: an iteration at 256^3
-// with 14.7 k band voxels (8 % of the runs hot) went from 38.4 to 20.0 us, where
-// hot pass and band pass, one after the other, bound it; 384^3 with 615 k from
-// 186 to 107 us.
+// with 14.7 k band voxels went from 38.3 to 20.0 us, where hot pass and band
+// pass, one after the other, bound it; 384^3 with 615 k from 183 to 107 us.
 constexpr int kSplitThreads = 1024;
 constexpr int kColdRuns = 4;        // runs a cold block takes
 constexpr int kHotBlocksPerSM = 5;  // resident CTAs of k_fused_stream (48 registers)
