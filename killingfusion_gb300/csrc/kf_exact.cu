@@ -1054,12 +1054,12 @@ __global__ void __launch_bounds__(kBlock) k_fuse_warped(float *__restrict__ phi1
 // float64 replay of the Jacobi psi update (KillingFusion.cpp:248-352)
 // ---------------------------------------------------------------------------
 // A voxel outside the band keeps psi, so its band test keeps failing: one dense
-// pass (k_exact_first) lists the band and copies the other voxels' psi to the
+// pass (k_exact_first) lists the band and copies psi to the
 // second buffer, and each iteration (k_exact_band) takes the voxels that the
 // one before handed on.
 
 // The band test of the first iteration: lists the band (st[0].list counts
-// it); psi of the other voxels goes to the output buffer too.
+// it); psi goes to the output buffer too.
 __global__ void __launch_bounds__(kBlock) k_exact_first(PhiView<double> live, PsiView<double, double> fin,
                                                         double *__restrict__ ox, double *__restrict__ oy,
                                                         double *__restrict__ oz, DevParams dp, IterStats *st,
@@ -1070,11 +1070,10 @@ __global__ void __launch_bounds__(kBlock) k_exact_first(PhiView<double> live, Ps
     int x, y, z;
     voxel_xyz(i, dp.nx, dp.ny, x, y, z);
     active = in_band(warped_distance(live, fin, x, y, z), dp.band_hi, -dp.unknown_clip);
-    if (!active) {
-      ox[i] = fin.px[i] + 0.0;
-      oy[i] = fin.py[i] + 0.0;
-      oz[i] = fin.pz[i] + 0.0;
-    }
+    // (the band's voxels too: none is left unwritten where a list's check fails)
+    ox[i] = fin.px[i] + 0.0;
+    oy[i] = fin.py[i] + 0.0;
+    oz[i] = fin.pz[i] + 0.0;
   }
   const unsigned ball = __ballot_sync(0xffffffffu, active);
   if (!ball) return;
