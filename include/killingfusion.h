@@ -60,7 +60,9 @@ typedef enum kf_precision {
 
 /* Form of the psi update kernel(s). */
 typedef enum kf_solver {
-  KF_SOLVER_FUSED = 0, /* one stencil pass per iteration, CUDA-graph loop  */
+  KF_SOLVER_FUSED = 0, /* the dense fused stencil, every voxel tested in every
+                          iteration: one persistent launch on small grids, a
+                          captured graph of passes on the others            */
   KF_SOLVER_PLAIN = 1, /* one kernel per energy term, fields through HBM   */
   KF_SOLVER_EXACT = 2, /* float64 replay of the reference (needs KF_F64 psi) */
   KF_SOLVER_BAND = 3,  /* the fused stencil on the band only: a voxel outside
@@ -137,8 +139,9 @@ void kf_params_reference(kf_params *p);
  * truncation band set to trunc_voxels voxels (config.cpp:32-41 comment). */
 void kf_params_paper(kf_params *p, double voxel_size, double trunc_voxels);
 /* Limit, in seconds, of one device-side wait: the grid-wide barrier between
- * the iterations of the persistent kernels (KF_SOLVER_BAND and the batched
- * solver run every iteration in one cooperative launch).  A wait that lasts
+ * the iterations of the persistent kernels (KF_SOLVER_BAND, the batched
+ * solver and, with a limit of at least 1 s, KF_SOLVER_FUSED on small grids run
+ * every iteration in one cooperative launch).  A wait that lasts
  * longer gives up, the kernel ends and the call returns KF_ERR_TIMEOUT, with
  * psi undefined.  No counterpart in the reference, which runs on the CPU.
  * Default 1 s, process-wide; 0 makes every wait give up at once (for testing

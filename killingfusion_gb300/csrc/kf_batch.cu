@@ -10,13 +10,15 @@
 //   k_batch_stream      the dense first pass over every tile of every problem
 //                       (one flat grid; a block finds its problem by binary
 //                       search over the tile prefix) building each problem's
-//                       band list;
+//                       band list, and one of its outer shell's voxels;
 //   k_batch_persistent  every band pass of every iteration, one cooperative
 //                       launch: per iteration the band voxels of all problems
 //                       are one work list cut into chunks that never cross a
 //                       problem; a block scans the per-problem chunk counts
 //                       into a prefix, finds each chunk's problem and hands
-//                       each thread its voxels; statistics stay in registers
+//                       each thread its voxels (a warp each of the shell's);
+//                       an entry turns -1 when its voxel leaves the band, so
+//                       the lists keep their order; statistics stay in registers
 //                       while the block works on one problem, are
 //                       warp-reduced into that problem's shared totals when
 //                       it moves on, and are flushed once per block and

@@ -4,9 +4,9 @@
 // compute-sanitizer is not available where this library is tested, so the
 // kernels of the hot path check, in this build, every index they take from
 // data rather than from their own loop bounds: band-list entries and the
-// positions they are appended at, the dense passes' shared-memory queues and
-// run tables, the in-place write-back, the side lists of warp + fuse and of
-// integration, and the marching-cubes block list and triangle slots.  An index outside its bound is not used (the access is
+// positions they are appended at, the dense passes' run tables, the in-place
+// write-back, the side lists of warp + fuse and of integration, and the
+// marching-cubes block list and triangle slots.  An index outside its bound is not used (the access is
 // skipped) and the first one is recorded -- its site, index and bound -- in
 // a device record that the host reads with kf_bounds_status.  In the normal
 // build every check compiles to nothing.
@@ -25,7 +25,6 @@
 enum KfBoundsSite {
   KF_SITE_BAND_LIST = 1,    // a voxel read from a band list
   KF_SITE_BAND_APPEND = 2,  // a position appended to in a band list
-  KF_SITE_STREAM_QUEUE = 3, // a dense pass's shared-memory queue
   KF_SITE_STREAM_LIST = 4,  // a position the dense pass lists a voxel at
   KF_SITE_WRITE_BACK = 5,   // a voxel or slot of the in-place write-back
   KF_SITE_SIDE_LIST = 7,    // warp + fuse's moved-voxel list

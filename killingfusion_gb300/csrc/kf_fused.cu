@@ -3,13 +3,17 @@
 // KillingFusion::computeEnergyGradient, :399-476) and the CUDA-graph capture
 // of the fixed-iteration loop.
 //
-// An iteration (KF_SOLVER_FUSED) is two passes over psi held in place:
+// KF_SOLVER_FUSED on small grids (persistent_test_blocks) is the band-only
+// solver's persistent launch with warps that test the voxels outside the band.
+// On the others an iteration is two passes over psi held in place, the first
+// one split after the first iteration (k_split_runs):
 //   k_fused_stream (dense)  reads psi and phi_live and applies the band test
 //     of KillingFusion.cpp:272-274.  The warped value phi_live(i + psi(i)) is
 //     phi_live(i) itself when psi(i) == 0 (zero interpolation weights), so only
 //     voxels that have moved gather their 8 corners.  A voxel outside the
 //     band keeps its psi, which therefore need not be written; the voxels
-//     inside are compacted into a list.  16 bytes per voxel.
+//     inside are compacted into a list.  16 bytes per voxel, 4 where psi is
+//     known to be zero.
 //   k_fused_band  evaluates the full gradient of every listed voxel, one
 //     thread per voxel: the thread loads the 20 psi neighbours
 //     of the stencil per component, takes the 25 warped-SDF samples of the
@@ -33,8 +37,8 @@
 //     diagonals;
 //   cell centre (at i + 0.5 + h*o):  m0 + h*(o.m1) + h^2*(pairwise o o.m2)
 //     from eight moments of the cell [i, i+1]^3.
-// Voxels on the grid's outer shell take the generic reference-order path
-// (truncating casts, linear-index wrap, outside values).
+// Voxels on the grid's outer shell take the reference-order path (truncating
+// casts, linear-index wrap, outside values), a warp per voxel.
 #include <algorithm>
 #include <type_traits>
 
@@ -432,9 +436,13 @@ __device__ __forceinline__ unsigned test_outside_band(const FusedArgs &a, int it
 }
 
 // Voxel v has left the band (test_outside_band tests it from the next
-// iteration on).
-__device__ __forceinline__ void note_dropped(unsigned *dropped, int v) {
-  atomicOr(dropped + (v >> 5), 1u << (v & 31));
+// iteration on).  shell: of which list it was; a voxel of the other list (the
+// bounds-check build's unwritten entries) has not left.
+__device__ __forceinline__ void note_dropped(const DevParams &dp, unsigned *dropped, int v, bool shell) {
+  if (!KF_IN_BOUNDS(v, dp.count, KF_SITE_BAND_LIST)) return;
+  int x, y, z;
+  voxel_xyz(dp, v, x, y, z);
+  if (interior_voxel(dp, x, y, z) != shell) atomicOr(dropped + (v >> 5), 1u << (v & 31));
 }
 
 // The first entry of the shell's list that is warp `warp`'s of this block; every
@@ -458,7 +466,7 @@ __device__ __forceinline__ void shell_round(bool odd, unsigned nblocks, int *she
     if (!warp_shell<kPsiL1>(&sh.args, &sh.scratch[warp], odd, v, (int)warp, &sh.shell, &sh.shell_fail) &&
         (threadIdx.x & 31) == 0) {
       __stcg(shell + j, -1);
-      if (kDense) note_dropped(dropped, v);
+      if (kDense) note_dropped(sh.args.dp, dropped, v, true);
     }
     __syncwarp();
   }
@@ -496,7 +504,7 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
   for (unsigned k = 0; k < sh.n[g]; k += 32) {
     if (w == last_role && k > 0) group_count(a, t, sh.stats[g], lane);  // the round before
     const int next = group_update<kPsiL1>(a, odd, v, v, sh.group[g], g, w, last_role, lane, t, diverged);
-    if (kDense && w == last_role && v >= 0 && next < 0) note_dropped(dropped, v);
+    if (kDense && w == last_role && v >= 0 && next < 0) note_dropped(a.dp, dropped, v, false);
     v = k + 32 + lane < sh.n[g] ? __ldcg((odd ? lst1 : lst0) + sh.k0[g] + k + 32 + lane) : -1;
     if (w == last_role) group_carry(next, lane, odd ? lst0 : lst1, per, sh, g);
   }

@@ -241,7 +241,7 @@ int kf_num_sms();
 // `percent` % of the largest shared-memory share
 // (cudaFuncAttributePreferredSharedMemoryCarveout); a preference only.
 //
-// The kernels that run beside the band-only solver's persistent kernel (the
+// The kernels that run beside the single-grid persistent solver's kernel (the
 // frame's integration and meshes, the zeroing of psi) and the solver itself
 // all ask for kBesideSolveCarveout, the largest shared share, which the
 // marching-cubes count pass wants for its cp.async rings.  The solve holds
