@@ -219,7 +219,8 @@ def bench_config(args):
         "frames": "frame 0 canonical, then live frames 1..%d in turn" % (seq.frames - 1),
         "step": "one processNextFrame: integrate, zero psi, %d psi iterations, 3 meshes, warp+fuse" % args.iters,
         "l2": ("inputs fit in L2 (16 B x 64^3 = 4.2 MB per iteration)" if sphere else
-               "inputs larger than L2 (psi 201 MB + phi_live 67 MB read per iteration)"),
+               "a frame's fields are larger than L2 (psi 201 MB, phi and weights of both SDFs 268 MB, all "
+               "read or written every step); an iteration reads phi_live (67 MB) and psi at the band"),
     }
 
 
