@@ -112,7 +112,9 @@ __global__ void __launch_bounds__(kThreads) k_band_first(FusedArgs a, int *__res
 // pass, one after the other, bound it; 384^3 with 615 k from 183 to 107 us.
 constexpr int kSplitThreads = 1024;
 constexpr int kColdRuns = 4;        // runs a cold block takes
-constexpr int kHotBlocksPerSM = 5;  // resident CTAs of k_fused_stream (48 registers)
+// resident CTAs of the hot passes (48 registers).  256^3 with 14.7 k band voxels, 200
+// iterations, with 5, 6 and 8: 4037, 4240 and 4231 us.
+constexpr int kHotBlocksPerSM = 5;
 
 __global__ void __launch_bounds__(kSplitThreads) k_split_runs(const int2 *__restrict__ runs, int nruns,
                                                              int *__restrict__ hot, int *__restrict__ cold,
@@ -230,7 +232,8 @@ __global__ void __launch_bounds__(kThreads, kCold ? 8 : 5) k_fused_stream_runs(F
 // The dense solver runs it beside the cold passes, which live on L1 and
 // occupancy, so it takes no shared memory to speak of: with the groups of four
 // warps of the band-only solver (13 KB a group) the 256^3 iteration took 42.7 us
-// against 41.6 us, and 53 us where their carveout was half the SM's.
+// against 41.6 us, and 53 us where their carveout was half the SM's (measured while
+// every cold run read psi; not since).
 template <bool kCarry, bool kInPlace, bool kTrust = false>
 __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(FusedArgs a, const int *__restrict__ list_in,
                                                              int *__restrict__ list_out) {
