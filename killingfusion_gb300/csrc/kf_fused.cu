@@ -341,6 +341,7 @@ struct PersistShared {
   GroupStats shell;                // entry w: warp w's voxels of the grid's outer shell
   unsigned nshell;                 // the grid's list of those
   unsigned band_blocks;            // the blocks that carry band voxels in their groups
+  bool shell_open[kPersistGroups * kGroupWarps];  // warp w's: some step above the threshold
   bool shell_fail;
   bool ok, any_open, any_fail;     // the barrier's verdict
   unsigned long long seen[2];      // grid_verdict's record of the two barrier words
@@ -523,12 +524,15 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
     const bool open = a.dp.early_exit && __any_sync(0xffffffffu, sh.stats[g].maxd[lane] > (float)a.dp.threshold);
     if (lane == 0) sh.open[g] = open;
   }
-  if (nshell) shell_round<kDense>(odd, nblocks, shell, dropped, sh);
+  if (nshell) {
+    shell_round<kDense>(odd, nblocks, shell, dropped, sh);
+    // (noted here: sh.shell is summed and cleared while the verdict is formed)
+    if (lane == 0) sh.shell_open[warp] = a.dp.early_exit && sh.shell.maxd[warp] > (float)a.dp.threshold;
+  }
   __syncthreads();
   if (threadIdx.x == 96 && !last) {
     bool open = false, fail = nshell && sh.shell_fail;
-    for (int k = 0; a.dp.early_exit && nshell && k < kPersistGroups * kGroupWarps; ++k)
-      open |= sh.shell.maxd[k] > (float)a.dp.threshold;
+    for (int k = 0; a.dp.early_exit && nshell && k < kPersistGroups * kGroupWarps; ++k) open |= sh.shell_open[k];
 #pragma unroll
     for (int k = 0; k < kPersistGroups; ++k) {
       open |= sh.open[k];
