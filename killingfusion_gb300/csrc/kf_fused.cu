@@ -347,7 +347,6 @@ struct PersistShared {
   unsigned long long seen[2];      // grid_verdict's record of the two barrier words
 };
 struct DensePersistShared : PersistShared {
-  unsigned entered[kTestThreads / 32];               // voxels that a test warp found in the band
   unsigned char first[kTestChunks][kTestThreads];    // test_outside_band
 };
 
@@ -496,7 +495,7 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
   if (kDense && g == kPersistGroups) {  // a test warp
     DensePersistShared &d = static_cast<DensePersistShared &>(sh);
     const unsigned entered = __reduce_add_sync(0xffffffffu, test_outside_band(a, it, nblocks, dropped, d.first));
-    if (lane == 0) d.entered[warp - kPersistGroups * kGroupWarps] = entered;
+    if (lane == 0 && entered) atomicAdd(&a.st[it].cold, entered);
     __syncthreads();
     __syncthreads();
     return !last && sh.ok && !sh.any_fail && (!a.dp.early_exit || sh.any_open);
@@ -581,12 +580,6 @@ __device__ __forceinline__ bool persistent_band_iteration(const FusedArgs &a, in
       b.diverged |= sh.part[k].diverged;
     }
     commit_iter_stats(a.st + it, b);
-    if (kDense) {
-      unsigned entered = 0;
-#pragma unroll
-      for (int k = 0; k < kTestThreads / 32; ++k) entered += static_cast<DensePersistShared &>(sh).entered[k];
-      if (entered) atomicAdd(&a.st[it].cold, entered);
-    }
   }
   if (last) return false;
   if (!sh.ok) {
