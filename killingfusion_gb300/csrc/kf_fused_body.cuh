@@ -1017,7 +1017,10 @@ __device__ __forceinline__ void group_middle(const FusedArgs &a, GroupShared &sh
     } else {
       if (interior) group_samples_spread(a, q, w, lane, sh.spread);
 #pragma unroll
-      for (int k = 0; k < 9; ++k) f[k] = sh.spread[max((int)c_group_sample[w][k], 0)][lane];
+      for (int k = 0; k < 9; ++k) {
+        const int j = c_group_sample[w][k];  // (roles 0 and 1 have eight samples; only their own are read)
+        f[k] = sh.spread[j < 0 ? c_group_sample[w][0] : j][lane];
+      }
     }
     float4 o = group_stencils(a, w, f);
     if (w == 2)
