@@ -599,15 +599,38 @@ static void turn_planes(kf_field f, T *aos, bool upload, cudaStream_t s) {
     k_soa_to_aos<T><<<nb, 256, 0, s>>>(aos, x, y, z, f->count);
 }
 
-// Whether p lies in memory of the current device.
-static bool on_this_device(const void *p) {
+// cuMemGetAddressRange, from the driver that the runtime has loaded (NULL: not
+// to be had).
+using AddressRangeFn = int (*)(unsigned long long *base, size_t *size, unsigned long long p);
+static AddressRangeFn address_range_fn() {
+  static const AddressRangeFn fn = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &found) != cudaSuccess) {
+      cudaGetLastError();
+      return (AddressRangeFn) nullptr;
+    }
+    return found == cudaDriverEntryPointSuccess ? (AddressRangeFn)f : nullptr;
+  }();
+  return fn;
+}
+
+// Whether the array at p lies in one allocation of the current device.  (That
+// both its ends lie in the device's memory is not enough: they may be in two
+// allocations.)
+static bool in_device_allocation(const void *p, size_t bytes) {
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   int dev = -1;
-  return at.type == cudaMemoryTypeDevice && cudaGetDevice(&dev) == cudaSuccess && at.device == dev;
+  if (at.type != cudaMemoryTypeDevice || cudaGetDevice(&dev) != cudaSuccess || at.device != dev) return false;
+  unsigned long long base = 0;
+  size_t size = 0;
+  const AddressRangeFn range = address_range_fn();
+  if (!range || range(&base, &size, (unsigned long long)(uintptr_t)p) != 0) return false;
+  return (uintptr_t)p - base + bytes <= size;
 }
 
 // A caller's device array is read or written in place.  Any other -- host
@@ -617,21 +640,28 @@ static bool on_this_device(const void *p) {
 // synchronisation (0.2-0.5 ms a call at 150^3 to 256^3).
 static int field_copy(kf_field f, void *xyz, bool upload, cudaStream_t s) {
   const size_t bytes = 3 * f->count * kf_prec_size(f->prec);
-  const bool direct = ((uintptr_t)xyz & (kf_prec_size(f->prec) - 1)) == 0 && on_this_device(xyz) &&
-                      on_this_device((const char *)xyz + bytes - 1);
+  const bool direct = ((uintptr_t)xyz & (kf_prec_size(f->prec) - 1)) == 0 && in_device_allocation(xyz, bytes);
   void *buf = xyz;
+  cudaError_t e = cudaSuccess;
   if (!direct) {
     KF_CHECK_CUDA(cudaMallocAsync(&buf, bytes, s));
-    if (upload) KF_CHECK_CUDA(cudaMemcpyAsync(buf, xyz, bytes, cudaMemcpyDefault, s));
+    if (upload) e = cudaMemcpyAsync(buf, xyz, bytes, cudaMemcpyDefault, s);
   }
-  if (f->prec == KF_F32)
-    turn_planes<float>(f, (float *)buf, upload, s);
-  else
-    turn_planes<double>(f, (double *)buf, upload, s);
-  KF_CHECK_LAUNCH("field layout conversion");
+  if (e == cudaSuccess) {
+    if (f->prec == KF_F32)
+      turn_planes<float>(f, (float *)buf, upload, s);
+    else
+      turn_planes<double>(f, (double *)buf, upload, s);
+    e = cudaGetLastError();
+  }
   if (!direct) {
-    if (!upload) KF_CHECK_CUDA(cudaMemcpyAsync(xyz, buf, bytes, cudaMemcpyDefault, s));
-    KF_CHECK_CUDA(cudaFreeAsync(buf, s));
+    if (e == cudaSuccess && !upload) e = cudaMemcpyAsync(xyz, buf, bytes, cudaMemcpyDefault, s);
+    const cudaError_t freed = cudaFreeAsync(buf, s);
+    if (e == cudaSuccess) e = freed;
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // (or the next launch's check would report it again)
+    return kf_cuda_fail(e, "field layout conversion");
   }
   KF_CHECK_CUDA(cudaStreamSynchronize(s));
   return KF_OK;
