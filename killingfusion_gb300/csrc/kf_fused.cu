@@ -56,7 +56,7 @@ namespace {
 template <bool kPassThrough>
 __global__ void __launch_bounds__(kThreads) k_fused_stream(FusedArgs a, int *__restrict__ list,
                                                           const int *__restrict__ prev_list,
-                                                          int2 *__restrict__ runs) {
+                                                          int2 *__restrict__ runs, int *__restrict__ shell) {
   if (runs && a.iter > 0 && !a.st[a.iter - 1].skipped) {
     const int2 r = runs[blockIdx.x];
     float *px = const_cast<float *>(a.ix), *py = const_cast<float *>(a.iy), *pz = const_cast<float *>(a.iz);
@@ -75,7 +75,8 @@ __global__ void __launch_bounds__(kThreads) k_fused_stream(FusedArgs a, int *__r
     if (blockIdx.x == 0 && threadIdx.x == 0) a.st[a.iter].skipped = 1;
     return;
   }
-  stream_flat<kPassThrough>(a, blockIdx.x, list, &a.st[a.iter].list, runs ? runs + blockIdx.x : nullptr);
+  stream_flat<kPassThrough>(a, blockIdx.x, list, &a.st[a.iter].list, runs ? runs + blockIdx.x : nullptr, shell,
+                            &a.st[a.iter].shell);
 }
 
 // The band-only solver's first band test when both psi buffers are zero at
@@ -84,13 +85,13 @@ __global__ void __launch_bounds__(kThreads) k_fused_stream(FusedArgs a, int *__r
 // copied by k_fused_stream<true>), and the second buffer already holds
 // every voxel's psi.  The same list as k_fused_stream<true> gives.
 __global__ void __launch_bounds__(kThreads) k_band_first_zero(FusedArgs a, int *__restrict__ list, int *__restrict__ shell) {
-  stream_flat<false, false, true>(a, blockIdx.x, list, &a.st[0].list, nullptr, shell, &a.st[1].list);
+  stream_flat<false, false, true, true>(a, blockIdx.x, list, &a.st[0].list, nullptr, shell, &a.st[1].list);
 }
 
 // The same where psi may be anything: k_fused_stream<true> with the band's
 // voxels of the outer shell in a list of their own.
 __global__ void __launch_bounds__(kThreads) k_band_first(FusedArgs a, int *__restrict__ list, int *__restrict__ shell) {
-  stream_flat<true>(a, blockIdx.x, list, &a.st[0].list, nullptr, shell, &a.st[1].list);
+  stream_flat<true, false, false, true>(a, blockIdx.x, list, &a.st[0].list, nullptr, shell, &a.st[1].list);
 }
 
 // Split dense schedule (grids above persistent_test_blocks' limit).  After the
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(kThreads, kCold ? 8 : 5) k_fused_stream_runs(F
                                                                const unsigned *__restrict__ counts,
                                                                int *__restrict__ list,
                                                                const int *__restrict__ prev_list,
-                                                               int2 *__restrict__ runs) {
+                                                               int2 *__restrict__ runs, int *__restrict__ shell) {
   const unsigned n = counts[kCold ? 1 : 0];
   if (kCold) {
     if (a.st[a.iter - 1].skipped) return;
@@ -218,7 +219,8 @@ __global__ void __launch_bounds__(kThreads, kCold ? 8 : 5) k_fused_stream_runs(F
       }
       __syncthreads();
     }
-    if (!gated) stream_flat<false>(a, r, list, &a.st[a.iter].list, runs + r);
+    if (!gated)
+      stream_flat<false>(a, r, list, &a.st[a.iter].list, runs + r, shell, &a.st[a.iter].shell);
     __syncthreads();
   }
 }
@@ -229,6 +231,13 @@ __global__ void __launch_bounds__(kThreads, kCold ? 8 : 5) k_fused_stream_runs(F
 // st[iter+1].list).  kInPlace: the new psi of list entry k goes to entry k
 // of the output planes, for k_fused_scatter to write back.  kTrust: the
 // trust-region step (dp.trust), followed by k_trust_fix.
+// Voxels of the outer shell (shell_in: their positions in list_in) follow, a
+// warp each (shell_gradient), dealt out over the whole launch: they lie next to
+// one another in index order, up to 2048 of them in a run along a z face.  Bands
+// cut by the face z = 0, 100 iterations at 112^3 (99 k band voxels), 160^3 (201 k)
+// and 256^3 (510 k): 3.4, 4.4 and 10.0 ms; 11.2, 13.4 and 17.1 ms where the warp
+// that met them took them one after the other, 5.9, 7.6 and 15.7 ms with a thread
+// per shell voxel.
 // The dense solver runs it beside the cold passes, which live on L1 and
 // occupancy, so it takes no shared memory to speak of: with the groups of four
 // warps of the band-only solver (13 KB a group) the 256^3 iteration took 42.7 us
@@ -236,7 +245,9 @@ __global__ void __launch_bounds__(kThreads, kCold ? 8 : 5) k_fused_stream_runs(F
 // every cold run read psi; not since).
 template <bool kCarry, bool kInPlace, bool kTrust = false>
 __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(FusedArgs a, const int *__restrict__ list_in,
-                                                             int *__restrict__ list_out) {
+                                                             int *__restrict__ list_out,
+                                                             const int *__restrict__ shell_in,
+                                                             int *__restrict__ shell_out) {
   if (iteration_gated(a.st, a.iter, a.dp)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) a.st[a.iter].skipped = 1;
     return;
@@ -246,10 +257,6 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
   const int nq = (int)a.st[a.iter].list;
   const int total_threads = gridDim.x * kLaneThreads;
   const int rounds = (nq + total_threads - 1) / total_threads;
-  if ((int)blockIdx.x * kLaneThreads < nq) {
-    if (threadIdx.x == 0) s_args = a;
-    __syncthreads();
-  }
   float maxd = 0.f;
   double energy = 0.0;  // this thread's voxels, summed in float64 as the block and grid sums
   unsigned active = 0;
@@ -257,10 +264,39 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
   for (int r = 0; r < rounds; ++r) {
     const int k = (r * gridDim.x + blockIdx.x) * kLaneThreads + threadIdx.x;
     const int v = k < nq ? list_in[k] : -1;
-    // the voxel this thread hands to the next iteration
-    const int next = update_band_voxel<kTrust>(a, s_args, s_shell[threadIdx.x >> 5], v, kInPlace ? k : v, maxd, energy,
-                                               active, diverged);
+    int x, y, z, next = -1;  // next: the voxel this thread hands to the next iteration
+    if (v >= 0) {
+      voxel_xyz(a.dp, v, x, y, z);
+      if (interior_voxel(a.dp, x, y, z))
+        next = update_interior_voxel<kTrust>(a, v, kInPlace ? k : v, maxd, energy, active, diverged);
+    }
     if (kCarry) block_append<kLaneWarps>(next, &a.st[a.iter + 1].list, list_out, a.dp.count);
+  }
+  const unsigned nshell = a.st[a.iter].shell;
+  if (blockIdx.x < nshell) {
+    if (threadIdx.x == 0) s_args = a;
+    __syncthreads();
+    const unsigned warp = threadIdx.x >> 5;
+    for (unsigned j = warp * gridDim.x + blockIdx.x; j < nshell; j += kLaneWarps * gridDim.x) {
+      const int k = shell_in[j];
+      if (!KF_IN_BOUNDS(k, a.dp.count, KF_SITE_BAND_LIST)) continue;
+      const int v = list_in[k];
+      if (!KF_IN_BOUNDS(v, a.dp.count, KF_SITE_BAND_LIST)) continue;
+      int x, y, z;
+      voxel_xyz(a.dp, v, x, y, z);
+      float d[3], s, en, c0[3];
+      shell_gradient<kPsiReadOnly>(s_args, false, x, y, z, s_shell[warp], d, &s, &en, c0);
+      if ((threadIdx.x & 31) == 0) {
+        const int next = settle_band_voxel<kTrust>(a, v, kInPlace ? k : v, x, y, z, s, en, c0, d, maxd, energy, active,
+                                                   diverged);
+        if (kCarry && next >= 0) {
+          const unsigned pos = atomicAdd(&a.st[a.iter + 1].list, 1u), at = atomicAdd(&a.st[a.iter + 1].shell, 1u);
+          if (KF_IN_BOUNDS(pos, a.dp.count, KF_SITE_BAND_APPEND)) list_out[pos] = next;
+          if (KF_IN_BOUNDS(at, shell_voxels(a.dp), KF_SITE_BAND_APPEND)) shell_out[at] = (int)pos;
+        }
+      }
+    }
+    __syncwarp();
   }
   reduce_iter_stats<kLaneThreads>(a.st + a.iter, active, maxd, energy, diverged);
 }
@@ -959,7 +995,7 @@ static void launch_split_iterations(FusedArgs a, kf_field psi, const DevParams &
   const unsigned cold_grid = (unsigned)((nruns + kColdRuns - 1) / kColdRuns);
   int *hot = reinterpret_cast<int *>(runs + nruns), *cold = hot + nruns;
   unsigned *counts = reinterpret_cast<unsigned *>(cold + nruns);
-  int *lst[2] = {lists, lists + dp.count};
+  int *lst[2] = {lists, lists + dp.count}, *shell = lists + 2 * dp.count;
   a.ix = (const float *)psi->p[0];
   a.iy = (const float *)psi->p[1];
   a.iz = (const float *)psi->p[2];
@@ -969,19 +1005,20 @@ static void launch_split_iterations(FusedArgs a, kf_field psi, const DevParams &
   for (int it = 0; it < iterations; ++it) {
     a.iter = it;
     if (it == 0) {
-      launch_prio(k_fused_stream<false>, grid, kThreads, s, hi, a, lst[0], lst[1], runs);
+      launch_prio(k_fused_stream<false>, grid, kThreads, s, hi, a, lst[0], lst[1], runs, shell);
       launch_prio(k_split_runs, 1, kSplitThreads, s, hi, (const int2 *)runs, (int)nruns, hot, cold, counts);
     } else {
       // cold runs beside the band pass of the iteration before
       cudaStreamWaitEvent(cold_s, fork, 0);
       launch_prio(k_fused_stream_runs<true>, cold_grid, kThreads, cold_s, mid, a, (const int *)cold,
-                  (const unsigned *)counts, (int *)nullptr, (const int *)nullptr, (int2 *)nullptr);
+                  (const unsigned *)counts, (int *)nullptr, (const int *)nullptr, (int2 *)nullptr,
+                  (int *)nullptr);
       launch_prio(k_fused_stream_runs<false>, hot_grid, kThreads, s, hi, a, (const int *)hot,
-                  (const unsigned *)counts, lst[it & 1], (const int *)lst[(it + 1) & 1], runs);
+                  (const unsigned *)counts, lst[it & 1], (const int *)lst[(it + 1) & 1], runs, shell);
     }
     if (it + 1 < iterations) cudaEventRecord(fork, s);
     launch_prio(k_fused_band<false, true>, band_blocks, kLaneThreads, s, hi, a, (const int *)lst[it & 1],
-                (int *)nullptr);
+                (int *)nullptr, (const int *)shell, (int *)nullptr);
     if (it == iterations - 1)
       launch_prio(k_fused_scatter, band_blocks, kThreads, s, hi, a, (const int *)lst[it & 1],
                   (float *)psi->p[0], (float *)psi->p[1], (float *)psi->p[2]);
@@ -1002,6 +1039,7 @@ static void launch_iterations(kf_grid live, kf_grid can, kf_field psi, const Dev
   FusedArgs a = make_args(live, can, dp, st);
   void *buf[2][3] = {{psi->p[0], psi->p[1], psi->p[2]}, {psi->q[0], psi->q[1], psi->q[2]}};
   int *lst[2] = {lists, lists + dp.count};
+  int *shell[2] = {lists + 2 * dp.count, lists + 2 * dp.count + shell_voxels(dp)};
   const int nrows = dp.ny * dp.nz;
   if (dp.trust) cudaMemsetAsync(rows, 0x7f, (size_t)nrows * sizeof(int), s);
   for (int it = 0; it < iterations; ++it) {
@@ -1019,16 +1057,17 @@ static void launch_iterations(kf_grid live, kf_grid can, kf_field psi, const Dev
     int *next_rows = dp.trust ? rows + ((it + 1) & 1) * nrows : nullptr;
     if (!band_only) {
       // lists alternate so that a run can still read the previous iteration's
-      k_fused_stream<false><<<grid, block, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1], runs);
-      k_fused_band<false, true, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], nullptr);
+      k_fused_stream<false><<<grid, block, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1], runs, shell[0]);
+      k_fused_band<false, true, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], nullptr, shell[0], nullptr);
       k_trust_fix<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], true, next_rows);
       if (it == iterations - 1)
         k_fused_scatter<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], (float *)in[0], (float *)in[1],
                                                         (float *)in[2]);
     } else {
-      if (it == 0) k_fused_stream<true><<<grid, block, 0, s>>>(a, lst[0], nullptr, nullptr);
+      if (it == 0) k_fused_stream<true><<<grid, block, 0, s>>>(a, lst[0], nullptr, nullptr, shell[0]);
       // (with the trust-region step; without it the solver is k_band_persistent)
-      k_fused_band<true, false, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1]);
+      k_fused_band<true, false, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1],
+                                                                         shell[it & 1], shell[(it + 1) & 1]);
       k_trust_fix<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], false, next_rows);
     }
   }
@@ -1228,7 +1267,7 @@ int kf_solve_pervoxel(kf_grid live, kf_grid can, kf_field psi, const DevParams &
   a.iter = 0;
   const unsigned grid = (unsigned)std::max<int64_t>((dp.count / 4 + kThreads * kFlatGroups - 1) /
                                                         (kThreads * kFlatGroups), 1);
-  k_fused_stream<false><<<grid, kThreads, 0, s>>>(a, psi->band, nullptr, nullptr);
+  k_fused_stream<false><<<grid, kThreads, 0, s>>>(a, psi->band, nullptr, nullptr, nullptr);
   // the colours' counts and cursors, and their lists in the second band list
   void *sync = nullptr;
   rc = kf_field_sync(psi, &sync);

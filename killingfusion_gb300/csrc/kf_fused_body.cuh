@@ -757,9 +757,10 @@ __device__ __forceinline__ void flat_test(const FusedArgs &a, float qx, float qy
 // A run's voxels are listed in index order: the lanes of a band pass then
 // hold neighbours along x, whose psi and phi share cache lines (in the order
 // of an atomic counter, 25 lanes' loads touched about 20 lines).
-// shell (NULL: all are in `list`): the list of the band voxels on the grid's
-// outer shell, counted in *shell_count, in any order.
-template <bool kPassThrough, bool kCheck = false, bool kPsiZero = false>
+// shell (or NULL): a list of the band voxels on the grid's outer shell, counted
+// in *shell_count, in any order.  kShellApart: of the voxels, which are then not
+// in `list`; otherwise of their positions there.
+template <bool kPassThrough, bool kCheck = false, bool kPsiZero = false, bool kShellApart = false>
 __device__ __forceinline__ void stream_flat(const FusedArgs &a, int64_t run, int *__restrict__ list,
                                             unsigned *count, int2 *__restrict__ range = nullptr,
                                             int *__restrict__ shell = nullptr, unsigned *shell_count = nullptr) {
@@ -828,7 +829,7 @@ __device__ __forceinline__ void stream_flat(const FusedArgs &a, int64_t run, int
     if (hit) atomicAdd(count, (unsigned)__popc(hit));
     return;
   }
-  if (shell) {
+  if (kShellApart) {
     for (unsigned h = hit; h; h &= h - 1) {
       const int bit = __ffs(h) - 1;
       const int64_t i = voxel(bit);
@@ -875,7 +876,15 @@ __device__ __forceinline__ void stream_flat(const FusedArgs &a, int64_t run, int
   for (int g = 0; g < 3; ++g) {
     for (unsigned h = g < 2 ? hit >> (4 * g) & 15u : hit >> 8; h; h &= h - 1) {
       const unsigned pos = base + at[g]++;
-      if (KF_IN_BOUNDS(pos, dp.count, KF_SITE_STREAM_LIST)) list[pos] = (int)voxel(4 * g + __ffs(h) - 1);
+      const int i = (int)voxel(4 * g + __ffs(h) - 1);
+      if (KF_IN_BOUNDS(pos, dp.count, KF_SITE_STREAM_LIST)) list[pos] = i;
+      if (!kShellApart && shell) {
+        int x, y, z;
+        voxel_xyz(dp, i, x, y, z);
+        if (interior_voxel(dp, x, y, z)) continue;
+        const unsigned j = atomicAdd(shell_count, 1u);
+        if (KF_IN_BOUNDS(j, shell_voxels(dp), KF_SITE_STREAM_LIST)) shell[j] = (int)pos;
+      }
     }
   }
   // where this run's band voxels sit in the list (for the next iteration's
@@ -1073,7 +1082,7 @@ __device__ __forceinline__ void group_step(const FusedArgs &a, const GroupShared
 }
 
 // Updates the voxels i (-1: none) of the lanes of group g, as
-// update_band_voxel does for one: every thread of the group calls it, in role
+// update_interior_voxel does for one: every thread of the group calls it, in role
 // w, with its lane's voxel, whose new psi goes to entry `slot` of the output
 // planes.  Part 3 and its results (the voxel for the next iteration's list,
 // or -1; the step for group_statistics; whether psi(i) is finite) are role
@@ -1312,8 +1321,17 @@ __device__ __forceinline__ int settle_band_voxel(const FusedArgs &a, int i, int 
   return next;
 }
 
-// As update_band_voxel, for a voxel known not to lie on the outer shell.
-template <bool kTrust, int kLoad>
+// Update band voxel i, which does not lie on the outer shell, and write its new
+// psi to entry `slot` of the output planes (slot == i for ping-pong buffers; the
+// voxel's list position for in-place updates).  The voxel is re-tested with its
+// warped value: one outside the band keeps its psi (it left the band in the
+// previous iteration).  Returns the voxel for the next iteration's list (-1 if
+// it left the band) and accumulates the statistics.
+// kTrust: the trust-region step (dp.trust set), a separate instantiation so
+// that the plain band pass carries no call to it.
+// kLoad: how psi is read (PsiLoad); the persistent passes, which write psi
+// between iterations, read it with kPsiL1.
+template <bool kTrust, int kLoad = kPsiReadOnly>
 __device__ __forceinline__ int update_interior_voxel(const FusedArgs &a, int i, int slot, float &maxd, double &energy,
                                                      unsigned &active, bool &diverged) {
   if (!KF_IN_BOUNDS(i, a.dp.count, KF_SITE_BAND_LIST) || !KF_IN_BOUNDS(slot, a.dp.count, KF_SITE_BAND_LIST)) return -1;
@@ -1322,44 +1340,6 @@ __device__ __forceinline__ int update_interior_voxel(const FusedArgs &a, int i, 
   float d[3], s, en, c0[3];
   gradient_lane<kLoad>(a, x, y, z, i, d, s, en, c0);
   return settle_band_voxel<kTrust>(a, i, slot, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
-}
-
-// Update band voxel i of each lane (-1: none; every lane of the warp calls it)
-// and write its new psi to entry `slot` of the output planes (slot == i for
-// ping-pong buffers; the voxel's list position for in-place updates).  The
-// voxel is re-tested with its warped value: one outside the band keeps its
-// psi (it left the band in the previous iteration).  Returns the voxel for
-// the next iteration's list (-1 if it left the band) and accumulates the
-// statistics.
-// kTrust: the trust-region step (dp.trust set), a separate instantiation so
-// that the plain band pass carries no call to it.
-// kLoad: how psi is read (PsiLoad); the persistent passes, which write psi
-// between iterations, read it with kPsiL1.
-// args: a copy of a in shared memory, sc: the warp's (shell_gradient).
-template <bool kTrust = false, int kLoad = kPsiReadOnly>
-__device__ __forceinline__ int update_band_voxel(const FusedArgs &a, const FusedArgs &args, ShellScratch &sc, int i,
-                                                 int slot, float &maxd, double &energy, unsigned &active,
-                                                 bool &diverged) {
-  const DevParams &dp = a.dp;
-  const bool have =
-      i >= 0 && KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST) && KF_IN_BOUNDS(slot, dp.count, KF_SITE_BAND_LIST);
-  int x = 0, y = 0, z = 0, next = -1;
-  if (have) voxel_xyz(dp, i, x, y, z);
-  const bool interior = have && interior_voxel(dp, x, y, z);
-  if (interior) {
-    float d[3], s, en, c0[3];
-    gradient_lane<kLoad>(a, x, y, z, i, d, s, en, c0);
-    next = settle_band_voxel<kTrust>(a, i, slot, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
-  }
-  for (unsigned rest = __ballot_sync(0xffffffffu, have && !interior); rest; rest &= rest - 1) {
-    const int owner = __ffs(rest) - 1;
-    float d[3], s, en, c0[3];
-    shell_gradient<kLoad>(args, false, __shfl_sync(0xffffffffu, x, owner), __shfl_sync(0xffffffffu, y, owner),
-                          __shfl_sync(0xffffffffu, z, owner), sc, d, &s, &en, c0);
-    if ((int)(threadIdx.x & 31) == owner)
-      next = settle_band_voxel<kTrust>(a, i, slot, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
-  }
-  return next;
 }
 
 // ---------------------------------------------------------------------------

@@ -45,7 +45,7 @@ struct kf_field_s {
   size_t plain_bytes;
   FusedGraph *graph;      // captured fused iteration loop
   int *band;              // band-voxel lists (two, of one int per voxel each,
-                          // and one of one int per voxel of the outer shell)
+                          // and two of one int per voxel of the outer shell)
   int2 *runs;             // per run of the dense pass: its entries of the list
   int64_t runs_cap;
   int *rows;              // trust-region step: the first x of each row (y, z)
@@ -174,6 +174,9 @@ struct IterStats {
   int timeout;            // record 0: a grid-wide wait of a persistent kernel
                           // gave up (KF_ERR_TIMEOUT)
   int executed;           // record 0, persistent dense solver: iterations run
+  unsigned int shell;     // k_fused_band: this iteration's list entries of the
+                          // outer shell (a list of their positions)
+  int pad_;
 };
 
 // The bounds-check build's record of one translation unit (kf_bounds.cuh).
