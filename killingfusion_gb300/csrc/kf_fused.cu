@@ -361,6 +361,7 @@ constexpr unsigned kShellPerBlock = 4;
 // against 15.6, 100^3 with 41.8 k 11 against 20.5.
 constexpr int kTestThreads = 128;
 constexpr int kTestChunks = 16;    // most groups of four voxels a test thread takes
+constexpr int kTestFlight = 2;     // voxels whose corners a lane loads at a time (test_moved)
 constexpr int kTestChunksMin = 4;  // the fewest worth a block
 
 struct PersistShared {
@@ -404,6 +405,73 @@ __device__ __forceinline__ void group_carry(int next, int lane, int *__restrict_
   __syncwarp();
 }
 
+// The band test of moved voxels by a whole warp, for voxels i0 .. i0 + 127: lane l's
+// `moved` names those of i0 + 4 l .. + 3 to test, its result those of them that are
+// in the band (warped_value).  A lane takes every 32nd voxel, so that the lanes'
+// gathers touch neighbouring cells, kTestFlight of them at a time.
+// What bounds it, and the dense solver where psi is non-zero everywhere: the
+// instructions of the four test warps, one on each scheduler.  60 iterations at
+// 64^3, 100^3 and 104^3 from a smooth psi: 0.75, 1.76 and 2.23 ms, from random
+// vectors of 0.4 voxel 0.78, 1.95 and 2.36 ms; 1.07, 4.23 and 5.25 ms, 1.93, 5.07 and
+// 6.80 ms where each lane gathered its own four voxels one after the other; four at
+// a time 0.81, 1.77 and 2.45 ms, 0.82, 2.19 and 2.88 ms (spills).  On the split
+// schedule's two passes an iteration: 1.34, 1.67 and 2.46 ms, 1.79, 2.18 and 2.50 ms.
+__device__ __forceinline__ unsigned test_moved(const FusedArgs &a, const float *px, const float *py, const float *pz,
+                                               int i0, unsigned moved) {
+  const DevParams &dp = a.dp;
+  const int lane = threadIdx.x & 31;
+  unsigned hit = 0;
+#pragma unroll 1
+  for (int e0 = 0; e0 < 4; e0 += kTestFlight) {
+    float t[kTestFlight][3], v[kTestFlight][8];
+    bool test[kTestFlight], in[kTestFlight], any = false;
+#pragma unroll
+    for (int e = 0; e < kTestFlight; ++e) {
+      test[e] = __shfl_sync(0xffffffffu, moved, 8 * (e0 + e) + (lane >> 2)) >> (lane & 3) & 1u;
+      any = any || test[e];
+    }
+    if (!__any_sync(0xffffffffu, any)) continue;
+#pragma unroll
+    for (int e = 0; e < kTestFlight; ++e) {
+      const int i = test[e] ? i0 + 32 * (e0 + e) + lane : 0;
+      t[e][0] = __ldcg(px + i);
+      t[e][1] = __ldcg(py + i);
+      t[e][2] = __ldcg(pz + i);
+    }
+#pragma unroll
+    for (int e = 0; e < kTestFlight; ++e) {
+      int x, y, z;
+      voxel_xyz(dp, test[e] ? i0 + 32 * (e0 + e) + lane : 0, x, y, z);
+      t[e][0] = fsb(fa(fa((float)x, t[e][0]), 0.5f), 0.5f);
+      t[e][1] = fsb(fa(fa((float)y, t[e][1]), 0.5f), 0.5f);
+      t[e][2] = fsb(fa(fa((float)z, t[e][2]), 0.5f), 0.5f);
+      const int b0 = (int)t[e][0], b1 = (int)t[e][1], b2 = (int)t[e][2];
+      in[e] = (unsigned)b0 < (unsigned)(dp.nx - 1) && (unsigned)b1 < (unsigned)(dp.ny - 1) &&
+              (unsigned)b2 < (unsigned)(dp.nz - 1);
+      const bool load = test[e] && in[e];
+      const float *p = a.live + (load ? (b2 * dp.ny + b1) * dp.nx + b0 : 0);
+      const int one = load ? 1 : 0, row = load ? dp.nx : 0, plane = load ? dp.nx * dp.ny : 0;
+      v[e][0] = __ldg(p);
+      v[e][1] = __ldg(p + one);
+      v[e][2] = __ldg(p + row);
+      v[e][3] = __ldg(p + row + one);
+      v[e][4] = __ldg(p + plane);
+      v[e][5] = __ldg(p + plane + one);
+      v[e][6] = __ldg(p + plane + row);
+      v[e][7] = __ldg(p + plane + row + one);
+    }
+#pragma unroll
+    for (int e = 0; e < kTestFlight; ++e) {
+      float s = lerp3f(v[e], fsb(t[e][0], (float)(int)t[e][0]), fsb(t[e][1], (float)(int)t[e][1]),
+                       fsb(t[e][2], (float)(int)t[e][2]));
+      if (test[e] && !in[e]) s = phi_tri(a, t[e][0], t[e][1], t[e][2]);  // some corners lie outside the grid
+      const unsigned ball = __ballot_sync(0xffffffffu, test[e] && in_band(s, a.band_hi, a.band_lo));
+      if (lane >> 3 == e0 + e) hit = ball >> (4 * (lane & 7)) & 15u;
+    }
+  }
+  return hit;
+}
+
 // A test warp's iteration.  Thread t of the grid's test threads takes the
 // groups of four voxels t, t + threads, ...; `first` keeps the four bits of each,
 // the voxels in the band at iteration 0.  Those are in the band list, whose
@@ -420,6 +488,7 @@ __device__ __forceinline__ unsigned test_outside_band(const FusedArgs &a, int it
   const int threads = (int)nblocks * kTestThreads;
   const float *px = plane_in<0>(a, odd), *py = plane_in<1>(a, odd), *pz = plane_in<2>(a, odd);
   unsigned entered = 0;
+  unsigned long long todo = 0;  // bits 4c .. 4c + 3: the moved voxels of the c-th group
   const int t = (int)threadIdx.x - kPersistThreads;
   int c = 0;
 #pragma unroll 2
@@ -459,15 +528,22 @@ __device__ __forceinline__ unsigned test_outside_band(const FusedArgs &a, int it
       moved = (moved & ~was) | left;  // (one that left is tested as the band pass did)
     }
     hit &= valid;
-    for (moved &= valid; moved; moved &= moved - 1) {
-      const int b = __ffs(moved) - 1, i = 4 * q + b;
-      int vx, vy, vz;
-      voxel_xyz(dp, i, vx, vy, vz);
-      const float w = warped_value(a, vx, vy, vz, __ldcg(px + i), __ldcg(py + i), __ldcg(pz + i));
-      if (in_band(w, a.band_hi, a.band_lo)) hit |= 1u << b;
-    }
+    todo |= (unsigned long long)(moved & valid) << (4 * c);
     if (it == 0)
       first[c][t] = (unsigned char)hit;
+    else
+      entered += (unsigned)__popc(hit);
+  }
+  // The voxels that have moved, in a pass of their own: where there are none, as
+  // outside the band with psi from zero, the loop above is all there is.
+  if (!__any_sync(0xffffffffu, todo != 0ull)) return entered;
+  int q0 = (int)blockIdx.x * kTestThreads + (t & ~31);
+  for (c = 0; q0 < n4 && c < kTestChunks; q0 += threads, ++c) {
+    const unsigned moved = (unsigned)(todo >> (4 * c)) & 15u;
+    if (!__any_sync(0xffffffffu, moved != 0u)) continue;
+    const unsigned hit = test_moved(a, px, py, pz, 4 * q0, moved);
+    if (it == 0)
+      first[c][t] |= (unsigned char)hit;
     else
       entered += (unsigned)__popc(hit);
   }
