@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
       if (!KF_IN_BOUNDS(v, a.dp.count, KF_SITE_BAND_LIST)) continue;
       int x, y, z;
       voxel_xyz(a.dp, v, x, y, z);
+      if (interior_voxel(a.dp, x, y, z)) continue;  // (the bounds-check build's unwritten entries)
       float d[3], s, en, c0[3];
       shell_gradient<kPsiReadOnly>(s_args, false, x, y, z, s_shell[warp], d, &s, &en, c0);
       if ((threadIdx.x & 31) == 0) {
