@@ -851,13 +851,29 @@ __global__ void __launch_bounds__(kThreads) k_trust_fix(FusedArgs a, const int *
 // in the reference's sequential loop, and the result does not depend on
 // scheduling.
 
-// The dense pass's list sorted into one list per colour: counts[c] voxels
-// from the sum of counts[0..c) on.  Two launches, kFill = false to count
-// (counts are zero before), then kFill = true to write (cursors are).
-template <bool kFill>
+// The dense pass's list sorted by colour: the voxels inside from the front of the
+// colour's part of `out` (counts[c]), those on the grid's outer shell from its back
+// (counts[8 + c]).  The part of a colour, [start[c], start[c + 1]), has room for
+// all the grid's voxels of it.
+struct ColourParts {
+  unsigned start[9];
+};
+constexpr int kColourCounts = 16;
+
+static ColourParts colour_parts(const DevParams &dp) {
+  ColourParts p;
+  p.start[0] = 0;
+  for (int c = 0; c < 8; ++c) {
+    const unsigned x = c & 1 ? dp.nx / 2 : (dp.nx + 1) / 2, y = c & 2 ? dp.ny / 2 : (dp.ny + 1) / 2,
+                   z = c & 4 ? dp.nz / 2 : (dp.nz + 1) / 2;
+    p.start[c + 1] = p.start[c] + x * y * z;
+  }
+  return p;
+}
+
 __global__ void __launch_bounds__(kThreads) k_colour_lists(FusedArgs a, const int *__restrict__ list,
-                                                          unsigned *__restrict__ counts,
-                                                          unsigned *__restrict__ cursors, int *__restrict__ out) {
+                                                          unsigned *__restrict__ counts, ColourParts parts,
+                                                          int *__restrict__ out) {
   const unsigned nq = a.st[0].list;
   const unsigned lane = threadIdx.x & 31;
   // whole warps loop together
@@ -866,17 +882,17 @@ __global__ void __launch_bounds__(kThreads) k_colour_lists(FusedArgs a, const in
     if (v >= 0 && !KF_IN_BOUNDS(v, a.dp.count, KF_SITE_BAND_LIST)) v = -1;
     int x = 0, y = 0, z = 0;
     if (v >= 0) voxel_xyz(a.dp, v, x, y, z);
-    const int colour = v >= 0 ? (x & 1) | (y & 1) << 1 | (z & 1) << 2 : 8;
-    const unsigned same = __match_any_sync(0xffffffffu, colour);
+    const int colour = (x & 1) | (y & 1) << 1 | (z & 1) << 2;
+    const bool inside = interior_voxel(a.dp, x, y, z);
+    const int which = v < 0 ? kColourCounts : colour + (inside ? 0 : 8);
+    const unsigned same = __match_any_sync(0xffffffffu, which);
     if (v < 0) continue;
     const int leader = __ffs(same) - 1;
-    unsigned base = 0;
-    if ((int)lane == leader) base = atomicAdd((kFill ? cursors : counts) + colour, (unsigned)__popc(same));
-    if (kFill) {
-      base = __shfl_sync(same, base, leader) + (unsigned)__popc(same & ((1u << lane) - 1u));
-      for (int c = 0; c < colour; ++c) base += counts[c];
-      if (KF_IN_BOUNDS(base, a.dp.count, KF_SITE_BAND_APPEND)) out[base] = v;
-    }
+    unsigned at = 0;
+    if ((int)lane == leader) at = atomicAdd(counts + which, (unsigned)__popc(same));
+    at = __shfl_sync(same, at, leader) + (unsigned)__popc(same & ((1u << lane) - 1u));
+    const unsigned pos = inside ? parts.start[colour] + at : parts.start[colour + 1] - 1u - at;
+    if (KF_IN_BOUNDS(pos, a.dp.count, KF_SITE_BAND_APPEND)) out[pos] = v;
   }
 }
 
@@ -896,47 +912,89 @@ __device__ __forceinline__ bool pervoxel_done(const FusedArgs &a, float dn, cons
   return !(dn / a.alpha > thr) || iter >= max_iters;
 }
 
-// The voxels of one colour, one warp each (warp_step): a voxel's neighbours are
-// loaded once and its psi stays on chip until the last step, so a step costs no
-// trip to memory beyond the samples' corners (L1).
+// The voxels of one colour.  Few of them take a warp each (warp_step): a voxel's
+// neighbours are loaded once and its psi stays on chip until the last step, so a
+// step costs no trip to memory beyond the samples' corners (L1).  Many take a
+// thread each (gradient_lane, the same roundings).  Voxels of the outer shell take a
+// warp each (shell_gradient).
 // Statistics: record 0 voxels (list, from the dense pass), last step, last
 // monitored energy, divergence; record 1 voxels that hit the cap (active) and
 // the most steps of one voxel (list).
-// What bounds it: the chain of a step times the steps of the slowest voxel.
-// One thread per voxel of the unsorted list (7 of 8 lanes of another colour,
-// 60 psi loads a step) took 2.4 us a step.
+// What bounds it: the chain of a step times the steps of the slowest voxel, and with
+// a warp each, above a voxel or so per resident warp, the instructions (350 a warp
+// and step against 62 a voxel as lanes of full warps).  60 steps from zero with 5.3 k,
+// 17 k, 27 k, 42 k and 107 k band voxels: a warp each 640, 818, 1345, 1954 and 4259 us, a
+// thread each 1110, 1157, 1158, 1166 and 1210 us.  Samples that do not share a cell
+// slow the threads alone (10 steps from a smooth psi, 20 k voxels: 299 us a warp each,
+// 640 us a thread each), so the line lies a little above one voxel per resident
+// warp.  One or two steps do not earn back the warps' start: 2 steps with 5.3 k, 10 k,
+// 14 k and 17 k voxels take 97, 111, 129 and 146 us a warp each, 111, 107, 104 and 109
+// us a thread each.
+// (A thread per voxel of the unsorted list, most lanes of another colour: 60 steps
+// 1170, 1184, 1441, 1607 and 2982 us.)
 constexpr int kPervoxelWarps = 4;
 constexpr int kPervoxelBlocksPerSM = 4;
+constexpr int kPervoxelFewSteps = 2;
 
 __global__ void __launch_bounds__(32 * kPervoxelWarps, kPervoxelBlocksPerSM)
-    k_pervoxel(FusedArgs a, const int *__restrict__ list, const unsigned *__restrict__ counts, int max_iters,
-               int colour) {
+    k_pervoxel(FusedArgs a, const int *__restrict__ list, const unsigned *__restrict__ counts, unsigned first,
+               unsigned end, int max_iters, int colour) {
   __shared__ WarpShared s_warp[kPervoxelWarps];
   __shared__ ShellScratch s_shell[kPervoxelWarps];
   __shared__ FusedArgs s_args;
   const DevParams &dp = a.dp;
-  unsigned first = 0;
-  for (int c = 0; c < colour; ++c) first += counts[c];
-  const unsigned nq = counts[colour];
-  if (blockIdx.x * kPervoxelWarps >= nq) return;
+  // (more than the colour's part holds: the bounds-check build's unwritten entries,
+  // which may name one voxel many times)
+  const unsigned ni = min(counts[colour], end - first), ns = min(counts[8 + colour], end - first);
+  if (blockIdx.x * kPervoxelWarps >= max(ni, ns)) return;
   if (threadIdx.x == 0) s_args = a;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  WarpShared &sh = s_warp[warp];
-  const WarpLane wl = warp_lane(a, lane);
+  const unsigned warps = gridDim.x * kPervoxelWarps, w0 = blockIdx.x * kPervoxelWarps + warp;
   // the same on every lane but where noted
   float maxd = 0.f;
   double energy = 0.0;  // lane 0: float64 from the per-voxel terms up
   unsigned capped = 0, most = 0;
   bool diverged = false;
-  for (unsigned k = blockIdx.x * kPervoxelWarps + warp; k < nq; k += gridDim.x * kPervoxelWarps) {
-    const int i = list[first + k];
+  for (unsigned k = w0; k < ns; k += warps) {
+    const int i = list[end - 1u - k];
     if (!KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST)) continue;
     int x, y, z, iter = 0;
     unsigned steps = 0;
     float dn = 0.f, en = 0.f;
     voxel_xyz(dp, i, x, y, z);
-    if (interior_voxel(dp, x, y, z)) {
+    while (true) {
+      float d[3], s, c0[3];
+      shell_gradient<kPsiL2>(s_args, false, x, y, z, s_shell[warp], d, &s, &en, c0);
+      const float n[3] = {c0[0] + d[0], c0[1] + d[1], c0[2] + d[2]};
+      __syncwarp();  // every lane has read psi
+      if (lane == 0) {
+        a.ox[i] = n[0];
+        a.oy[i] = n[1];
+        a.oz[i] = n[2];
+      }
+      __syncwarp();
+      ++steps;
+      dn = sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0]))));
+      if (pervoxel_done(a, dn, n, max_iters, iter, diverged)) break;
+    }
+    if (lane == 0) energy += en;
+    maxd = fmaxf(maxd, dn);
+    capped += iter >= max_iters;
+    most = max(most, steps);
+  }
+  __syncwarp();
+  if (ni <= (max_iters > kPervoxelFewSteps ? warps + warps / 8 : warps / 2)) {
+    WarpShared &sh = s_warp[warp];
+    const WarpLane wl = warp_lane(a, lane);
+    for (unsigned k = w0; k < ni; k += warps) {
+      const int i = list[first + k];
+      if (!KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST)) continue;
+      int x, y, z, iter = 0;
+      unsigned steps = 0;
+      float dn = 0.f;
+      voxel_xyz(dp, i, x, y, z);
+      if (!interior_voxel(dp, x, y, z)) continue;  // (the bounds-check build's unwritten entries)
       const float can = __ldg(a.can + i);
       __syncwarp();
       warp_neighbours<kPsiL2>(a, i, lane, wl, sh);
@@ -968,27 +1026,47 @@ __global__ void __launch_bounds__(32 * kPervoxelWarps, kPervoxelBlocksPerSM)
         group_statistics(a, t, m, e, one);
         energy += e;
       }
-    } else {
+      maxd = fmaxf(maxd, dn);
+      capped += iter >= max_iters;
+      most = max(most, steps);
+    }
+  } else {
+    float lane_maxd = 0.f;
+    double lane_energy = 0.0;
+    unsigned lane_capped = 0, lane_most = 0;
+    bool lane_diverged = false;
+    for (unsigned k = 32 * w0 + lane; k < ni; k += 32 * warps) {
+      const int i = list[first + k];
+      if (!KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST)) continue;
+      int x, y, z, iter = 0;
+      unsigned steps = 0;
+      float dn, en;
+      voxel_xyz(dp, i, x, y, z);
+      if (!interior_voxel(dp, x, y, z)) continue;
       while (true) {
         float d[3], s, c0[3];
-        shell_gradient<kPsiL2>(s_args, false, x, y, z, s_shell[warp], d, &s, &en, c0);
+        gradient_lane<kPsiL2>(a, x, y, z, i, d, s, en, c0);
         const float n[3] = {c0[0] + d[0], c0[1] + d[1], c0[2] + d[2]};
-        __syncwarp();  // every lane has read psi
-        if (lane == 0) {
-          a.ox[i] = n[0];
-          a.oy[i] = n[1];
-          a.oz[i] = n[2];
-        }
-        __syncwarp();
+        a.ox[i] = n[0];
+        a.oy[i] = n[1];
+        a.oz[i] = n[2];
         ++steps;
         dn = sqrtf(ff(d[2], d[2], ff(d[1], d[1], fm(d[0], d[0]))));
-        if (pervoxel_done(a, dn, n, max_iters, iter, diverged)) break;
+        if (pervoxel_done(a, dn, n, max_iters, iter, lane_diverged)) break;
       }
-      if (lane == 0) energy += en;
+      lane_energy += en;
+      lane_maxd = fmaxf(lane_maxd, dn);
+      lane_capped += iter >= max_iters;
+      lane_most = max(lane_most, steps);
     }
-    maxd = fmaxf(maxd, dn);
-    capped += iter >= max_iters;
-    most = max(most, steps);
+    __syncwarp();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) lane_energy += __shfl_xor_sync(0xffffffffu, lane_energy, o);
+    energy += lane_energy;
+    maxd = fmaxf(maxd, __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(lane_maxd))));
+    capped += __reduce_add_sync(0xffffffffu, lane_capped);
+    most = max(most, __reduce_max_sync(0xffffffffu, lane_most));
+    diverged = __any_sync(0xffffffffu, lane_diverged) || diverged;
   }
   if (lane == 0) {
     commit_iter_stats(a.st, BlockStats{energy, 0u, maxd, diverged});
@@ -1345,19 +1423,19 @@ int kf_solve_pervoxel(kf_grid live, kf_grid can, kf_field psi, const DevParams &
   const unsigned grid = (unsigned)std::max<int64_t>((dp.count / 4 + kThreads * kFlatGroups - 1) /
                                                         (kThreads * kFlatGroups), 1);
   k_fused_stream<false><<<grid, kThreads, 0, s>>>(a, psi->band, nullptr, nullptr, nullptr);
-  // the colours' counts and cursors, and their lists in the second band list
+  // the colours' counts, and their lists in the second band list
   void *sync = nullptr;
   rc = kf_field_sync(psi, &sync);
   if (rc) return rc;
-  unsigned *counts = static_cast<unsigned *>(sync), *cursors = counts + 8;
-  KF_CHECK_CUDA(cudaMemsetAsync(counts, 0, 16 * sizeof(unsigned), s));
+  unsigned *counts = static_cast<unsigned *>(sync);
+  KF_CHECK_CUDA(cudaMemsetAsync(counts, 0, kColourCounts * sizeof(unsigned), s));
   int *lists = psi->band + dp.count;
   const unsigned spread = (unsigned)kf_num_sms() * 4;
-  k_colour_lists<false><<<spread, kThreads, 0, s>>>(a, psi->band, counts, cursors, lists);
-  k_colour_lists<true><<<spread, kThreads, 0, s>>>(a, psi->band, counts, cursors, lists);
+  const ColourParts parts = colour_parts(dp);
+  k_colour_lists<<<spread, kThreads, 0, s>>>(a, psi->band, counts, parts, lists);
   for (int colour = 0; colour < 8; ++colour)
-    k_pervoxel<<<(unsigned)kf_num_sms() * kPervoxelBlocksPerSM, 32 * kPervoxelWarps, 0, s>>>(a, lists, counts,
-                                                                                          max_iters, colour);
+    k_pervoxel<<<(unsigned)kf_num_sms() * kPervoxelBlocksPerSM, 32 * kPervoxelWarps, 0, s>>>(
+        a, lists, counts, parts.start[colour], parts.start[colour + 1], max_iters, colour);
   KF_CHECK_LAUNCH("per-voxel solve");
   return KF_OK;
 }
