@@ -1102,6 +1102,13 @@ __global__ void __launch_bounds__(kBlock) k_exact_first(PhiView<double> live, Ps
 // took 410 us an iteration at 64^3.
 constexpr int kExactVoxels = 16;
 constexpr int kExactSamples = 44;
+// From this many voxels an SM on a thread takes a whole voxel (exact_voxel): the
+// warps are full then, where the parts between two barriers leave the float64 unit
+// idle.  An iteration with 10.3 k, 17.3 k, 38 k band voxels (68, 114, 254 an SM) and
+// all 33 k, 111 k, 262 k, 885 k voxels of a grid in the band: in parts 165, 264, 528, 454,
+// 1489, 3487 and 11796 us, a thread each 234, 223, 411, 353, 1137, 2666 and 9024 us.
+// (A thread per voxel of the dense grid: 408, 712, 1205, 396, 1180, 2746 and 9019 us.)
+constexpr unsigned kExactLaneShare = 112;
 constexpr int kExactThreads = kExactVoxels * kExactSamples;  // 22 warps
 
 // The cell-centre offsets (units of h): the gradient's +-e_k, then the 19 of
@@ -1143,6 +1150,64 @@ __device__ __forceinline__ void killing_sample(const PsiView<double, double> &f,
   for (int k = 0; k < 3; ++k) out[k] = lerp1(lerp1(v[0][k], v[1][k], t0), lerp1(v[2][k], v[3][k], t0), t1);
 }
 
+// A warp's voxels i with the steps md: those in the band are counted and listed for
+// the next iteration.
+__device__ __forceinline__ void exact_count(IterStats *st, int iter, bool active, float md, int i, const DevParams &dp,
+                                            int *__restrict__ list_out) {
+  const int lane = threadIdx.x & 31;
+  const unsigned ball = __ballot_sync(0xffffffffu, active);
+  md = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(md)));
+  unsigned base = 0;
+  if (lane == 0 && ball) {
+    atomicAdd(&st[iter].active, (unsigned)__popc(ball));
+    atomicMax(&st[iter].max_delta, __float_as_uint(md));
+    base = atomicAdd(&st[iter + 1].list, (unsigned)__popc(ball));
+  }
+  base = __shfl_sync(0xffffffffu, base, 0) + (unsigned)__popc(ball & ((1u << lane) - 1u));
+  if (active && KF_IN_BOUNDS(base, dp.count, KF_SITE_BAND_APPEND)) list_out[base] = i;
+}
+
+// An iteration of band voxel i by one thread (a: in shared memory): its step's
+// length, -1 where it has left the band.
+struct ExactArgs {
+  PhiView<double> live, can;
+  PsiView<double, double> fin;
+  double *ox, *oy, *oz;
+  DevParams dp;
+  int *diverged, *rows;
+};
+
+__device__ __noinline__ float exact_voxel(const ExactArgs *a, int i) {
+  const PhiView<double> &live = a->live, &can = a->can;
+  const PsiView<double, double> &fin = a->fin;
+  const DevParams &dp = a->dp;
+  int x, y, z;
+  voxel_xyz(i, dp.nx, dp.ny, x, y, z);
+  const double c[3] = {fin.px[i], fin.py[i], fin.pz[i]}, s = warped_distance(live, fin, x, y, z);
+  double d[3] = {0.0, 0.0, 0.0};
+  float step = -1.f;
+  if (in_band(s, dp.band_hi, -dp.unknown_clip)) {
+    const TParams<double> tp(dp);
+    double g[3], u[3];
+    energy_gradient(live, can, fin, tp, x, y, z, g);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) u[q] = -tp.alpha * g[q];
+    if (dp.trust && !trust_step(live, can.at(x, y, z), s, x, y, z, c, g, tp.alpha, u)) {
+      atomicMin(a->rows + ((int64_t)z * dp.ny + y), x);
+    } else {
+      // the update field starts at zero (KillingFusion.cpp:256, 316)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) d[q] = d[q] + u[q];
+    }
+    if (!isfinite(c[0]) || !isfinite(c[1]) || !isfinite(c[2])) *a->diverged = 1;
+    step = (float)sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+  }
+  a->ox[i] = c[0] + d[0];
+  a->oy[i] = c[1] + d[1];
+  a->oz[i] = c[2] + d[2];
+  return step;
+}
+
 __global__ void __launch_bounds__(kExactThreads, 1) k_exact_band(PhiView<double> live, PhiView<double> can,
                                                                  PsiView<double, double> fin,
                                                                  double *__restrict__ ox, double *__restrict__ oy,
@@ -1166,6 +1231,25 @@ __global__ void __launch_bounds__(kExactThreads, 1) k_exact_band(PhiView<double>
   const unsigned n = st[iter].list;
   const unsigned per = min(max((n + gridDim.x - 1) / gridDim.x, 1u), (unsigned)kExactVoxels);
   const int tid = threadIdx.x;
+  const unsigned share = (n + gridDim.x - 1) / gridDim.x;
+  if (share >= kExactLaneShare) {
+    __shared__ ExactArgs s_args;
+    if (tid == 0) s_args = ExactArgs{live, can, fin, ox, oy, oz, dp, &st[iter].diverged, rows};
+    __syncthreads();
+    // its share in rounds of equally many warps
+    const unsigned end = min((blockIdx.x + 1) * share, n), warps = (share + 31) / 32;
+    const unsigned rounds = (warps + kExactThreads / 32 - 1) / (kExactThreads / 32);
+    const unsigned stride = 32 * ((warps + rounds - 1) / rounds);
+    if ((unsigned)tid >= stride) return;
+    for (unsigned k0 = blockIdx.x * share + (tid & ~31); k0 < end; k0 += stride) {
+      const unsigned k = k0 + (tid & 31);
+      const int i = k < end ? list[k] : -1;
+      const float md = k < end && KF_IN_BOUNDS(i, dp.count, KF_SITE_BAND_LIST) ? exact_voxel(&s_args, i) : -1.f;
+      __syncwarp();
+      exact_count(st, iter, !(md < 0.f), md < 0.f ? 0.f : md, i, dp, list_out);  // (a NaN step is in the band)
+    }
+    return;
+  }
   for (unsigned k0 = blockIdx.x * per; k0 < n; k0 += gridDim.x * per) {
     const int m = (int)min(n - k0, per);
     if (tid < m) {
@@ -1307,16 +1391,7 @@ __global__ void __launch_bounds__(kExactThreads, 1) k_exact_band(PhiView<double>
         oy[i] = c[1] + d[1];
         oz[i] = c[2] + d[2];
       }
-      const unsigned ball = __ballot_sync(0xffffffffu, active);
-      md = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(md)));
-      unsigned base = 0;
-      if (tid == 0 && ball) {
-        atomicAdd(&st[iter].active, (unsigned)__popc(ball));
-        atomicMax(&st[iter].max_delta, __float_as_uint(md));
-        base = atomicAdd(&st[iter + 1].list, (unsigned)__popc(ball));
-      }
-      base = __shfl_sync(0xffffffffu, base, 0) + (unsigned)__popc(ball & ((1u << tid) - 1u));
-      if (active && KF_IN_BOUNDS(base, dp.count, KF_SITE_BAND_APPEND)) list_out[base] = i;
+      exact_count(st, iter, active, md, i, dp, list_out);
     }
     __syncthreads();  // this chunk's values are read before the next one's
   }
