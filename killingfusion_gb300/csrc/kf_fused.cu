@@ -165,6 +165,37 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_runs(const int2 *__rest
   }
 }
 
+// The band test of kColdRuns cold runs (entries ~run) whose psi is zero, all their
+// loads in flight together.
+__device__ __forceinline__ void test_zero_runs(const FusedArgs &a, const int entry[kColdRuns], int runs_in_grid) {
+  const DevParams &dp = a.dp;
+  const int n4 = (int)(dp.count >> 2), tid = threadIdx.x;
+  const float4 *lv = reinterpret_cast<const float4 *>(a.live);
+  float4 ph[kColdRuns][kFlatGroups];
+#pragma unroll
+  for (int j = 0; j < kColdRuns; ++j) {
+    const bool known = KF_IN_BOUNDS(~entry[j], runs_in_grid, KF_SITE_RUNS);
+#pragma unroll
+    for (int g = 0; g < kFlatGroups; ++g) {
+      const int q = ~entry[j] * (kThreads * kFlatGroups) + g * kThreads + tid;
+      // (one past the grid's end: outside any band)
+      const float far = __int_as_float(0x7f800000);
+      ph[j][g] = known && q < n4 ? __ldg(lv + q) : make_float4(far, far, far, far);
+    }
+  }
+  unsigned hits = 0;
+#pragma unroll
+  for (int j = 0; j < kColdRuns; ++j) {
+#pragma unroll
+    for (int g = 0; g < kFlatGroups; ++g)
+      hits += in_band(ph[j][g].x, a.band_hi, a.band_lo) + in_band(ph[j][g].y, a.band_hi, a.band_lo) +
+              in_band(ph[j][g].z, a.band_hi, a.band_lo) + in_band(ph[j][g].w, a.band_hi, a.band_lo);
+    // the ragged end, run 0's
+    if (entry[j] == ~0 && tid < (int)(dp.count & 3)) hits += in_band(__ldg(a.live + 4 * n4 + tid), a.band_hi, a.band_lo);
+  }
+  if (hits) atomicAdd(&a.st[a.iter].cold, hits);
+}
+
 // Dense pass of iteration a.iter >= 1 over the listed runs (counts[0] hot
 // runs, counts[1] cold runs), a run per loop step.  Hot: each run writes
 // back its band voxels' new psi from the iteration before (as
@@ -173,11 +204,14 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_runs(const int2 *__rest
 // st[iter].cold.  A cold pass stops once the iteration before it was
 // skipped (the statistics of that iteration's band pass may still be in
 // flight when it runs, so it may run once after convergence, to no effect).
-// Eight CTAs per SM of the cold pass (32 registers), for the loads in flight:
-// the dense 256^3 iteration takes 41.5 us, with six CTAs 41.6 us, with five
-// (44 registers) 42.9 us.
+// A block whose kColdRuns runs all have zero psi loads them at once
+// (test_zero_runs), the others take one run after the other, whose moved voxels'
+// gathers want the registers (five CTAs per SM): 512^3 frames from zero 66.5 ms
+// against 68.9 ms with eight CTAs of 32 registers and a run at a time (80.5 and 85.7
+// ms with six and five of those); 128^3 from random psi, 60 iterations, 2.85 ms
+// against 3.00 ms, from a smooth one 2.32 against 2.55 ms, 256^3 11.0 against 10.7.
 template <bool kCold>
-__global__ void __launch_bounds__(kThreads, kCold ? 8 : 5) k_fused_stream_runs(FusedArgs a, const int *__restrict__ run_list,
+__global__ void __launch_bounds__(kThreads, 5) k_fused_stream_runs(FusedArgs a, const int *__restrict__ run_list,
                                                                const unsigned *__restrict__ counts,
                                                                int *__restrict__ list,
                                                                const int *__restrict__ prev_list,
@@ -185,15 +219,28 @@ __global__ void __launch_bounds__(kThreads, kCold ? 8 : 5) k_fused_stream_runs(F
   const unsigned n = counts[kCold ? 1 : 0];
   if (kCold) {
     if (a.st[a.iter - 1].skipped) return;
-    for (unsigned idx = blockIdx.x; idx < n; idx += gridDim.x) {
-      const int entry = run_list[idx], r = entry < 0 ? ~entry : entry;
-      if (!KF_IN_BOUNDS(r, max((a.dp.count / 4 + kThreads * kFlatGroups - 1) / (kThreads * kFlatGroups), (int64_t)1),
-                        KF_SITE_RUNS))
+    const int runs_in_grid = (int)max((a.dp.count / 4 + kFlatVoxels / 4 - 1) / (kFlatVoxels / 4), (int64_t)1);
+    for (unsigned k0 = blockIdx.x; k0 < n; k0 += gridDim.x * kColdRuns) {
+      int entry[kColdRuns];
+      bool all_zero = k0 + (kColdRuns - 1) * gridDim.x < n;
+#pragma unroll
+      for (int j = 0; j < kColdRuns; ++j) {
+        entry[j] = k0 + j * gridDim.x < n ? run_list[k0 + j * gridDim.x] : 0;
+        all_zero = all_zero && entry[j] < 0;
+      }
+      if (all_zero) {
+        test_zero_runs(a, entry, runs_in_grid);
         continue;
-      if (entry < 0)
-        stream_flat<false, true, true>(a, r, nullptr, &a.st[a.iter].cold);
-      else
-        stream_flat<false, true>(a, r, nullptr, &a.st[a.iter].cold);
+      }
+#pragma unroll 1
+      for (unsigned k = k0; k < n && k < k0 + kColdRuns * gridDim.x; k += gridDim.x) {
+        const int e = run_list[k], r = e < 0 ? ~e : e;
+        if (!KF_IN_BOUNDS(r, runs_in_grid, KF_SITE_RUNS)) continue;
+        if (e < 0)
+          stream_flat<false, true, true>(a, r, nullptr, &a.st[a.iter].cold);
+        else
+          stream_flat<false, true>(a, r, nullptr, &a.st[a.iter].cold);
+      }
     }
     return;
   }
