@@ -970,6 +970,15 @@ __device__ __forceinline__ void fuse_kept(float *__restrict__ phi1, int32_t *__r
   }
 }
 
+// `loaders` threads of a CTA load four voxels each; a CTA with fewer of them leaves
+// its moved voxels, which a whole CTA resamples, more threads.  Where the grid does not
+// fill the SMs that counts.  All of psi non-zero, 32^3, 64^3, 80^3, 104^3: 48.0, 75.6,
+// 136 and 254 us with 256, 29.9, 74.9, 118 and 237 us with 128, 23.6, 66.9, 119 and
+// 230 us with 64 (22.5, 68.5, 123 and 240 us with a voxel a thread throughout); 3 % of it:
+// 23.7, 25.0, 28.0 and 36.0 us, 21.7, 23.2, 30.1 and 41.6 us, 22.2, 29.9, 37.0 and 60.3
+// us (22.8, 60.2, 95.0 and 182 us).  In voxels per SM:
+constexpr int kFuseSmall = 2048, kFuseMiddle = 8192;
+
 template <typename P>
 __device__ __forceinline__ unsigned moved_of_four(PsiPlanes<P> f, int64_t q) {
   unsigned moved = 0;
@@ -996,19 +1005,19 @@ template <typename P>
 __global__ void __launch_bounds__(kBlock) k_fuse_warped(float *__restrict__ phi1, int32_t *__restrict__ w1,
                                                         const float *__restrict__ phi2,
                                                         const int32_t *__restrict__ w2, PsiPlanes<P> f, int nx, int ny,
-                                                        int nz, double oob) {
+                                                        int nz, double oob, int loaders) {
   __shared__ int s_list[4 * kBlock];
   __shared__ int s_n;
   const int64_t N = (int64_t)nx * ny * nz;
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i0 = 4 * q;
+  const int64_t q = (int64_t)blockIdx.x * loaders + threadIdx.x, i0 = 4 * q;
   int32_t b[4] = {0, 0, 0, 0};
   unsigned moved = 0;
-  const bool whole = i0 + 3 < N;
+  const bool loads = (int)threadIdx.x < loaders, whole = loads && i0 + 3 < N;
   if (whole) {
     moved = moved_of_four(f, q);
     const int4 v = __ldcs(reinterpret_cast<const int4 *>(w2) + q);
     b[0] = v.x, b[1] = v.y, b[2] = v.z, b[3] = v.w;
-  } else {
+  } else if (loads) {
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
       if (i0 + e >= N) break;
@@ -1039,7 +1048,7 @@ __global__ void __launch_bounds__(kBlock) k_fuse_warped(float *__restrict__ phi1
   }
   __syncthreads();
   for (int k = threadIdx.x; k < s_n; k += kBlock) {
-    const int64_t i = 4 * (int64_t)blockIdx.x * kBlock + s_list[k];
+    const int64_t i = 4 * (int64_t)blockIdx.x * loaders + s_list[k];
     int x, y, z;
     voxel_xyz(i, nx, ny, x, y, z);
     double d2, b;
@@ -1536,13 +1545,15 @@ int kf_launch_fuse(kf_grid can, kf_grid other, cudaStream_t s) {
 
 int kf_launch_fuse_warped(kf_grid dst, kf_grid other, kf_field psi, const DevParams &dp,
                           cudaStream_t s) {
-  const unsigned blocks = blocks_for((dst->count + 3) / 4);
+  const int64_t per_sm = dst->count / kf_num_sms();
+  const int loaders = per_sm < kFuseSmall ? kBlock / 4 : (per_sm < kFuseMiddle ? kBlock / 2 : kBlock);
+  const unsigned blocks = blocks_for((dst->count + 3) / 4, loaders);
   if (psi->prec == KF_F32)
     k_fuse_warped<float><<<blocks, kBlock, 0, s>>>(dst->phi, dst->w, other->phi, other->w, planes<float>(psi),
-                                                   dst->n[0], dst->n[1], dst->n[2], dp.oob_phi);
+                                                   dst->n[0], dst->n[1], dst->n[2], dp.oob_phi, loaders);
   else
     k_fuse_warped<double><<<blocks, kBlock, 0, s>>>(dst->phi, dst->w, other->phi, other->w, planes<double>(psi),
-                                                    dst->n[0], dst->n[1], dst->n[2], dp.oob_phi);
+                                                    dst->n[0], dst->n[1], dst->n[2], dp.oob_phi, loaders);
   KF_CHECK_LAUNCH("k_fuse_warped");
   return KF_OK;
 }
