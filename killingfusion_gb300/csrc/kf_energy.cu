@@ -264,17 +264,18 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_partials(const double *part
 // of the grid that samples phi_w seven times and takes whole Jacobians.
 constexpr int kRun = 256, kRunThreads = 128;
 
-// The entries u < kRun of the run from voxel v0 on for which pred(voxel) holds,
-// in order, into list; their number.  Every thread of the block calls it.
+// The entries u < kRun of the run from voxel v0 on (v1: where the pass ends) for
+// which pred(voxel) holds, in order, into list; their number.  Every thread of the
+// block calls it.
 template <typename Pred>
-__device__ __forceinline__ int gather_run(int64_t v0, int64_t N, int16_t *list, Pred pred) {
+__device__ __forceinline__ int gather_run(int64_t v0, int64_t v1, int16_t *list, Pred pred) {
   __shared__ int s_cnt[kRun / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned ball[kRun / kRunThreads];
 #pragma unroll
   for (int r = 0; r < kRun / kRunThreads; ++r) {
     const int u = r * kRunThreads + (int)threadIdx.x;
-    ball[r] = __ballot_sync(0xffffffffu, v0 + u < N && pred(v0 + u));
+    ball[r] = __ballot_sync(0xffffffffu, v0 + u < v1 && pred(v0 + u));
     if (lane == 0) s_cnt[r * (kRunThreads / 32) + warp] = __popc(ball[r]);
   }
   __syncthreads();
@@ -316,31 +317,45 @@ __device__ __forceinline__ bool is_needed(const EArgs<T, P> &a, int64_t i) {
          (z + 1 < a.nz && is_active(a, i + plane));
 }
 
-// phi_w at the needed voxels, and with kGrad its derivative (dv: three planes
-// of N).  odd (kGrad): set when live holds a value that is not finite.
+// The passes take the voxels [v0, v1); their buffers are indexed by the voxel
+// itself (part_buffer).
+
+// phi_w at the needed voxels, and with kGrad its derivative (dv: three planes, `step`
+// apart) at those in [d0, d1).  odd (or NULL): set when live holds a value that is not
+// finite.
 template <typename T, typename P, bool kGrad>
-__global__ void __launch_bounds__(kRunThreads) k_warped(EArgs<T, P> a, int64_t N, T *__restrict__ w,
-                                                        T *__restrict__ dv, int *__restrict__ odd) {
+__global__ void __launch_bounds__(kRunThreads) k_warped(EArgs<T, P> a, int64_t v0, int64_t v1, T *__restrict__ w,
+                                                        T *__restrict__ dv, int64_t step, int64_t d0, int64_t d1,
+                                                        int *__restrict__ odd) {
   __shared__ int16_t s_list[kRun];
-  const int64_t v0 = (int64_t)blockIdx.x * kRun;
-  if (kGrad) {
+  v0 += (int64_t)blockIdx.x * kRun;
+  if (kGrad && odd) {
     bool bad = false;
-    for (int u = threadIdx.x; u < kRun; u += kRunThreads) bad = bad || (v0 + u < N && !isfinite(__ldg(a.live + v0 + u)));
+    for (int u = threadIdx.x; u < kRun; u += kRunThreads) bad = bad || (v0 + u < v1 && !isfinite(__ldg(a.live + v0 + u)));
     if (bad) *odd = 1;
   }
-  const int n = gather_run(v0, N, s_list, [&](int64_t i) { return is_needed(a, i); });
+  const int n = gather_run(v0, v1, s_list, [&](int64_t i) { return is_needed(a, i); });
   for (int k = threadIdx.x; k < n; k += kRunThreads) {
     const int64_t i = v0 + s_list[k];
     int x, y, z;
     coords(a, i, x, y, z);
     T d[3];
     w[i] = warped(a, x, y, z, d);
-    if (kGrad) {
+    if (kGrad && i >= d0 && i < d1) {
       dv[i] = d[0];
-      dv[N + i] = d[1];
-      dv[2 * N + i] = d[2];
+      dv[step + i] = d[1];
+      dv[2 * step + i] = d[2];
     }
   }
+}
+
+// *odd = 1 where live holds a value that is not finite.
+__global__ void __launch_bounds__(kThreads) k_not_finite(const float *__restrict__ live, int64_t N,
+                                                         int *__restrict__ odd) {
+  bool bad = false;
+  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < N; i += (int64_t)gridDim.x * kThreads)
+    bad = bad || !isfinite(__ldg(live + i));
+  if (bad) *odd = 1;
 }
 
 // ls_gradient from phi_w.
@@ -356,11 +371,11 @@ __device__ __forceinline__ void ls_gradient_w(const EArgs<T, P> &a, const T *__r
 
 // The energy of a run's active voxels (voxel_energy's terms).
 template <typename T, typename P>
-__global__ void __launch_bounds__(kRunThreads) k_energy_runs(EArgs<T, P> a, int64_t N, const T *__restrict__ w,
-                                                             double *__restrict__ partial) {
+__global__ void __launch_bounds__(kRunThreads) k_energy_runs(EArgs<T, P> a, int64_t v0, int64_t v1,
+                                                             const T *__restrict__ w, double *__restrict__ partial) {
   __shared__ int16_t s_list[kRun];
-  const int64_t v0 = (int64_t)blockIdx.x * kRun;
-  const int n = gather_run(v0, N, s_list, [&](int64_t i) { return is_active(a, i); });
+  v0 += (int64_t)blockIdx.x * kRun;
+  const int n = gather_run(v0, v1, s_list, [&](int64_t i) { return is_active(a, i); });
   double acc[3] = {0.0, 0.0, 0.0};
   if (n == 0) {  // (the sums of nothing would cost the float64 unit as much as others)
     if (threadIdx.x < 3) partial[3 * (int64_t)blockIdx.x + threadIdx.x] = 0.0;
@@ -384,11 +399,12 @@ __global__ void __launch_bounds__(kRunThreads) k_energy_runs(EArgs<T, P> a, int6
 // Level-set coefficient of active voxel i: d E_ls(i) / d g_k(i) / 2, i.e. the
 // weight of d phi_w(p_k(i)) (+) and d phi_w(m_k(i)) (-).
 template <typename P>
-__global__ void __launch_bounds__(kRunThreads) k_ls_coef(EArgs<double, P> a, int64_t N, const double *__restrict__ w,
-                                                         double *__restrict__ S) {
+__global__ void __launch_bounds__(kRunThreads) k_ls_coef(EArgs<double, P> a, int64_t v0, int64_t v1,
+                                                         const double *__restrict__ w, double *__restrict__ S,
+                                                         int64_t step) {
   __shared__ int16_t s_list[kRun];
-  const int64_t v0 = (int64_t)blockIdx.x * kRun;
-  const int n = gather_run(v0, N, s_list, [&](int64_t i) { return is_active(a, i); });
+  v0 += (int64_t)blockIdx.x * kRun;
+  const int n = gather_run(v0, v1, s_list, [&](int64_t i) { return is_active(a, i); });
   for (int k = threadIdx.x; k < n; k += kRunThreads) {
     const int64_t i = v0 + s_list[k];
     int x, y, z;
@@ -398,7 +414,7 @@ __global__ void __launch_bounds__(kRunThreads) k_ls_coef(EArgs<double, P> a, int
     const double nr = sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2] + a.ve * a.ve);
     const double coef = a.omega_s * (nr / a.v - 1.0) / (a.v * nr);
 #pragma unroll
-    for (int q = 0; q < 3; ++q) S[q * N + i] = coef * g[q] * 0.5;
+    for (int q = 0; q < 3; ++q) S[q * step + i] = coef * g[q] * 0.5;
   }
 }
 
@@ -406,14 +422,14 @@ __global__ void __launch_bounds__(kRunThreads) k_ls_coef(EArgs<double, P> a, int
 // voxels that no active one reads have a zero gradient (as the sum of nothing;
 // where phi_w there is not finite, 0 times its derivative is kept).
 template <typename P>
-__global__ void __launch_bounds__(kRunThreads) k_adjoint(EArgs<double, P> a, int64_t N, const double *__restrict__ w,
-                                                         const double *__restrict__ dvs,
-                                                         const double *__restrict__ S, const int *__restrict__ odd,
-                                                         double *__restrict__ grad) {
+__global__ void __launch_bounds__(kRunThreads) k_adjoint(EArgs<double, P> a, int64_t v0, int64_t v1,
+                                                         const double *__restrict__ w, const double *__restrict__ dvs,
+                                                         int64_t dv_step, const double *__restrict__ S, int64_t s_step,
+                                                         const int *__restrict__ odd, double *__restrict__ grad) {
   __shared__ int16_t s_list[kRun];
-  const int64_t v0 = (int64_t)blockIdx.x * kRun;
+  v0 += (int64_t)blockIdx.x * kRun;
   const bool all = *odd != 0;
-  const int n = gather_run(v0, N, s_list, [&](int64_t i) {
+  const int n = gather_run(v0, v1, s_list, [&](int64_t i) {
     if (is_needed(a, i)) return true;
     if (a.use_ls && (all || !isfinite(a.px[i]) || !isfinite(a.py[i]) || !isfinite(a.pz[i]))) return true;
     grad[3 * i] = grad[3 * i + 1] = grad[3 * i + 2] = 0.0;
@@ -430,7 +446,7 @@ __global__ void __launch_bounds__(kRunThreads) k_adjoint(EArgs<double, P> a, int
     if (is_needed(a, j)) {
       wj = w[j];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) dv[q] = dvs[q * N + j];
+      for (int q = 0; q < 3; ++q) dv[q] = dvs[q * dv_step + j];
     } else {
       wj = warped(a, c[0], c[1], c[2], dv);
     }
@@ -451,7 +467,7 @@ __global__ void __launch_bounds__(kRunThreads) k_adjoint(EArgs<double, P> a, int
         const int64_t i = u == 0 ? j - step[k] : (u == 1 ? j + step[k] : j);
         const int sg = u == 0 ? 1 : (u == 1 ? -1 : self);
         if (!is_active(a, i)) continue;
-        if (a.use_ls) ls += sg * S[(int64_t)k * N + i];
+        if (a.use_ls) ls += sg * S[(int64_t)k * s_step + i];
         if (a.use_k) {
           // column k and row k of the Jacobian at i
           double col[3], row[3];
@@ -569,8 +585,8 @@ int run_energy(kf_grid live, kf_grid can, kf_field psi, const DevParams &dp, con
   return KF_OK;
 }
 
-// `doubles` float64 values of workspace: the field's, kept with it (an
-// allocation from the stream's pool is mapped anew after each
+// `doubles` float64 values of workspace (bounded, kEnergyBytes): the field's, kept with
+// it (an allocation from the stream's pool is mapped anew after each
 // synchronisation), or, where the stream is being captured, the graph's own
 // (*own: the caller frees it on the stream).
 int energy_scratch(kf_field psi, size_t doubles, cudaStream_t s, double **out, bool *own) {
@@ -597,21 +613,46 @@ int energy_scratch(kf_field psi, size_t doubles, cudaStream_t s, double **out, b
   return KF_OK;
 }
 
+// Above this the passes over the whole grid take it in parts (ranges of voxels, runs
+// kept whole, so that the sums are the same), and that is the most a field keeps: 56 B
+// a voxel for the gradient and 8 B for the energy would be 7.5 and 1 GB at 512^3.
+constexpr size_t kEnergyBytes = (size_t)512 << 20;
+
+// The voxels of a part, of `total` with `each` bytes for a voxel and `halo` bytes
+// beside them.
+int64_t part_voxels(int64_t total, int64_t each, int64_t halo) {
+  if (total * each <= (int64_t)kEnergyBytes) return total;
+  const int64_t fit = ((int64_t)kEnergyBytes - halo) / each;
+  return std::max<int64_t>(fit, (int64_t)1 << 20) / kRun * kRun;
+}
+
+// A buffer of the voxels from lo on, indexed by the voxel itself.
+template <typename T>
+T *part_buffer(T *buf, int64_t lo) {
+  return reinterpret_cast<T *>(reinterpret_cast<uintptr_t>(buf) - (uintptr_t)(lo * (int64_t)sizeof(T)));
+}
+
+unsigned run_blocks(int64_t v0, int64_t v1) { return (unsigned)((v1 - v0 + kRun - 1) / kRun); }
+
 // run_energy over the whole grid.
 template <typename T, typename P>
 int run_energy_runs(kf_grid live, kf_grid can, kf_field psi, const DevParams &dp, const uint8_t *active,
                     double terms[3], cudaStream_t s) {
-  const int64_t N = live->count;
-  const int blocks = (int)((N + kRun - 1) / kRun);
+  const int64_t N = live->count, plane = (int64_t)live->n[0] * live->n[1];
+  const int64_t part = part_voxels(N, sizeof(double), 2 * plane * (int64_t)sizeof(double));
+  const unsigned blocks = run_blocks(0, N);
   double *buf = nullptr;
   bool own = false;
-  int rc = energy_scratch(psi, 3 + 3 * (size_t)blocks + (size_t)N, s, &buf, &own);
+  int rc = energy_scratch(psi, 3 + 3 * (size_t)blocks + (size_t)std::min(part + 2 * plane, N), s, &buf, &own);
   if (rc) return rc;
-  T *w = reinterpret_cast<T *>(buf + 3 + 3 * (size_t)blocks);
   EArgs<T, P> a = make_args<T, P>(live, can, psi, dp, active);
-  k_warped<T, P, false><<<blocks, kRunThreads, 0, s>>>(a, N, w, (T *)nullptr, nullptr);
-  k_energy_runs<T, P><<<blocks, kRunThreads, 0, s>>>(a, N, w, buf + 3);
-  k_sum_partials<<<1, kSumThreads, 0, s>>>(buf + 3, blocks, buf);
+  for (int64_t v0 = 0; v0 < N; v0 += part) {
+    const int64_t v1 = std::min(v0 + part, N), lo = std::max<int64_t>(v0 - plane, 0), hi = std::min(v1 + plane, N);
+    T *w = part_buffer(reinterpret_cast<T *>(buf + 3 + 3 * (size_t)blocks), lo);
+    k_warped<T, P, false><<<run_blocks(lo, hi), kRunThreads, 0, s>>>(a, lo, hi, w, (T *)nullptr, 0, 0, 0, nullptr);
+    k_energy_runs<T, P><<<run_blocks(v0, v1), kRunThreads, 0, s>>>(a, v0, v1, w, buf + 3 + 3 * (v0 / kRun));
+  }
+  k_sum_partials<<<1, kSumThreads, 0, s>>>(buf + 3, (int)blocks, buf);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(terms, buf, 3 * sizeof(double), cudaMemcpyDeviceToHost, s);
   if (own) cudaFreeAsync(buf, s);
@@ -623,20 +664,30 @@ int run_energy_runs(kf_grid live, kf_grid can, kf_field psi, const DevParams &dp
 template <typename P>
 int run_adjoint(kf_grid live, kf_grid can, kf_field psi, const DevParams &dp, const uint8_t *active,
                 double *grad, cudaStream_t s) {
-  const int64_t N = live->count;
+  const int64_t N = live->count, plane = (int64_t)live->n[0] * live->n[1];
   EArgs<double, P> a = make_args<double, P>(live, can, psi, dp, active);
-  const int blocks = (int)((N + kRun - 1) / kRun);
-  // phi_w, its derivative, the level-set coefficients; a flag
+  // a flag; phi_w of a part and two planes to either side, its derivative, the
+  // level-set coefficients of the part and a plane to either side
+  const int64_t part = part_voxels(N, 7 * sizeof(double), 10 * plane * (int64_t)sizeof(double));
+  const int64_t nw = std::min(part + 4 * plane, N), ns = std::min(part + 2 * plane, N);
   double *buf = nullptr;
   bool own = false;
-  int rc = energy_scratch(psi, 7 * (size_t)N + 1, s, &buf, &own);
+  int rc = energy_scratch(psi, 1 + (size_t)nw + 3 * (size_t)part + 3 * (size_t)ns, s, &buf, &own);
   if (rc) return rc;
-  double *w = buf + 1, *dv = w + N, *S = dv + 3 * N;
   int *odd = reinterpret_cast<int *>(buf);
   cudaMemsetAsync(odd, 0, sizeof(int), s);
-  k_warped<double, P, true><<<blocks, kRunThreads, 0, s>>>(a, N, w, dv, odd);
-  if (dp.use_levelset) k_ls_coef<P><<<blocks, kRunThreads, 0, s>>>(a, N, w, S);
-  k_adjoint<P><<<blocks, kRunThreads, 0, s>>>(a, N, w, dv, S, odd, grad);
+  if (part < N) k_not_finite<<<(unsigned)kf_num_sms() * 8, kThreads, 0, s>>>(live->phi, N, odd);
+  for (int64_t v0 = 0; v0 < N; v0 += part) {
+    const int64_t v1 = std::min(v0 + part, N);
+    const int64_t w0 = std::max<int64_t>(v0 - 2 * plane, 0), w1 = std::min(v1 + 2 * plane, N);
+    const int64_t s0 = std::max<int64_t>(v0 - plane, 0), s1 = std::min(v1 + plane, N);
+    double *w = part_buffer(buf + 1, w0), *dv = part_buffer(buf + 1 + nw, v0),
+           *S = part_buffer(buf + 1 + nw + 3 * part, s0);
+    k_warped<double, P, true><<<run_blocks(w0, w1), kRunThreads, 0, s>>>(a, w0, w1, w, dv, part, v0, v1,
+                                                                         part < N ? nullptr : odd);
+    if (dp.use_levelset) k_ls_coef<P><<<run_blocks(s0, s1), kRunThreads, 0, s>>>(a, s0, s1, w, S, ns);
+    k_adjoint<P><<<run_blocks(v0, v1), kRunThreads, 0, s>>>(a, v0, v1, w, dv, part, S, ns, odd, grad);
+  }
   cudaError_t e = cudaGetLastError();
   if (own) {
     const cudaError_t f = cudaFreeAsync(buf, s);
