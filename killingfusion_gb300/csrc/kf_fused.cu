@@ -1172,11 +1172,19 @@ static void launch_prio(void (*kernel)(KArgs...), unsigned grid, unsigned block,
   cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// Whether the grid is small enough for the dense solver in one persistent launch
+// (persistent_test_blocks).
+static bool persistent_size(const DevParams &dp) {
+  return (dp.count + 3) / 4 <= (int64_t)kf_num_sms() * kTestThreads * kTestChunks;
+}
+
 // The split schedule's lists after the run table: hot runs, cold runs (one
-// int per run each) and their two counts.
-static size_t runs_table_bytes(int64_t nruns) {
-  const size_t table = (size_t)nruns * sizeof(int2) + ((size_t)2 * nruns + 4) * sizeof(int);
-  const size_t bits = (size_t)nruns * (kThreads * kFlatGroups * 4 / 8) + 16;  // (and a ragged end)
+// int per run each) and their two counts.  On small grids the same memory
+// also holds the persistent kernel's bit per voxel.
+static size_t runs_table_bytes(const DevParams &dp) {
+  const size_t nruns = (size_t)num_runs(dp);
+  const size_t table = nruns * sizeof(int2) + (2 * nruns + 4) * sizeof(int);
+  const size_t bits = persistent_size(dp) ? (size_t)((dp.count + 31) / 32) * sizeof(unsigned) : 0;
   return std::max(table, bits);
 }
 
@@ -1318,7 +1326,7 @@ static int persistent_blocks_per_sm() {
 static unsigned persistent_test_blocks(const DevParams &dp, cudaStream_t s) {
   if (dp.trust || kf_wait_limit_ns() < kDefaultWaitLimitNs) return 0;
   const int64_t groups = (dp.count + 3) / 4, sms = kf_num_sms();
-  if (groups > sms * kTestThreads * kTestChunks || persistent_blocks_per_sm<true>() < 1) return 0;
+  if (!persistent_size(dp) || persistent_blocks_per_sm<true>() < 1) return 0;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusActive;
   if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return 0;
   return (unsigned)std::min((groups + kTestThreads * kTestChunksMin - 1) / (kTestThreads * kTestChunksMin), sms);
@@ -1388,12 +1396,12 @@ int kf_solve_fused(kf_grid live, kf_grid can, kf_field psi, const DevParams &dp,
   if (rc) return rc;
   rc = kf_field_band_list(psi, &psi->band);
   if (rc) return rc;
-  const int64_t nruns = num_runs(dp);  // (the table also holds the persistent kernel's bit per voxel)
+  const int64_t nruns = num_runs(dp);
   if (psi->runs_cap < nruns) {
     cudaFree(psi->runs);
     psi->runs = nullptr;
     psi->runs_cap = 0;
-    if (cudaMalloc(&psi->runs, runs_table_bytes(nruns)) != cudaSuccess) {
+    if (cudaMalloc(&psi->runs, runs_table_bytes(dp)) != cudaSuccess) {
       cudaGetLastError();
       return kf_fail(KF_ERR_OOM, "cudaMalloc of the dense pass's run table failed");
     }
