@@ -405,7 +405,7 @@ __device__ __forceinline__ bool depth_ff(const uint16_t *__restrict__ depth, int
 }
 
 // The voxel on the float64 path once its pixel k is known (the float-float
-// decision could not be made, or the voxel holds a weight already): the
+// decision could not be made, or its weight or value is out of that form's range): the
 // reference's distance, clip test and running mean.  Out of line: it is
 // rare, and inline its float64 registers would crowd the common path.
 template <typename D, bool kFresh>

@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
 // per SM) in one round.  104 registers a thread: fewer spill loop state, which
 // costs a trip to L2 after every barrier, more leave the SM's L1 less
 // (sequences at 256^3 with 80, 88, 96, 104, 112, 128: 5258, 5297, 5210, 4913,
-// 5017, 5025 us for ten frames).
+// 5017, 5025 us for four frames).
 // Measured at 256^3 (14.7 k band voxels, 200 iterations): 4.7 us an iteration
 // against 8.9 us with one thread per voxel in 96-thread blocks, where 97 voxels
 // took two rounds; 64^3 (1.7 k band voxels): 3.4 us against 6.0 us.
@@ -1307,13 +1307,6 @@ static int persistent_blocks_per_sm() {
   return cached[dev];
 }
 
-// KF_SOLVER_BAND without the trust-region step: the dense first pass (on
-// phi_live alone when both buffers are zero), then every band pass in one
-// cooperative launch (k_band_persistent).  Iteration k reads buffer k % 2
-// and writes (k + 1) % 2, as the per-iteration form.  From a zero p the
-// first pass leaves both buffers zero outside its list (it copies p to q),
-// and the solve records the list: the field's buffers are then zero outside
-// its records (kf_field_zero clears just those).
 // The blocks that the dense solver's test warps need in the persistent kernel;
 // 0: it takes another schedule.  That is for large grids (above 1.2 M voxels,
 // kTestChunks: their bands take the groups of the persistent kernel many
@@ -1332,6 +1325,13 @@ static unsigned persistent_test_blocks(const DevParams &dp, cudaStream_t s) {
   return (unsigned)std::min((groups + kTestThreads * kTestChunksMin - 1) / (kTestThreads * kTestChunksMin), sms);
 }
 
+// KF_SOLVER_BAND without the trust-region step: the dense first pass (on
+// phi_live alone when both buffers are zero), then every band pass in one
+// cooperative launch (k_band_persistent).  Iteration k reads buffer k % 2
+// and writes (k + 1) % 2, as the per-iteration form.  From a zero p the
+// first pass leaves both buffers zero outside its list (it copies p to q),
+// and the solve records the list: the field's buffers are then zero outside
+// its records (kf_field_zero clears just those).
 // kDense: the dense solver (psi ends in the primary planes; nothing is
 // recorded of what the field's planes hold) with its persistent_test_blocks.
 template <bool kDense>

@@ -267,7 +267,6 @@ inline void kf_prefer_carveout(const void *func, int percent, bool (&done)[64]) 
 
 // launches implemented in kf_exact.cu (float64 arithmetic without fused
 // multiply-add where the reference's rounding decides a discrete outcome)
-int kf_grid_ensure_alt(kf_grid g);
 // fresh_phi == NULL: integrate into the grid as it is; otherwise the grid is
 // taken as reset to (*fresh_phi, 0) and every voxel is written
 int kf_launch_integrate_u16(kf_grid g, const uint16_t *depth_dev, double scale, int width, int height,
