@@ -1117,6 +1117,10 @@ constexpr int kExactSamples = 44;
 // all 33 k, 111 k, 262 k, 885 k voxels of a grid in the band: in parts 165, 264, 528, 454,
 // 1489, 3487 and 11796 us, a thread each 234, 223, 411, 353, 1137, 2666 and 9024 us.
 // (A thread per voxel of the dense grid: 408, 712, 1205, 396, 1180, 2746 and 9019 us.)
+// With the trust-region step a thread takes a voxel always: its search runs on the
+// voxel's own thread, and the data term alone leaves 7 of the 45 samples.  2.0 k, 10.3 k
+// and 38 k band voxels: in parts 114, 249 and (above the line) 97 us, a thread each 128,
+// 129 and 97 us (a thread per voxel of the dense grid 135, 154 and 289 us).
 constexpr unsigned kExactLaneShare = 112;
 constexpr int kExactThreads = kExactVoxels * kExactSamples;  // 22 warps
 
@@ -1240,8 +1244,9 @@ __global__ void __launch_bounds__(kExactThreads, 1) k_exact_band(PhiView<double>
   const unsigned n = st[iter].list;
   const unsigned per = min(max((n + gridDim.x - 1) / gridDim.x, 1u), (unsigned)kExactVoxels);
   const int tid = threadIdx.x;
+  const int nc = tp.use_levelset ? 25 : (tp.use_data ? 6 : 0), nk = tp.use_killing ? 19 : 0;
   const unsigned share = (n + gridDim.x - 1) / gridDim.x;
-  if (share >= kExactLaneShare) {
+  if (share >= kExactLaneShare || dp.trust) {
     __shared__ ExactArgs s_args;
     if (tid == 0) s_args = ExactArgs{live, can, fin, ox, oy, oz, dp, &st[iter].diverged, rows};
     __syncthreads();
@@ -1266,12 +1271,12 @@ __global__ void __launch_bounds__(kExactThreads, 1) k_exact_band(PhiView<double>
       s_v[tid] = KF_IN_BOUNDS(v, dp.count, KF_SITE_BAND_LIST) ? v : -1;
     }
     __syncthreads();
-    // the samples: 25 m at the cell centre, 19 m of the Killing stencil, m
-    // warped values
-    for (int t = tid; t < (kExactSamples + 1) * m; t += kExactThreads) {
-      const bool centre = t < 25 * m, killing = !centre && t < kExactSamples * m;
-      const int vox = centre ? t / 25 : (killing ? (t - 25 * m) / 19 : t - kExactSamples * m);
-      const int j = centre ? t % 25 : (t - 25 * m) % 19;
+    // the samples that the terms in use read: nc m at the cell centre, nk m of the
+    // Killing stencil, m warped values
+    for (int t = tid; t < (nc + nk + 1) * m; t += kExactThreads) {
+      const bool centre = t < nc * m, killing = !centre && t < (nc + nk) * m;
+      const int vox = centre ? t / nc : (killing ? (t - nc * m) / nk : t - (nc + nk) * m);
+      const int j = centre ? t % nc : (killing ? (t - nc * m) % nk : 0);
       const int i = s_v[vox];
       if (i < 0) continue;
       int x, y, z;

@@ -42,6 +42,22 @@ def test_equals_oracle(gpu, oracle, count, shell, moved, trust):
     assert moved or st["active_first"] == count
 
 
+@pytest.mark.parametrize("count", [3000, 17000])
+@pytest.mark.parametrize("data,levelset,killing", [(1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 1, 0), (1, 0, 1), (0, 1, 1),
+                                                   (0, 0, 0)])
+def test_terms_in_use(gpu, oracle, count, data, levelset, killing):
+    """The samples of terms that are switched off are not taken."""
+    shape = (33, 41, 39)
+    P = gpu.Params.reference(VOXEL, 5.0).with_(gamma_k=0.3, use_data=bool(data), use_levelset=bool(levelset),
+                                               use_killing=bool(killing))
+    live, can = scattered_pair(shape, count, count // 20, count, P)
+    psi0 = np.random.default_rng(count).normal(0.0, 0.2, shape + (3,))
+    f, run = solve(gpu, live, can, psi0, P, 2)
+    run()
+    _, want = oracle.solve(live.astype(np.float64), can.astype(np.float64), psi0, 2, oracle_params(P))
+    np.testing.assert_array_equal(f.download(), want)
+
+
 def test_non_finite_psi_stops_the_solve(gpu):
     shape = (33, 41, 39)
     P = gpu.Params.reference(VOXEL, 5.0)
