@@ -369,9 +369,9 @@ int kf_field_stats(kf_field f, int iterations, IterStats **dev) {
 }
 
 int kf_field_band_list(kf_field f, int **out) {
-  // (two of all voxels and two of the outer shell's)
+  // (two of all voxels and one of the outer shell's)
   const int64_t inner = (int64_t)std::max(f->n[0] - 2, 0) * std::max(f->n[1] - 2, 0) * std::max(f->n[2] - 2, 0);
-  if (!f->band && cudaMalloc(&f->band, (4 * f->count - 2 * inner) * sizeof(int)) != cudaSuccess) {
+  if (!f->band && cudaMalloc(&f->band, (3 * f->count - inner) * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     f->band = nullptr;
     return kf_fail(KF_ERR_OOM, "cudaMalloc of the band voxel list failed");

@@ -278,13 +278,19 @@ __global__ void __launch_bounds__(kThreads, 5) k_fused_stream_runs(FusedArgs a, 
 // st[iter+1].list).  kInPlace: the new psi of list entry k goes to entry k
 // of the output planes, for k_fused_scatter to write back.  kTrust: the
 // trust-region step (dp.trust), followed by k_trust_fix.
-// Voxels of the outer shell (shell_in: their positions in list_in) follow, a
+// Voxels of the outer shell (shell: their positions in list_in) follow, a
 // warp each (shell_gradient), dealt out over the whole launch: they lie next to
 // one another in index order, up to 2048 of them in a run along a z face.  Bands
 // cut by the face z = 0, 100 iterations at 112^3 (99 k band voxels), 160^3 (201 k)
 // and 256^3 (510 k): 3.4, 4.4 and 10.0 ms; 11.2, 13.4 and 17.1 ms where the warp
 // that met them took them one after the other, 5.9, 7.6 and 15.7 ms with a thread
-// per shell voxel.
+// per shell voxel.  With the trust-region step, which takes the data term alone, they
+// stay on their lanes (shell_data_gradient): its search is the longer part, and a
+// warp runs it once for both kinds.  A block's two warps then take entries apart
+// (voxels whose search is long lie together): bands with a face, 40 iterations at 48^3
+// and 100^3: 5.4 and 12.5 ms, band-only 4.3 and 6.5 ms; 5.4, 13.0, 4.3 and 7.5 ms with
+// the warps' entries together, 9.0, 17.9, 6.1 and 13.3 ms with a warp per shell voxel
+// (5.7, 12.0, 4.6 and 8.3 ms with a thread each in the order of an atomic counter).
 // The dense solver runs it beside the cold passes, which live on L1 and
 // occupancy, so it takes no shared memory to speak of: with the groups of four
 // warps of the band-only solver (13 KB a group) the 256^3 iteration took 42.7 us
@@ -293,8 +299,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_fused_stream_runs(FusedArgs a, 
 template <bool kCarry, bool kInPlace, bool kTrust = false>
 __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(FusedArgs a, const int *__restrict__ list_in,
                                                              int *__restrict__ list_out,
-                                                             const int *__restrict__ shell_in,
-                                                             int *__restrict__ shell_out) {
+                                                             const int *__restrict__ shell) {
   if (iteration_gated(a.st, a.iter, a.dp)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) a.st[a.iter].skipped = 1;
     return;
@@ -308,24 +313,43 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
   double energy = 0.0;  // this thread's voxels, summed in float64 as the block and grid sums
   unsigned active = 0;
   bool diverged = false;
+  if (kTrust) {
+    if (threadIdx.x == 0) s_args = a;
+    __syncthreads();
+  }
   for (int r = 0; r < rounds; ++r) {
-    const int k = (r * gridDim.x + blockIdx.x) * kLaneThreads + threadIdx.x;
+    const int k = kTrust ? ((r * kLaneWarps + (int)(threadIdx.x >> 5)) * (int)gridDim.x + (int)blockIdx.x) * 32 +
+                               (int)(threadIdx.x & 31)
+                         : (r * gridDim.x + blockIdx.x) * kLaneThreads + threadIdx.x;
     const int v = k < nq ? list_in[k] : -1;
     int x, y, z, next = -1;  // next: the voxel this thread hands to the next iteration
+    const int slot = kInPlace ? k : v;
     if (v >= 0) {
       voxel_xyz(a.dp, v, x, y, z);
-      if (interior_voxel(a.dp, x, y, z))
-        next = update_interior_voxel<kTrust>(a, v, kInPlace ? k : v, maxd, energy, active, diverged);
+      const bool interior = interior_voxel(a.dp, x, y, z);
+      if (kTrust) {
+        // (one call for both kinds: a warp with both searches once)
+        if (KF_IN_BOUNDS(v, a.dp.count, KF_SITE_BAND_LIST) && KF_IN_BOUNDS(slot, a.dp.count, KF_SITE_BAND_LIST)) {
+          float d[3], s, en, c0[3];
+          if (interior)
+            gradient_lane<kPsiReadOnly>(a, x, y, z, v, d, s, en, c0);
+          else
+            shell_data_gradient(s_args, x, y, z, d, &s, &en, c0);
+          next = settle_band_voxel<true>(a, v, slot, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
+        }
+      } else if (interior) {
+        next = update_interior_voxel<false>(a, v, slot, maxd, energy, active, diverged);
+      }
     }
     if (kCarry) block_append<kLaneWarps>(next, &a.st[a.iter + 1].list, list_out, a.dp.count);
   }
-  const unsigned nshell = a.st[a.iter].shell;
+  const unsigned nshell = kTrust ? 0u : a.st[a.iter].shell;
   if (blockIdx.x < nshell) {
     if (threadIdx.x == 0) s_args = a;
     __syncthreads();
     const unsigned warp = threadIdx.x >> 5;
     for (unsigned j = warp * gridDim.x + blockIdx.x; j < nshell; j += kLaneWarps * gridDim.x) {
-      const int k = shell_in[j];
+      const int k = shell[j];
       if (!KF_IN_BOUNDS(k, a.dp.count, KF_SITE_BAND_LIST)) continue;
       const int v = list_in[k];
       if (!KF_IN_BOUNDS(v, a.dp.count, KF_SITE_BAND_LIST)) continue;
@@ -334,15 +358,8 @@ __global__ void __launch_bounds__(kLaneThreads, kLaneBlocksPerSM) k_fused_band(F
       if (interior_voxel(a.dp, x, y, z)) continue;  // (the bounds-check build's unwritten entries)
       float d[3], s, en, c0[3];
       shell_gradient<kPsiReadOnly>(s_args, false, x, y, z, s_shell[warp], d, &s, &en, c0);
-      if ((threadIdx.x & 31) == 0) {
-        const int next = settle_band_voxel<kTrust>(a, v, kInPlace ? k : v, x, y, z, s, en, c0, d, maxd, energy, active,
-                                                   diverged);
-        if (kCarry && next >= 0) {
-          const unsigned pos = atomicAdd(&a.st[a.iter + 1].list, 1u), at = atomicAdd(&a.st[a.iter + 1].shell, 1u);
-          if (KF_IN_BOUNDS(pos, a.dp.count, KF_SITE_BAND_APPEND)) list_out[pos] = next;
-          if (KF_IN_BOUNDS(at, shell_voxels(a.dp), KF_SITE_BAND_APPEND)) shell_out[at] = (int)pos;
-        }
-      }
+      if ((threadIdx.x & 31) == 0)
+        settle_band_voxel<false>(a, v, kInPlace ? k : v, x, y, z, s, en, c0, d, maxd, energy, active, diverged);
     }
     __syncwarp();
   }
@@ -1228,7 +1245,7 @@ static void launch_split_iterations(FusedArgs a, kf_field psi, const DevParams &
     }
     if (it + 1 < iterations) cudaEventRecord(fork, s);
     launch_prio(k_fused_band<false, true>, band_blocks, kLaneThreads, s, hi, a, (const int *)lst[it & 1],
-                (int *)nullptr, (const int *)shell, (int *)nullptr);
+                (int *)nullptr, (const int *)shell);
     if (it == iterations - 1)
       launch_prio(k_fused_scatter, band_blocks, kThreads, s, hi, a, (const int *)lst[it & 1],
                   (float *)psi->p[0], (float *)psi->p[1], (float *)psi->p[2]);
@@ -1249,7 +1266,6 @@ static void launch_iterations(kf_grid live, kf_grid can, kf_field psi, const Dev
   FusedArgs a = make_args(live, can, dp, st);
   void *buf[2][3] = {{psi->p[0], psi->p[1], psi->p[2]}, {psi->q[0], psi->q[1], psi->q[2]}};
   int *lst[2] = {lists, lists + dp.count};
-  int *shell[2] = {lists + 2 * dp.count, lists + 2 * dp.count + shell_voxels(dp)};
   const int nrows = dp.ny * dp.nz;
   if (dp.trust) cudaMemsetAsync(rows, 0x7f, (size_t)nrows * sizeof(int), s);
   for (int it = 0; it < iterations; ++it) {
@@ -1267,17 +1283,17 @@ static void launch_iterations(kf_grid live, kf_grid can, kf_field psi, const Dev
     int *next_rows = dp.trust ? rows + ((it + 1) & 1) * nrows : nullptr;
     if (!band_only) {
       // lists alternate so that a run can still read the previous iteration's
-      k_fused_stream<false><<<grid, block, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1], runs, shell[0]);
-      k_fused_band<false, true, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], nullptr, shell[0], nullptr);
+      k_fused_stream<false><<<grid, block, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1], runs, nullptr);
+      k_fused_band<false, true, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], nullptr, nullptr);
       k_trust_fix<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], true, next_rows);
       if (it == iterations - 1)
         k_fused_scatter<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], (float *)in[0], (float *)in[1],
                                                         (float *)in[2]);
     } else {
-      if (it == 0) k_fused_stream<true><<<grid, block, 0, s>>>(a, lst[0], nullptr, nullptr, shell[0]);
+      if (it == 0) k_fused_stream<true><<<grid, block, 0, s>>>(a, lst[0], nullptr, nullptr, nullptr);
       // (with the trust-region step; without it the solver is k_band_persistent)
       k_fused_band<true, false, true><<<band_blocks, kLaneThreads, 0, s>>>(a, lst[it & 1], lst[(it + 1) & 1],
-                                                                         shell[it & 1], shell[(it + 1) & 1]);
+                                                                         nullptr);
       k_trust_fix<<<band_blocks, kThreads, 0, s>>>(a, lst[it & 1], false, next_rows);
     }
   }

@@ -45,7 +45,7 @@ struct kf_field_s {
   size_t plain_bytes;
   FusedGraph *graph;      // captured fused iteration loop
   int *band;              // band-voxel lists (two, of one int per voxel each,
-                          // and two of one int per voxel of the outer shell)
+                          // and one of one int per voxel of the outer shell)
   int2 *runs;             // per run of the dense pass: its entries of the list
   int64_t runs_cap;
   int *rows;              // trust-region step: the first x of each row (y, z)
