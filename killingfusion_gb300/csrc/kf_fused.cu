@@ -1233,7 +1233,8 @@ static void launch_split_iterations(FusedArgs a, kf_field psi, const DevParams &
     a.iter = it;
     if (it == 0) {
       launch_prio(k_fused_stream<false>, grid, kThreads, s, hi, a, lst[0], lst[1], runs, shell);
-      launch_prio(k_split_runs, 1, kSplitThreads, s, hi, (const int2 *)runs, (int)nruns, hot, cold, counts);
+      if (iterations > 1)
+        launch_prio(k_split_runs, 1, kSplitThreads, s, hi, (const int2 *)runs, (int)nruns, hot, cold, counts);
     } else {
       // cold runs beside the band pass of the iteration before
       cudaStreamWaitEvent(cold_s, fork, 0);
@@ -1328,12 +1329,13 @@ static int persistent_blocks_per_sm() {
 // kTestChunks: their bands take the groups of the persistent kernel many
 // rounds.  100 iterations at 104^3 with 45 k, 506 k and 1.1 M band voxels: 1.1,
 // 7.9 and 28.7 ms against 2.0, 16.6 and 49.6 on the split schedule; 128^3 with
-// 68 k and 341 k: 2.0 and 4.7 ms against 2.2 and 4.1), a wait limit
+// 68 k and 341 k: 2.0 and 4.7 ms against 2.2 and 4.1), a single iteration, which
+// its three launches and two clears outweigh (64^3 and 100^3: 26 and 36 us against 16 and 17), a wait limit
 // below the default (the other schedules wait for nothing, so no limit makes
 // them fail) and a stream that is being captured (which refuses the others'
 // graph).
-static unsigned persistent_test_blocks(const DevParams &dp, cudaStream_t s) {
-  if (dp.trust || kf_wait_limit_ns() < kDefaultWaitLimitNs) return 0;
+static unsigned persistent_test_blocks(const DevParams &dp, int iterations, cudaStream_t s) {
+  if (dp.trust || iterations < 2 || kf_wait_limit_ns() < kDefaultWaitLimitNs) return 0;
   const int64_t groups = (dp.count + 3) / 4, sms = kf_num_sms();
   if (!persistent_size(dp) || persistent_blocks_per_sm<true>() < 1) return 0;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusActive;
@@ -1425,7 +1427,7 @@ int kf_solve_fused(kf_grid live, kf_grid can, kf_field psi, const DevParams &dp,
   }
   if (band_only && !dp.trust)
     return launch_band_persistent<false>(live, can, psi, dp, iterations, st, p_zero, q_zero, 1u, s);
-  if (const unsigned test_blocks = band_only ? 0u : persistent_test_blocks(dp, s))
+  if (const unsigned test_blocks = band_only ? 0u : persistent_test_blocks(dp, iterations, s))
     return launch_band_persistent<true>(live, can, psi, dp, iterations, st, p_zero, q_zero, test_blocks, s);
   int *rows = nullptr;
   if (dp.trust) {
