@@ -62,7 +62,11 @@ typedef enum kf_precision {
 typedef enum kf_solver {
   KF_SOLVER_FUSED = 0, /* the dense fused stencil, every voxel tested in every
                           iteration: one persistent launch on small grids, a
-                          captured graph of passes on the others            */
+                          captured graph of passes on the others.  The
+                          persistent launches (this one and KF_SOLVER_BAND)
+                          take every SM: solves on several streams run one
+                          after the other, and wait until a caller's kernels
+                          have left room on every SM                        */
   KF_SOLVER_PLAIN = 1, /* one kernel per energy term, fields through HBM   */
   KF_SOLVER_EXACT = 2, /* float64 replay of the reference (needs KF_F64 psi) */
   KF_SOLVER_BAND = 3,  /* the fused stencil on the band only: a voxel outside
